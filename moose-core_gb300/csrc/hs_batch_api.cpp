@@ -412,7 +412,7 @@ int buildFp64(HsBatch* b, const HsCellDesc* cells) {
             const Table& T = pass ? b->plans[c].caTable : b->plans[c].vTable;
             auto key = std::make_pair(fnv(T.data.data(), T.data.size() * 8), T.data.size());
             auto it = tabDev.find(key);
-            if (it == tabDev.end()) it = tabDev.emplace(key, b->buf.up(T.data, b->st)).first;
+            if (it == tabDev.end()) it = tabDev.emplace(key, b->buf.up(pairTable(T), b->st)).first;
             (pass ? catab : vtab)[c] = it->second;
         }
     }

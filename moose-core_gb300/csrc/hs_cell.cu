@@ -27,6 +27,33 @@ struct Uploader {
 
 }  // namespace
 
+// Per row i and species {A_i, A_{i+1} - A_i, B_i, B_{i+1} - B_i}: the lookups
+// interpolate between rows i and i + 1, and the last row is never the lower.
+std::vector<double> pairTable(const Table& t) {
+    std::vector<double> out;
+    if (!t.nCol) return out;
+    out.reserve(2 * (size_t)(t.nPts - 1) * t.nCol);
+    for (uint32_t i = 0; i + 1 < t.nPts; ++i) {
+        const double* a = t.data.data() + (size_t)i * t.nCol;
+        for (uint32_t k = 0; k < t.nCol; ++k) {
+            out.push_back(a[k]);
+            out.push_back(a[t.nCol + k] - a[k]);
+        }
+    }
+    return out;
+}
+
+namespace {
+
+uint32_t powCode(double p) {
+    if (!(p > 0.0)) return 0;
+    for (uint32_t k = 1; k <= 4; ++k)
+        if (p == (double)k) return k;
+    return kPowGeneral;
+}
+
+}  // namespace
+
 cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCap,
                        cudaStream_t st, const CellShared* sh) {
     Uploader u{a, st};
@@ -86,9 +113,13 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.state = u.put(P.state0);
     c.extCa = u.zeros<double>(P.C);
     c.instant = u.put(P.instant);
-    c.stateOff = u.put(P.stateOff);
-    c.colX = u.put(P.colX);
-    c.colY = u.put(P.colY);
+    {
+        std::vector<uint4> ca(P.C);
+        for (uint32_t q = 0; q < P.C; ++q)
+            ca[q] = make_uint4(powCode(P.Xpow[q]) | powCode(P.Ypow[q]) << 4 | powCode(P.Zpow[q]) << 8,
+                               (uint32_t)P.stateOff[q], (uint32_t)P.colX[q], (uint32_t)P.colY[q]);
+        c.chanA = u.put(ca);
+    }
     c.colZ = u.put(P.colZ);
     c.zSrc = u.put(P.zSrc);
     {
@@ -107,10 +138,14 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.iCa = u.zeros<double>(P.P);
     c.feedPtr = u.put(P.feedPtr);
     c.feedChan = u.put(P.feedChan);
-    c.vTab = sh ? sh->vTab : u.put(P.vTable.data);
+    c.vTab = sh ? sh->vTab : u.put(pairTable(P.vTable));
     c.vCol = P.vTable.nCol; c.vMin = P.vTable.min; c.vMax = P.vTable.max; c.vDx = P.vTable.dx;
-    c.caTab = sh ? sh->caTab : u.put(P.caTable.data);
+    c.vRows = P.vTable.nPts;
+    c.vRdx = 1.0 / c.vDx;
+    c.caTab = sh ? sh->caTab : u.put(pairTable(P.caTable));
     c.caCol = P.caTable.nCol; c.caMin = P.caTable.min; c.caMax = P.caTable.max; c.caDx = P.caTable.dx;
+    c.caRows = P.caTable.nPts;
+    c.caRdx = 1.0 / c.caDx;
     {
         std::vector<double> AB, geom;
         std::vector<uint64_t> off;
@@ -136,11 +171,16 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     }
     c.c2dCompt = u.put(P.c2dCompt);
     c.c2dGate = u.put(P.c2dGate);
-    c.c2dDep0 = u.put(P.c2dDep0);
-    c.c2dDep1 = u.put(P.c2dDep1);
+    {
+        auto dep = [](int32_t d) { return d < 0 || d > 2 ? 3u : (uint32_t)d; };
+        std::vector<uint32_t> ka(P.K2);
+        for (uint32_t k = 0; k < P.K2; ++k)
+            ka[k] = powCode(P.c2dXpow[k]) | dep(P.c2dDep0[k]) << 4 | dep(P.c2dDep1[k]) << 8 |
+                    ((uint32_t)P.c2dInstant[k] & 0xFu) << 12;
+        c.c2dA = u.put(ka);
+    }
     c.c2dConc1 = u.put(P.c2dConc1);
     c.c2dConc2 = u.put(P.c2dConc2);
-    c.c2dInstant = u.put(P.c2dInstant);
     c.c2dGbar = u.put(P.c2dGbar);
     c.c2dEk = u.put(P.c2dEk);
     c.c2dXpow = u.put(P.c2dXpow);

@@ -29,6 +29,7 @@ struct Arena {
 // A batch passes `shared`: device arrays it owns (initVm and SynChan
 // constants of all cells contiguous, for one-copy reinit) and rate tables
 // shared by the cells that have identical ones.
+std::vector<double> pairTable(const Table& t);   // rate table as the FP64 kernels read it (DevCell::vTab)
 struct CellShared {
     double* initVm = nullptr;
     double* synConst = nullptr;

@@ -16,6 +16,8 @@
 
 #include <cstdint>
 
+#include "hs_exact.cuh"
+
 namespace hsg {
 
 constexpr uint32_t kDifState = 13;
@@ -57,25 +59,28 @@ struct DevCell {
     // channels
     double *Gbar, *Ek, *Xpow, *Ypow, *Zpow, *mod, *Gk, *state, *extCa;
     int32_t* instant;
-    const int32_t *stateOff, *colX, *colY, *colZ, *zSrc;
+    const int32_t *colZ, *zSrc;
+    const uint4* chanA;          // per channel: power codes (kPow*, bits 0-3 X, 4-7 Y, 8-11 Z), first state, X and Y columns
     const uint32_t* chanCompt;
     // pools
     double *c, *CaBasal, *f1, *f2, *ceil, *floor_, *ca, *iCa;
     const uint32_t *feedPtr, *feedChan;
-    // rate tables
+    // rate tables, per row and species {A, A of the next row - A, B, B of the
+    // next row - B} (pairTable); vRdx = RN(1 / vDx)
     const double* vTab;
-    uint32_t vCol;
-    double vMin, vMax, vDx;
+    uint32_t vCol, vRows;
+    double vMin, vMax, vDx, vRdx;
     const double* caTab;
-    uint32_t caCol;
-    double caMin, caMax, caDx;
+    uint32_t caCol, caRows;
+    double caMin, caMax, caDx, caRdx;
     // HHChannel2D
     const double* g2dAB;
     const uint64_t* g2dOff;          // per gate2d: offset (in doubles) into g2dAB
     const double* g2dGeom;           // per gate2d: xmin,xmax,ymin,ymax,invDx,invDy
     const uint32_t* g2dN;            // per gate2d: nx, ny
     const uint32_t* c2dCompt;
-    const int32_t *c2dGate, *c2dDep0, *c2dDep1, *c2dConc1, *c2dConc2, *c2dInstant;
+    const int32_t *c2dGate, *c2dConc1, *c2dConc2;
+    const uint32_t* c2dA;            // X power code (bits 0-3), inputs (4-7, 8-11: 0 Vm, 1 conc1, 2 conc2, 3 none), instant bits (12-15)
     double *c2dGbar, *c2dEk, *c2dXpow, *c2dMod, *c2dX, *c2dGk, *c2dVm, *c2dC1, *c2dC2;
     const double* c2dX0;         // X at reinit
     // SynChans
@@ -120,6 +125,8 @@ struct FieldWrite {
     uint32_t pad;
 };
 
+#ifdef __CUDACC__
+
 // The value a recording entry names (hsolve/HSolveActive.cpp:354-385 for Ik).
 __device__ __forceinline__ double recValue(const DevCell& c, uint32_t e) {
     const uint32_t i = e & ((1u << kRecShift) - 1);
@@ -134,48 +141,48 @@ __device__ __forceinline__ double recValue(const DevCell& c, uint32_t e) {
 // ---------------------------------------------------------------------------
 // FP64 helpers, reference order
 
+// Power codes: 0 the gate is absent, 1..4 that power, kPowGeneral any other.
+constexpr uint32_t kPowGeneral = 5;
+
 struct Row {
-    int64_t off;      // first column of the row
+    uint32_t i;       // table row
     double frac;
 };
 
-__device__ __forceinline__ Row tableRow(double x, double mn, double mx, double dx, uint32_t nCol) {
-    if (x < mn) x = mn;
-    else if (x > mx) x = mx;
-    double div = (x - mn) / dx;
-    unsigned int integer = (unsigned int)(div);
+__device__ __forceinline__ Row tableRow(double x, double mn, double mx, double dx, double rdx, uint32_t nRows) {
+    if (lessThan(x, mn)) x = mn;
+    else if (lessThan(mx, x)) x = mx;
     Row r;
-    r.frac = div - integer;
-    r.off = (int64_t)integer * nCol;
+    r.i = min(splitFraction(quotientBy(x - mn, dx, rdx), r.frac), nRows - 2);
     return r;
 }
 
+// One 32-byte read per gate; the difference of the two rows is tabulated (the
+// same rounded subtraction), which takes two of six FP64 operations away.
 __device__ __forceinline__ void tableLookup(const double* T, uint32_t nCol, int32_t column,
                                             const Row& r, double& C1, double& C2) {
-    const double* ap = T + r.off + column;
-    const double* bp = ap + nCol;
-    double a = ap[0], b = bp[0];
-    C1 = a + (b - a) * r.frac;
-    a = ap[1];
-    b = bp[1];
-    C2 = a + (b - a) * r.frac;
+    const double2* p = reinterpret_cast<const double2*>(T + 2 * ((size_t)r.i * nCol + column));
+    const double2 a = __ldg(p), b = __ldg(p + 1);
+    C1 = a.x + a.y * r.frac;
+    C2 = b.x + b.y * r.frac;
 }
 
 __device__ __forceinline__ double gateStep(double x, double C1, double C2, double dt, bool inst) {
-    if (inst) return C1 / C2;
-    double temp = 1.0 + dt / 2.0 * C2;
-    return (x * (2.0 - temp) + dt * C1) / temp;
+    if (inst) return plainQuotient(C1, C2);
+    const double temp = 1.0 + dt / 2.0 * C2;
+    return quotient(x * (2.0 - temp) + dt * C1, temp);
 }
 
-__device__ __forceinline__ double takePower(double x, double p) {
-    if (p == 1.0) return x;
-    if (p == 2.0) return x * x;
-    if (p == 3.0) return x * x * x;
-    if (p == 4.0) {
-        double y = x * x;
+// x to the power of `code`; `p` holds a general power.
+__device__ __forceinline__ double takePower(double x, uint32_t code, const double* p) {
+    if (code == 1) return x;
+    if (code == 2) return x * x;
+    if (code == 3) return x * x * x;
+    if (code == 4) {
+        const double y = x * x;
         return y * y;
     }
-    if (x > 0.0) return exp(p * log(x));
+    if (lessThan(0.0, x)) return exp(*p * log(x));
     return 0.0;
 }
 
@@ -183,23 +190,25 @@ __device__ __forceinline__ double takePower(double x, double p) {
 __device__ __forceinline__ void interp2dBoth(const double* AB, const double* geom, uint32_t nx,
                                              uint32_t ny, double x, double y, double& A,
                                              double& B) {
-    double xmin = geom[0], xmax = geom[1], ymin = geom[2], ymax = geom[3];
-    if (x < xmin) x = xmin;
-    if (x > xmax) x = xmax;
-    if (y < ymin) y = ymin;
-    if (y > ymax) y = ymax;
-    double xv = (x - xmin) * geom[4];
-    unsigned long xi = (unsigned long)xv;
-    if (xi >= nx) xi = nx - 1;
-    bool endX = xi == nx - 1;
-    double xF = xv - xi;
-    double yv = (y - ymin) * geom[5];
-    unsigned long yi = (unsigned long)yv;
-    if (yi >= ny) yi = ny - 1;
-    bool endY = yi == ny - 1;
-    double yF = yv - yi;
+    const double xmin = geom[0], xmax = geom[1], ymin = geom[2], ymax = geom[3];
+    if (lessThan(x, xmin)) x = xmin;
+    if (lessThan(xmax, x)) x = xmax;
+    if (lessThan(y, ymin)) y = ymin;
+    if (lessThan(ymax, y)) y = ymax;
+    double xF, yF;
+    const double xv = (x - xmin) * geom[4], yv = (y - ymin) * geom[5];
+    uint32_t xi = splitFraction(xv, xF), yi = splitFraction(yv, yF);
+    if (xi >= nx) {
+        xi = nx - 1;
+        xF = xv - xi;
+    }
+    if (yi >= ny) {
+        yi = ny - 1;
+        yF = yv - yi;
+    }
+    const bool endX = xi == nx - 1, endY = yi == ny - 1;
     double xFyF = xF * yF;
-    const double* p00 = AB + 2 * (xi * ny + yi);
+    const double* p00 = AB + 2 * ((size_t)xi * ny + yi);
     double a00 = p00[0], b00 = p00[1];
     double a01 = 0.0, b01 = 0.0, a10 = 0.0, b10 = 0.0, a11 = 0.0, b11 = 0.0;
     if (!endX) {
@@ -216,5 +225,7 @@ __device__ __forceinline__ void interp2dBoth(const double* AB, const double* geo
     A = a00 * w00 + a10 * w10 + a01 * w01 + a11 * xFyF;
     B = b00 * w00 + b10 * w10 + b01 * w01 + b11 * xFyF;
 }
+
+#endif  // __CUDACC__
 
 }  // namespace hsg

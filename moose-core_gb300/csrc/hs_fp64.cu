@@ -197,13 +197,13 @@ __device__ __forceinline__ void synchanStep(const DevCell& c, uint32_t k, double
     // SimpleSynHandler::vProcess: deliver events with time <= currTime
     double activation = 0.0;
     uint32_t e = c.evCur[k], end = c.evPtr[k + 1];
-    while (e < end && c.evTime[e] <= currTime) {
+    while (e < end && atMost(c.evTime[e], currTime)) {
         activation += c.evW[e] / c.dt;
         ++e;
     }
     c.evCur[k] = e;
     double act = c.synAct[k];
-    if (activation != 0.0) act += activation;
+    if (!isZero(activation)) act += activation;
     // SynChan::calcGk
     double X = act * c.synXc1[k] + c.synX[k] * c.synXc2[k];
     double Y = X * c.synYc1[k] + c.synY[k] * c.synYc2[k];
@@ -213,77 +213,80 @@ __device__ __forceinline__ void synchanStep(const DevCell& c, uint32_t k, double
     c.synGk[k] = Y * c.synNorm[k] * c.synMod[k];
 }
 
-__device__ __forceinline__ double depValue(int dep, double vm, double c1, double c2) {
+__device__ __forceinline__ double depValue(uint32_t dep, double vm, double c1, double c2) {
     return dep == 0 ? vm : dep == 1 ? c1 : dep == 2 ? c2 : 0.0;
 }
 
 __device__ __forceinline__ void chan2dStep(const DevCell& c, uint32_t k) {
     double g = c.c2dGbar[k];
-    double xp = c.c2dXpow[k];
-    if (xp > 0) {
-        int gi = c.c2dGate[k];
-        double vm = c.c2dVm[k], c1 = c.c2dC1[k], c2 = c.c2dC2[k];
-        double x = depValue(c.c2dDep0[k], vm, c1, c2);
-        double y = depValue(c.c2dDep1[k], vm, c1, c2);
+    const uint32_t a = c.c2dA[k];
+    if (a & 15u) {
+        const int gi = c.c2dGate[k];
+        const double vm = c.c2dVm[k], c1 = c.c2dC1[k], c2 = c.c2dC2[k];
+        const double x = depValue((a >> 4) & 15u, vm, c1, c2);
+        const double y = depValue((a >> 8) & 15u, vm, c1, c2);
         double A, B;
         interp2dBoth(c.g2dAB + c.g2dOff[gi], c.g2dGeom + 6 * gi, c.g2dN[2 * gi],
                      c.g2dN[2 * gi + 1], x, y, A, B);
         double X = c.c2dX[k];
-        if (c.c2dInstant[k] & 1) {
-            X = A / B;
-        } else if (B > 1.0e-10) {   // HHChannelBase::integrate (exponential Euler)
-            double e = exp(-B * c.dt);
-            X = X * e + (A / B) * (1 - e);
+        if ((a >> 12) & 1u) {
+            X = plainQuotient(A, B);
+        } else if (lessThan(1.0e-10, B)) {   // HHChannelBase::integrate (exponential Euler)
+            const double e = exp(-B * c.dt);
+            X = X * e + quotient(A, B) * (1 - e);
         } else {
             X = X + A * c.dt;
         }
         c.c2dX[k] = X;
-        g *= takePower(X, xp);
+        g *= takePower(X, a & 15u, c.c2dXpow + k);
     }
-    c.c2dGk[k] = g * c.c2dMod[k];
+    const double mod = c.c2dMod[k];
+    c.c2dGk[k] = isOne(mod) ? g : g * mod;
 }
 
 // ---- tick 6, per compartment: channels + matrix row -----------------------
+// Bound by the FP64 pipe (76 cycles per warp instruction and sub-partition):
+// the gates run in one loop over X, Y, Z, and what is not an operation of the
+// reference's arithmetic (compares, row indices, powers of 1, factors of 1)
+// is kept off that pipe.
 __device__ __forceinline__ void comptStep(const DevCell& c, uint32_t ic) {
     double V = c.V[ic];
-    Row vRow = tableRow(V, c.vMin, c.vMax, c.vDx, c.vCol);
+    const Row vRow = tableRow(V, c.vMin, c.vMax, c.vDx, c.vRdx, c.vRows);
     double GkSum = 0.0, GkEkSum = 0.0;
     for (uint32_t q = c.chanPtr[ic]; q < c.chanPtr[ic + 1]; ++q) {
-        int32_t s = c.stateOff[q];
-        int inst = c.instant[q];
+        const uint4 A = c.chanA[q];
+        const int inst = c.instant[q];
         double fraction = c.mod[q];
-        double C1, C2;
-        double xp = c.Xpow[q], yp = c.Ypow[q], zp = c.Zpow[q];
-        double xs = 0, ys = 0, zs = 0;
-        if (xp > 0.0) {
-            tableLookup(c.vTab, c.vCol, c.colX[q], vRow, C1, C2);
-            xs = gateStep(c.state[s], C1, C2, c.dt, inst & 1);
-            c.state[s++] = xs;
-        }
-        if (yp > 0.0) {
-            tableLookup(c.vTab, c.vCol, c.colY[q], vRow, C1, C2);
-            ys = gateStep(c.state[s], C1, C2, c.dt, inst & 2);
-            c.state[s++] = ys;
-        }
-        if (zp > 0.0) {
-            int32_t src = c.zSrc[q];
-            if (src >= 0) {
-                Row r = tableRow(c.ca[src], c.caMin, c.caMax, c.caDx, c.caCol);
-                tableLookup(c.caTab, c.caCol, c.colZ[q], r, C1, C2);
-            } else if (c.extCa[q] > 0) {
-                Row r = tableRow(c.extCa[q], c.caMin, c.caMax, c.caDx, c.caCol);
-                tableLookup(c.caTab, c.caCol, c.colZ[q], r, C1, C2);
-            } else {
-                tableLookup(c.vTab, c.vCol, c.colZ[q], vRow, C1, C2);
+        bool one = isOne(fraction);
+        uint32_t s = A.y;
+        int32_t col = (int32_t)A.z;
+        for (uint32_t g = 0; g < 3; ++g) {      // X, Y, Z (ChannelStruct::process multiplies in that order)
+            const uint32_t code = (A.x >> (4 * g)) & 15u;
+            if (code) {
+                Row r = vRow;
+                const double* T = c.vTab;
+                uint32_t nCol = c.vCol;
+                if (g == 2) {
+                    const int32_t src = c.zSrc[q];
+                    col = c.colZ[q];
+                    const double ca = src >= 0 ? c.ca[src] : c.extCa[q];
+                    if (src >= 0 || lessThan(0.0, ca)) {
+                        r = tableRow(ca, c.caMin, c.caMax, c.caDx, c.caRdx, c.caRows);
+                        T = c.caTab;
+                        nCol = c.caCol;
+                    }
+                }
+                double C1, C2;
+                tableLookup(T, nCol, col, r, C1, C2);
+                const double x = gateStep(c.state[s], C1, C2, c.dt, inst & (1 << g));
+                c.state[s++] = x;
+                const double pw = takePower(x, code, (g == 0 ? c.Xpow : g == 1 ? c.Ypow : c.Zpow) + q);
+                fraction = one ? pw : fraction * pw;
+                one = false;
             }
-            zs = gateStep(c.state[s], C1, C2, c.dt, inst & 4);
-            c.state[s] = zs;
+            col = (int32_t)A.w;
         }
-        // ChannelStruct::process
-        if (xp > 0.0) fraction *= takePower(xs, xp);
-        if (yp > 0.0) fraction *= takePower(ys, yp);
-        if (zp > 0.0) fraction *= takePower(zs, zp);
-        double gk = c.Gbar[q] * fraction;
+        const double gk = c.Gbar[q] * fraction;
         c.Gk[q] = gk;
         GkSum += gk;
         GkEkSum += gk * c.Ek[q];
@@ -330,7 +333,7 @@ __device__ __forceinline__ void forwardCableRun(const DevCell& c, uint32_t r, ui
             dNext = M[r + 1];
             rNext = M[N + r + 1];
         }
-        const double q = o / d;
+        const double q = quotient(o, d);
         d = dr - q * o;
         rhs = rr - q * rhs;
         M[r] = d;
@@ -353,9 +356,9 @@ __device__ __forceinline__ void backwardCableRun(const DevCell& c, uint32_t i, u
         }
         double v = r;
         v -= o * vNext;
-        v /= dg;
+        v = quotient(v, dg);
         c.VMid[i] = v;
-        c.V[i] = 2 * v - vo;
+        c.V[i] = __fma_rn(2.0, v, -vo);     // 2 v is exact
         vNext = v;
     }
 }
@@ -382,7 +385,7 @@ __device__ __forceinline__ void eliminate(const DevCell& c, uint32_t tid, uint32
         for (uint32_t w = 0; w < c.fWaves; ++w) {
             for (uint32_t k = c.fWavePtr[w] + tid; k < c.fWavePtr[w + 1]; k += nth) {
                 const int4 x = c.fWaveOps[2 * k], y = c.fWaveOps[2 * k + 1];
-                const double q = M[y.x] / M[y.y];
+                const double q = quotient(M[y.x], M[y.y]);
                 M[x.x] -= q * M[x.y];
                 if (x.z >= 0) M[x.z] -= q * M[x.w];
             }
@@ -407,13 +410,13 @@ __device__ __forceinline__ void eliminate(const DevCell& c, uint32_t tid, uint32
                 }
             }
             if (k0 < e) {
-                const double q = M[y0.x] / M[y0.y];
+                const double q = quotient(M[y0.x], M[y0.y]);
                 M[x0.x] -= q * M[x0.y];
                 if (x0.z >= 0) M[x0.z] -= q * M[x0.w];
             }
             for (uint32_t k = k0 + nth; k < e; k += nth) {
                 const int4 x = c.fWaveOps[2 * k], y = c.fWaveOps[2 * k + 1];
-                const double q = M[y.x] / M[y.y];
+                const double q = quotient(M[y.x], M[y.y]);
                 M[x.x] -= q * M[x.y];
                 if (x.z >= 0) M[x.z] -= q * M[x.w];
             }
@@ -438,7 +441,7 @@ __device__ __forceinline__ void eliminate(const DevCell& c, uint32_t tid, uint32
             for (uint32_t o = c.fOpPtr[k]; o < c.fOpPtr[k + 1]; ++o) {
                 int4 op = c.fOps[o];
                 if (op.y != ql || op.w != qp) {
-                    q = M[op.y] / M[op.w];
+                    q = quotient(M[op.y], M[op.w]);
                     ql = op.y;
                     qp = op.w;
                 }
@@ -468,9 +471,9 @@ __device__ __forceinline__ void eliminate(const DevCell& c, uint32_t tid, uint32
                     int2 term = c.bTerms[t];
                     v -= M[term.x] * c.VMid[term.y];
                 }
-                v /= M[i];
+                v = quotient(v, M[i]);
                 c.VMid[i] = v;
-                c.V[i] = 2 * v - c.V[i];
+                c.V[i] = __fma_rn(2.0, v, -c.V[i]);
             }
             levelSync<WARP>();
         }
@@ -510,9 +513,9 @@ __device__ __forceinline__ void eliminate(const DevCell& c, uint32_t tid, uint32
                 int2 term = c.bTerms[t];
                 v -= M[term.x] * c.VMid[term.y];
             }
-            v /= d0;
+            v = quotient(v, d0);
             c.VMid[i0] = v;
-            c.V[i0] = 2 * v - v0;
+            c.V[i0] = __fma_rn(2.0, v, -v0);
         }
         for (uint32_t k = k0 + nth; k < e; k += nth) {
             uint32_t i = c.bRows[k];
@@ -521,9 +524,9 @@ __device__ __forceinline__ void eliminate(const DevCell& c, uint32_t tid, uint32
                 int2 term = c.bTerms[t];
                 v -= M[term.x] * c.VMid[term.y];
             }
-            v /= M[i];
+            v = quotient(v, M[i]);
             c.VMid[i] = v;
-            c.V[i] = 2 * v - c.V[i];
+            c.V[i] = __fma_rn(2.0, v, -c.V[i]);
         }
         levelSync<WARP>();
     }
@@ -535,16 +538,16 @@ __device__ __forceinline__ void poolStep(const DevCell& c, uint32_t p) {
     for (uint32_t f = c.feedPtr[p]; f < c.feedPtr[p + 1]; ++f) {
         uint32_t q = c.feedChan[f];
         uint32_t ic = c.chanCompt[q];
-        double v = c.caAdvance == 1 ? c.VMid[ic] : (2 * c.VMid[ic] - c.V[ic]);
+        const double v = c.caAdvance == 1 ? c.VMid[ic] : __fma_rn(2.0, c.VMid[ic], -c.V[ic]);
         act += c.Gk[q] * (c.Ek[q] - v);
     }
     double cc = c.f1[p] * c.c[p] + c.f2[p] * act;
     double ca = c.CaBasal[p] + cc;
-    if (c.ceil[p] > 0 && ca > c.ceil[p]) {
+    if (lessThan(0.0, c.ceil[p]) && lessThan(c.ceil[p], ca)) {
         ca = c.ceil[p];
         cc = ca - c.CaBasal[p];
     }
-    if (ca < c.floor_[p]) {
+    if (lessThan(ca, c.floor_[p])) {
         ca = c.floor_[p];
         cc = ca - c.CaBasal[p];
     }
@@ -652,7 +655,7 @@ __global__ void __launch_bounds__(256, 1) hsStepFp64(DevCell c, uint32_t nsteps)
 // them.
 __device__ __forceinline__ void waveUpdate(const DevCell& c, double* M, uint32_t k) {
     const int4 x = c.fWaveOps[2 * k], y = c.fWaveOps[2 * k + 1];
-    const double q = M[y.x] / M[y.y];
+    const double q = quotient(M[y.x], M[y.y]);
     M[x.x] -= q * M[x.y];
     if (x.z >= 0) M[x.z] -= q * M[x.w];
 }
@@ -664,9 +667,9 @@ __device__ __forceinline__ void backRow(const DevCell& c, const double* M, uint3
         int2 term = c.bTerms[t];
         v -= M[term.x] * c.VMid[term.y];
     }
-    v /= M[i];
+    v = quotient(v, M[i]);
     c.VMid[i] = v;
-    c.V[i] = 2 * v - c.V[i];
+    c.V[i] = __fma_rn(2.0, v, -c.V[i]);
 }
 
 // The elimination of a cell stepped by a cluster.  A forward wave or a
@@ -855,25 +858,24 @@ __global__ void __launch_bounds__(256) hsBatchStepFp64(const DevCell* __restrict
 }
 
 __device__ void reinitGatesCompt(const DevCell& c, uint32_t ic) {
-    Row vRow = tableRow(c.V[ic], c.vMin, c.vMax, c.vDx, c.vCol);
+    const Row vRow = tableRow(c.V[ic], c.vMin, c.vMax, c.vDx, c.vRdx, c.vRows);
     for (uint32_t q = c.chanPtr[ic]; q < c.chanPtr[ic + 1]; ++q) {
-        int32_t s = c.stateOff[q];
+        const uint4 A = c.chanA[q];
+        uint32_t s = A.y;
         double C1, C2;
-        if (c.Xpow[q] > 0.0) {
-            tableLookup(c.vTab, c.vCol, c.colX[q], vRow, C1, C2);
+        if (A.x & 0xFu) {
+            tableLookup(c.vTab, c.vCol, (int32_t)A.z, vRow, C1, C2);
             c.state[s++] = C1 / C2;
         }
-        if (c.Ypow[q] > 0.0) {
-            tableLookup(c.vTab, c.vCol, c.colY[q], vRow, C1, C2);
+        if (A.x & 0xF0u) {
+            tableLookup(c.vTab, c.vCol, (int32_t)A.w, vRow, C1, C2);
             c.state[s++] = C1 / C2;
         }
-        if (c.Zpow[q] > 0.0) {
-            int32_t src = c.zSrc[q];
-            if (src >= 0) {
-                Row r = tableRow(c.ca[src], c.caMin, c.caMax, c.caDx, c.caCol);
-                tableLookup(c.caTab, c.caCol, c.colZ[q], r, C1, C2);
-            } else if (c.extCa[q] > 0) {
-                Row r = tableRow(c.extCa[q], c.caMin, c.caMax, c.caDx, c.caCol);
+        if (A.x & 0xF00u) {
+            const int32_t src = c.zSrc[q];
+            const double ca = src >= 0 ? c.ca[src] : c.extCa[q];
+            if (src >= 0 || ca > 0) {
+                const Row r = tableRow(ca, c.caMin, c.caMax, c.caDx, c.caRdx, c.caRows);
                 tableLookup(c.caTab, c.caCol, c.colZ[q], r, C1, C2);
             } else {
                 tableLookup(c.vTab, c.vCol, c.colZ[q], vRow, C1, C2);
