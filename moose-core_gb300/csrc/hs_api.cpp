@@ -443,19 +443,23 @@ int hs_process_group(HsSolver* const* solvers, uint32_t n, uint32_t nsteps) {
     // members by the CTAs that step them: one launch per class, on the
     // stream of the class's first member (the clusters first: they need
     // whole free SM groups)
-    std::vector<std::vector<uint32_t>> cls(9);
+    // (of one CTA each, those whose matrix lets two CTAs share an SM first)
+    const uint32_t room = fp64MatrixRoom();
+    std::vector<std::vector<uint32_t>> cls(10);
     for (uint32_t k = 0; k < n; ++k) {
         HsSolver* s = solvers[k];
         int rc = flushEvents(s);
         if (!rc) rc = flushWrites(s);
         if (rc) return rc;
         arenaMoved(s);
-        cls[stepCtas(s)].push_back(k);
+        const uint32_t ctas = stepCtas(s);
+        cls[ctas == 1 && s->dc.smWords <= room / 2 - 512 ? 1 : ctas + 1].push_back(k);
     }
     cudaError_t e = cudaSuccess;
-    for (uint32_t ctas = 8; ctas >= 1 && e == cudaSuccess; --ctas) {
-        const std::vector<uint32_t>& m = cls[ctas];
+    for (uint32_t k9 = 9; k9 >= 1 && e == cudaSuccess; --k9) {
+        const std::vector<uint32_t>& m = cls[k9];
         if (m.empty()) continue;
+        const uint32_t ctas = k9 == 1 ? 1 : k9 - 1;
         cudaStream_t gst = solvers[m[0]]->st;
         // The launch follows each member's work: what was queued on its own
         // stream since its last group launch (an event there) and the
@@ -463,9 +467,11 @@ int hs_process_group(HsSolver* const* solvers, uint32_t n, uint32_t nsteps) {
         // that repeats on the same streams, with nothing queued between
         // its calls, needs neither: stream order covers it.
         std::vector<DevCell> cells(m.size());
+        uint32_t words = 0;
         for (size_t k = 0; k < m.size() && e == cudaSuccess; ++k) {
             HsSolver* s = solvers[m[k]];
             cells[k] = s->dc;
+            if (s->dc.smWords <= room) words = std::max(words, s->dc.smWords);
             if (s->st != gst && s->queued) {
                 if (!s->evQueued) e = cudaEventCreateWithFlags(&s->evQueued, cudaEventDisableTiming);
                 if (e == cudaSuccess) e = cudaEventRecord(s->evQueued, s->st);
@@ -478,7 +484,7 @@ int hs_process_group(HsSolver* const* solvers, uint32_t n, uint32_t nsteps) {
         // (a copy from pageable memory has read `cells` when it returns)
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(dCells, cells.data(), m.size() * sizeof(DevCell), cudaMemcpyHostToDevice, gst);
-        if (e == cudaSuccess) e = launchGroupStepFp64(dCells, (uint32_t)m.size(), ctas, nsteps, gst);
+        if (e == cudaSuccess) e = launchGroupStepFp64(dCells, (uint32_t)m.size(), ctas, words, nsteps, gst);
         if (dCells) cudaFreeAsync(dCells, gst);
         auto done = std::make_shared<HsGroupDone>();
         done->st = gst;
@@ -940,6 +946,9 @@ int installRecording(HsSolver* s, std::vector<uint32_t>&& rows, uint32_t stride,
         return cudaErr(e, "record");
     }
     s->dc.nRec = n;
+    s->dc.recChan = 0;
+    for (uint32_t r : s->recHost)
+        if ((r >> kRecShift) == kRecIk || (r >> kRecShift) == kRecGk) s->dc.recChan = 1;
     s->dc.recLd = n;
     s->dc.recStride = stride;
     s->dc.recCap = capacity;

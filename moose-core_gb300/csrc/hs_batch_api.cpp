@@ -147,10 +147,11 @@ struct HsBatch {
     uint32_t elimWarps = 4;      // mixed: eliminator warps of the split step (0: no split)
     uint32_t waitRounds = 1u << 24;   // mixed: sleep rounds of one bounded wait (~128 ns each)
     bool useGraph = true;
-    uint32_t nWarps = 0, nCtas = 0;
-    uint32_t *dWarpPtr = nullptr, *dWarpCells = nullptr;
-    uint32_t *dCtaCellPtr = nullptr, *dCtaCells = nullptr;   // FP64: cells stepped by a whole CTA
-    uint32_t nCtaWhole = 0;
+    uint32_t nCtas = 0;
+    // FP64: one block per SM of nTeams teams (threads_per_cta threads each,
+    // ctas_per_sm of them); cells stepped by a whole block, and by a team
+    uint32_t nBlocks = 0, nTeams = 0, batchWords = 0;
+    uint32_t *dWholePtr = nullptr, *dWholeCells = nullptr, *dTeamPtr = nullptr, *dTeamCells = nullptr;
     // mixed: forests per CTA, shared-memory forest capacity
     uint32_t *dCtaPtr = nullptr, *dCtaForests = nullptr;
     uint32_t mixCap = 0, mixSmem = 0;
@@ -233,8 +234,8 @@ namespace {
 
 cudaError_t launchStep(HsBatch* b, uint32_t k) {
     if (b->precision == HS_PREC_FP64)
-        return launchBatchStepFp64(b->dDcs, b->dWarpPtr, b->dWarpCells, b->nWarps, b->dCtaCellPtr, b->dCtaCells, k,
-                                   b->threadsPerCta, b->st);
+        return launchBatchStepFp64(b->dDcs, b->dWholePtr, b->dWholeCells, b->dTeamPtr, b->dTeamCells, b->nBlocks,
+                                   b->nTeams, b->threadsPerCta, b->batchWords, k, b->st);
     const uint32_t ew = b->elimWarps && b->threadsPerCta > 32 * b->elimWarps ? b->elimWarps : 0;
     b->mb.waitRounds = b->waitRounds;
     if (b->clusterCtas > 1) {
@@ -249,14 +250,15 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
                                  b->mixCap, ew, k, b->st);
 }
 
-// Packing of the FP64 batch into one wave of CTAs (as many per SM as the
-// kernel's registers allow, at most ctas_per_sm).  A warp steps its cells
-// one after the other, so a cell costing more than the balanced load of one
-// warp would bound the step by itself: such cells are stepped by a whole
-// CTA instead (its warps share each compartment loop and each elimination
-// level, as in the drop-in), packed longest first over enough CTAs to carry
-// their load; the other cells are packed longest first over the remaining
-// CTAs and then over their warps.
+// Packing of the FP64 batch: one block per SM, in teams (hsBatchStepFp64).
+// A step of a cell costs FP64 pipe time, which the cells of a block share, and
+// latency, the chains of its elimination, which a team spends alone (estimates
+// in cycles, from the pipe's 76 cycles per warp instruction and sub-partition
+// and ~650 cycles measured per wave or level).  Cells go to the blocks longest
+// first by pipe time.  In a block, the k largest cells are stepped by the
+// whole block one after the other and the others by the teams side by side;
+// k is the one with the least estimated time, and at least covers the cells
+// whose matrix does not fit a team's share of the shared memory.
 int repack(HsBatch* b) {
     if (b->gexec) {
         cudaGraphExecDestroy(b->gexec);
@@ -265,104 +267,83 @@ int repack(HsBatch* b) {
     if (b->precision != HS_PREC_FP64) return HS_OK;
     b->packBuf.freeAll();
     b->packBuf.err = cudaSuccess;
-    const uint32_t warpsPerCta = b->threadsPerCta / 32;
-    const int fit = fp64BatchCtasPerSm(b->threadsPerCta);
-    const uint32_t cps = std::max<uint32_t>(1, fit > 0 ? std::min<uint32_t>(b->ctasPerSm, (uint32_t)fit) : b->ctasPerSm);
-    b->nCtas = std::max<uint32_t>(1, b->nSm * cps);
-    b->nWarps = b->nCtas * warpsPerCta;
-    std::vector<double> cost(b->nCells);
-    double total = 0;
-    for (uint32_t c = 0; c < b->nCells; ++c) {
+    const uint32_t nC = b->nCells, warps = b->threadsPerCta / 32;
+    b->nTeams = std::max<uint32_t>(1, std::min<uint32_t>(b->ctasPerSm, kBatchThreads / b->threadsPerCta));
+    b->nBlocks = std::max(1, b->nSm);
+    b->nCtas = b->nBlocks * b->nTeams;
+    b->batchWords = fp64BatchWords(b->nTeams);
+    const uint32_t share = b->batchWords / b->nTeams;
+    std::vector<double> pipe(nC), chain(nC);
+    for (uint32_t c = 0; c < nC; ++c) {
         const CellPlan& P = b->plans[c];
-        cost[c] = P.N + 0.3 * P.C + 0.5 * P.S + 2.0 * (P.fLevelPtr.size() + P.bLevelPtr.size());
-        total += cost[c];
+        const double rows = std::ceil(P.N / 32.0), waves = P.fWavePtr.empty() ? 0.0 : P.fWavePtr.size() - 1.0;
+        const double ops = 20.0 + (13.0 * P.G + 5.0 * P.C + 45.0 * P.K2 + 9.0 * P.P) / P.N;
+        pipe[c] = 76.0 / 4 * (rows * (ops + 12.0) + 10.0 * P.S / 32 + 6.0 * P.fWaveOps.size() / 32 + 6.0 * waves +
+                              5.0 * P.bLevelPtr.size());
+        chain[c] = 650.0 * ((waves > 0 ? waves : (double)P.fLevelPtr.size()) + P.bLevelPtr.size()) + 4000.0;
     }
-    std::vector<uint32_t> order(b->nCells);
-    for (uint32_t c = 0; c < b->nCells; ++c) order[c] = c;
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return cost[x] > cost[y]; });
-    // a whole CTA steps a cell at a fraction of its warps' combined rate
-    // (a barrier per elimination level, levels narrower than the CTA); this
-    // estimate of the fraction only decides which cells get whole CTAs
-    constexpr double kCtaEfficiency = 0.6;
-    const double ctaRate = warpsPerCta > 1 ? warpsPerCta * kCtaEfficiency : 1.0;
-    // the k costliest cells on m whole CTAs, the rest over the warps of the
-    // other CTAs: estimated step time, the larger of the two groups' (each
-    // bounded below by its largest cell and by its load spread evenly)
-    const uint32_t nC = b->nCells;
-    std::vector<double> prefix(nC + 1, 0.0);
-    for (uint32_t i = 0; i < nC; ++i) prefix[i + 1] = prefix[i] + cost[order[i]];
-    uint32_t bestK = 0, bestM = 0;
-    double bestT = std::max(nC ? cost[order[0]] : 0.0, total / b->nWarps);
-    if (warpsPerCta > 1 && b->nCtas > 1)
-        for (uint32_t k = 1; k <= nC; ++k) {
-            const double sb = prefix[k], ss = total - sb;
-            const double bigMax = cost[order[0]] / ctaRate, smallMax = k < nC ? cost[order[k]] : 0.0;
-            // m balancing sb / (m ctaRate) against ss / ((nCtas - m) warpsPerCta)
-            const double mf = k < nC ? b->nCtas * sb / ctaRate / (sb / ctaRate + ss / warpsPerCta) : b->nCtas;
-            for (int dm = 0; dm <= 1; ++dm) {
-                uint32_t m = (uint32_t)std::floor(mf) + dm;
-                m = std::max<uint32_t>(1, std::min<uint32_t>(m, k < nC ? b->nCtas - 1 : b->nCtas));
-                m = std::min<uint32_t>(m, k);
-                const double tb = std::max(bigMax, sb / (m * ctaRate));
-                const double ts = k < nC ? std::max(smallMax, ss / ((double)(b->nCtas - m) * warpsPerCta)) : 0.0;
-                const double t = std::max(tb, ts);
-                if (t < bestT) {
-                    bestT = t;
-                    bestK = k;
-                    bestM = m;
-                }
-            }
-        }
-    std::vector<uint32_t> big(order.begin(), order.begin() + bestK), small(order.begin() + bestK, order.end());
-    const uint32_t mCta = bestM;
+    auto alone = [&](uint32_t c, uint32_t w) { return pipe[c] * 4.0 / std::min<uint32_t>(4, w) + chain[c]; };
+    std::vector<uint32_t> order(nC);
+    for (uint32_t c = 0; c < nC; ++c) order[c] = c;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return pipe[x] > pipe[y]; });
     using Item = std::pair<double, uint32_t>;
-    std::vector<std::vector<uint32_t>> ctaWhole(b->nCtas);
+    using Queue = std::priority_queue<Item, std::vector<Item>, std::greater<Item>>;
+    std::vector<std::vector<uint32_t>> bins(b->nBlocks);
     {
-        std::priority_queue<Item, std::vector<Item>, std::greater<Item>> q;
-        for (uint32_t k = 0; k < mCta; ++k) q.push({0.0, k});
-        for (uint32_t c : big) {
+        Queue q;
+        for (uint32_t k = 0; k < b->nBlocks; ++k) q.push({0.0, k});
+        for (uint32_t c : order) {
             Item it = q.top();
             q.pop();
-            ctaWhole[it.second].push_back(c);
-            q.push({it.first + cost[c] / ctaRate, it.second});
+            bins[it.second].push_back(c);
+            q.push({it.first + pipe[c] + 0.3 * chain[c], it.second});
         }
     }
-    std::priority_queue<Item, std::vector<Item>, std::greater<Item>> cta;
-    for (uint32_t k = mCta; k < b->nCtas; ++k) cta.push({0.0, k});
-    std::vector<std::vector<uint32_t>> ctaCells(b->nCtas);
-    for (uint32_t c : small) {
-        Item it = cta.top();
-        cta.pop();
-        ctaCells[it.second].push_back(c);
-        // a CTA runs its warps concurrently: its load is spread over them
-        cta.push({it.first + cost[c] / warpsPerCta, it.second});
-    }
-    std::vector<std::vector<uint32_t>> warpCells(b->nWarps);
-    for (uint32_t k = 0; k < b->nCtas; ++k) {
-        std::priority_queue<Item, std::vector<Item>, std::greater<Item>> wq;
-        for (uint32_t w = 0; w < warpsPerCta; ++w) wq.push({0.0, k * warpsPerCta + w});
-        for (uint32_t c : ctaCells[k]) {
-            Item it = wq.top();
-            wq.pop();
-            warpCells[it.second].push_back(c);
-            wq.push({it.first + cost[c], it.second});
+    std::vector<uint32_t> wholePtr(1, 0), wholeCells, teamPtr(1, 0), teamCells;
+    for (uint32_t k = 0; k < b->nBlocks; ++k) {
+        const std::vector<uint32_t>& cells = bins[k];
+        const uint32_t n = (uint32_t)cells.size();
+        uint32_t least = 0;
+        for (uint32_t i = 0; i < n; ++i)
+            if (2 * (uint64_t)b->plans[cells[i]].N + b->plans[cells[i]].H > share) least = i + 1;
+        // the cells after the first `k0` to the teams, longest first; estimated time
+        std::vector<std::vector<uint32_t>> best, lists;
+        double bestT = 0;
+        uint32_t bestK = n;
+        for (uint32_t k0 = least; k0 <= n; ++k0) {
+            double t = 0, sum = 0, longest = 0;
+            for (uint32_t i = 0; i < k0; ++i) t += alone(cells[i], warps * b->nTeams);
+            lists.assign(b->nTeams, {});
+            Queue q;
+            for (uint32_t m = 0; m < b->nTeams; ++m) q.push({0.0, m});
+            for (uint32_t i = k0; i < n; ++i) {
+                Item it = q.top();
+                q.pop();
+                lists[it.second].push_back(cells[i]);
+                const double end = it.first + alone(cells[i], warps);
+                sum += pipe[cells[i]];
+                longest = std::max(longest, end);
+                q.push({end, it.second});
+            }
+            t += std::max(sum, longest);
+            if (k0 == least || t < bestT) {
+                bestT = t;
+                bestK = k0;
+                best = lists;
+            }
+        }
+        wholeCells.insert(wholeCells.end(), cells.begin(), cells.begin() + bestK);
+        wholePtr.push_back((uint32_t)wholeCells.size());
+        best.resize(b->nTeams);
+        for (const auto& l : best) {
+            teamCells.insert(teamCells.end(), l.begin(), l.end());
+            teamPtr.push_back((uint32_t)teamCells.size());
         }
     }
-    std::vector<uint32_t> ptr(b->nWarps + 1, 0), cells;
-    for (uint32_t w = 0; w < b->nWarps; ++w) {
-        ptr[w + 1] = ptr[w] + (uint32_t)warpCells[w].size();
-        cells.insert(cells.end(), warpCells[w].begin(), warpCells[w].end());
-    }
-    std::vector<uint32_t> cptr(b->nCtas + 1, 0), ccells;
-    for (uint32_t k = 0; k < b->nCtas; ++k) {
-        cptr[k + 1] = cptr[k] + (uint32_t)ctaWhole[k].size();
-        ccells.insert(ccells.end(), ctaWhole[k].begin(), ctaWhole[k].end());
-    }
-    b->dWarpPtr = b->packBuf.up(ptr, b->st);
-    b->dWarpCells = b->packBuf.up(cells, b->st);
-    b->dCtaCellPtr = b->packBuf.up(cptr, b->st);
-    b->dCtaCells = b->packBuf.up(ccells, b->st);
-    b->nCtaWhole = mCta;
+    b->dWholePtr = b->packBuf.up(wholePtr, b->st);
+    b->dWholeCells = b->packBuf.up(wholeCells, b->st);
+    b->dTeamPtr = b->packBuf.up(teamPtr, b->st);
+    b->dTeamCells = b->packBuf.up(teamCells, b->st);
     if (b->packBuf.err == cudaSuccess) b->packBuf.err = cudaStreamSynchronize(b->st);
     if (b->packBuf.err != cudaSuccess) return cerr(b->packBuf.err, "batch packing");
     return HS_OK;

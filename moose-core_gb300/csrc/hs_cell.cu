@@ -52,6 +52,112 @@ uint32_t powCode(double p) {
     return kPowGeneral;
 }
 
+// The sweeps' programs with 16-bit entries for a matrix in shared memory
+// (DevCell::fW, bW, ...); false where they do not fit the encoding.
+struct Compact {
+    std::vector<uint4> fW, bW, fLane, bLane;
+    std::vector<uint32_t> bX;
+    std::vector<uint2> fSeg, bSeg;
+    bool split = true;
+};
+
+bool compactPrograms(const CellPlan& P, Compact& C) {
+    const uint32_t N = P.N, offBase = 2 * N + P.H, kNone = 0xFFFFu, kOff = 0xFFFEu;
+    if (offBase >= kOff) return false;
+    auto offOf = [&](uint32_t row) {
+        uint64_t u = 0;
+        if (row < N) std::memcpy(&u, &P.off[row], 8);
+        return make_uint2((uint32_t)u, (uint32_t)(u >> 32));
+    };
+    for (const FwdPair& f : P.fWaveOps) {
+        uint32_t row = 0xFFFFFFFFu, l = (uint32_t)f.l;
+        if (l >= offBase) {
+            row = l - offBase;
+            l = kOff;
+        }
+        bool ok = true;
+        auto entry = [&](int32_t a) {
+            if ((uint32_t)a < offBase) return (uint32_t)a;
+            ok = ok && (uint32_t)a - offBase == row;      // the update's own off-diagonal
+            return kOff;
+        };
+        const uint32_t a1 = entry(f.a1), a2 = f.t2 >= 0 ? entry(f.a2) : 0u, t2 = f.t2 >= 0 ? (uint32_t)f.t2 : kNone;
+        if (!ok) return false;
+        const uint2 o = offOf(row);
+        C.fW.push_back(make_uint4((uint32_t)f.t1 | a1 << 16, t2 | a2 << 16, l | (uint32_t)f.p << 16, 0));
+        C.fW.push_back(make_uint4(o.x, o.y, 0, 0));
+        if (f.t2 >= 0) {
+            // two lanes may change an update's entries where neither reads
+            // what the other writes
+            for (int32_t r : {f.l, f.p, f.a1, f.a2})
+                if (r == f.t1 || r == f.t2) C.split = false;
+            if (f.t1 == f.t2) C.split = false;
+        }
+    }
+    for (size_t k = 0; k < P.bRows.size(); ++k) {
+        const uint32_t i = P.bRows[k], t0 = P.bTermPtr[k], n = P.bTermPtr[k + 1] - t0;
+        if (n > 0xFFFFu) return false;
+        uint32_t term[4] = {kNone, 0, 0, 0}, row = N;
+        const uint32_t x0 = (uint32_t)C.bX.size();
+        for (uint32_t t = 0; t < n; ++t) {
+            const BwdTerm& x = P.bTerms[t0 + t];
+            uint32_t co = (uint32_t)x.coef;
+            if (co >= offBase) {
+                if (t || co - offBase != i) return false;
+                co = kOff;
+                row = i;
+            }
+            const uint32_t w = co | (uint32_t)x.src << 16;
+            if (t < 4) term[t] = w;
+            else C.bX.push_back(w);
+        }
+        const uint2 o = offOf(row);
+        C.bW.push_back(make_uint4(i | n << 16, term[0], term[1], term[2]));
+        C.bW.push_back(make_uint4(o.x, o.y, term[3], x0));
+    }
+    auto grow = [](std::vector<uint2>& seg, uint32_t kind, uint32_t first) {
+        if (!seg.empty() && (seg.back().x & kSegKind) == kind && kind != kSegRun) ++seg.back().x;
+        else seg.push_back(make_uint2(1u | kind, first));
+    };
+    const uint32_t W = P.fWavePtr.empty() ? 0 : (uint32_t)P.fWavePtr.size() - 1;
+    const uint4 idle = make_uint4(kNone, 0, 0, 0);
+    for (uint32_t w = 0; w < W; ++w) {
+        const uint32_t b = P.fWavePtr[w], n = P.fWavePtr[w + 1] - b;
+        if (!C.split || n > 16) {
+            grow(C.fSeg, 0, w);
+            continue;
+        }
+        grow(C.fSeg, kSegNarrow, (uint32_t)C.fLane.size());
+        for (uint32_t lane = 0; lane < 32; ++lane) {
+            if (lane >= 2 * n) {
+                C.fLane.push_back(idle);
+                continue;
+            }
+            const uint4 d = C.fW[2 * (b + lane / 2)], o = C.fW[2 * (b + lane / 2) + 1];
+            C.fLane.push_back(make_uint4(lane & 1 ? d.y : d.x, d.z, o.x, o.y));
+        }
+    }
+    const uint32_t L = (uint32_t)P.bLevelPtr.size() - 1;
+    for (uint32_t l = 0; l < L; ++l) {
+        if (P.bRun[l]) {
+            C.bSeg.push_back(make_uint2(P.bRun[l] | kSegRun, P.bRunRow[l]));
+            l += P.bRun[l] - 1;
+            continue;
+        }
+        const uint32_t b = P.bLevelPtr[l], n = P.bLevelPtr[l + 1] - b;
+        if (n > 32) {
+            grow(C.bSeg, 0, l);
+            continue;
+        }
+        grow(C.bSeg, kSegNarrow, (uint32_t)C.bLane.size() / 2);
+        for (uint32_t lane = 0; lane < 32; ++lane) {
+            C.bLane.push_back(lane < n ? C.bW[2 * (b + lane)] : idle);
+            C.bLane.push_back(lane < n ? C.bW[2 * (b + lane) + 1] : idle);
+        }
+    }
+    return true;
+}
+
 }  // namespace
 
 cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCap,
@@ -103,6 +209,22 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.fWaves = P.fWavePtr.empty() ? 0 : (uint32_t)P.fWavePtr.size() - 1;
     c.fWavePtr = u.put(P.fWavePtr);
     c.fWaveOps = reinterpret_cast<const int4*>(u.put(P.fWaveOps));
+    {
+        Compact C;
+        const bool compact = compactPrograms(P, C);
+        if (!compact) C = Compact();
+        c.smWords = compact ? 2 * N + H : 0;
+        c.fSplit = C.split;
+        c.fW = u.put(C.fW);
+        c.bW = u.put(C.bW);
+        c.bX = u.put(C.bX);
+        c.fLane = u.put(C.fLane);
+        c.bLane = u.put(C.bLane);
+        c.fSeg = u.put(C.fSeg);
+        c.bSeg = u.put(C.bSeg);
+        c.nfSeg = (uint32_t)C.fSeg.size();
+        c.nbSeg = (uint32_t)C.bSeg.size();
+    }
     c.Gbar = u.put(P.Gbar);
     c.Ek = u.put(P.Ek);
     c.Xpow = u.put(P.Xpow);
@@ -127,6 +249,17 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         for (uint32_t ic = 0; ic < N; ++ic)
             for (uint32_t q = P.chanPtr[ic]; q < P.chanPtr[ic + 1]; ++q) cc[q] = ic;
         c.chanCompt = u.put(cc);
+        std::vector<uint32_t> poolCompt(P.P);
+        for (uint32_t ic = 0; ic < N; ++ic)
+            for (uint32_t p = P.poolPtr[ic]; p < P.poolPtr[ic + 1]; ++p) poolCompt[p] = ic;
+        bool local = true;
+        for (uint32_t p = 0; p < P.P; ++p)
+            for (uint32_t f = P.feedPtr[p]; f < P.feedPtr[p + 1]; ++f) local = local && cc[P.feedChan[f]] == poolCompt[p];
+        for (uint32_t q = 0; q < P.C; ++q)
+            local = local && (P.zSrc[q] < 0 || poolCompt[P.zSrc[q]] == cc[q]);
+        for (uint32_t k = 0; k < P.K2; ++k)
+            for (int32_t p : {P.c2dConc1[k], P.c2dConc2[k]}) local = local && (p < 0 || poolCompt[p] == P.c2dCompt[k]);
+        c.local = local;
     }
     c.c = u.put(P.c0);
     c.CaBasal = u.put(P.CaBasal);

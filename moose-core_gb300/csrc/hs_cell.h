@@ -47,7 +47,8 @@ void synConsts(const CellPlan& P, double dt, double* out);
 
 cudaError_t launchStepFp64(const DevCell& c, uint32_t nsteps, cudaStream_t st);
 cudaError_t launchStepFp64Cluster(const DevCell& c, uint32_t ctas, uint32_t nsteps, cudaStream_t st);
-cudaError_t launchGroupStepFp64(const DevCell* cells, uint32_t n, uint32_t ctas, uint32_t nsteps,
+uint32_t fp64MatrixRoom();      // doubles of shared memory a drop-in CTA has for its matrix
+cudaError_t launchGroupStepFp64(const DevCell* cells, uint32_t n, uint32_t ctas, uint32_t words, uint32_t nsteps,
                                 cudaStream_t st);
 // The queued field writes of a drop-in solver, one thread each (distinct
 // addresses).
@@ -64,11 +65,11 @@ cudaError_t launchSpikeCountsFp64(const DevCell* cells, uint32_t nCells, uint32_
 cudaError_t launchGatherSpikes(const DevCell* cells, const uint32_t* srcGen, const float* srcTime, uint32_t cap,
                                uint32_t nCells, const uint32_t* off, uint32_t* gen, double* time,
                                cudaStream_t st);
-cudaError_t launchBatchStepFp64(const DevCell* cells, const uint32_t* warpCellPtr,
-                                const uint32_t* warpCells, uint32_t nWarps, const uint32_t* ctaCellPtr,
-                                const uint32_t* ctaCells, uint32_t nsteps, uint32_t threadsPerCta,
+constexpr uint32_t kBatchThreads = 512;     // most threads of the FP64 batch's CTA (128 registers each)
+uint32_t fp64BatchWords(uint32_t teams);    // doubles of shared memory it has for matrices
+cudaError_t launchBatchStepFp64(const DevCell* cells, const uint32_t* wholePtr, const uint32_t* wholeCells,
+                                const uint32_t* teamPtr, const uint32_t* teamCells, uint32_t nBlocks,
+                                uint32_t teams, uint32_t teamThreads, uint32_t words, uint32_t nsteps,
                                 cudaStream_t st);
-// CTAs of the FP64 batch kernel that fit on one SM at once (0 if unknown).
-int fp64BatchCtasPerSm(uint32_t threadsPerCta);
 
 }  // namespace hsg

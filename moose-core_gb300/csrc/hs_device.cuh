@@ -29,6 +29,9 @@ constexpr uint32_t kDifState = 13;
 constexpr uint32_t kRecShift = 28;
 constexpr uint32_t kRecVm = 0, kRecIk = 1, kRecGk = 2, kRecCa = 3;
 
+// kinds of segments of the sweeps (DevCell::fSeg, bSeg)
+constexpr uint32_t kSegNarrow = 0x80000000u, kSegRun = 0x40000000u, kSegKind = kSegNarrow | kSegRun;
+
 struct DevCtl {
     unsigned long long nSteps;   // steps since reinit
     uint32_t stimPtr;
@@ -54,6 +57,23 @@ struct DevCell {
     const uint32_t *bLevelPtr, *bRows, *bTermPtr;
     const int2* bTerms;
     const uint32_t *fRun, *fRunRow, *bRun, *bRunRow;   // cable runs per level
+    // the sweeps in shared memory (16-bit entries; smWords = 2N + H doubles, 0:
+    // not built).  fW, two uint4 per fused update: {t1 | a1 << 16, t2 | a2 << 16,
+    // l | p << 16, -}, {off-diagonal, -}.  bW, two per row of bRows: {row |
+    // terms << 16, coefficient | source << 16 of the first three terms},
+    // {off-diagonal, fourth term, first of the others in bX}.  fLane, bLane:
+    // the narrow waves' and levels' entries one per lane, 32 per wave (one
+    // uint4 {t | a << 16, l | p << 16, off-diagonal}) or level (two, as bW).
+    // fSeg, bSeg: segments {count | kind, first wave or level; narrow: first
+    // of fLane, of bLane / 2; run: first row}
+    uint32_t smWords;
+    uint32_t fSplit;             // an update's two entries may be changed by two lanes
+    uint32_t local;              // pools and HHChannel2Ds read and feed their own compartment only
+    uint32_t recChan;            // a channel's Gk or Ik is recorded
+    const uint4 *fW, *bW, *fLane, *bLane;
+    const uint2 *fSeg, *bSeg;
+    uint32_t nfSeg, nbSeg;
+    const uint32_t* bX;
     const uint32_t* fWavePtr;
     const int4* fWaveOps;        // per fused update: {t1, a1, t2, a2}, {l, p, -, -}
     // channels
@@ -167,20 +187,26 @@ __device__ __forceinline__ void tableLookup(const double* T, uint32_t nCol, int3
     C2 = b.x + b.y * r.frac;
 }
 
-__device__ __forceinline__ double gateStep(double x, double C1, double C2, double dt, bool inst) {
+// hdt = dt / 2 (exact)
+__device__ __forceinline__ double gateStep(double x, double C1, double C2, double dt, double hdt, bool inst) {
     if (inst) return plainQuotient(C1, C2);
-    const double temp = 1.0 + dt / 2.0 * C2;
+    const double temp = 1.0 + hdt * C2;
     return quotient(x * (2.0 - temp) + dt * C1, temp);
 }
+
+// Keeps the compiler from running a conditional FP64 operation
+// unconditionally and selecting: a branch costs less.
+__device__ __forceinline__ void keepBranch() { asm volatile(""); }
 
 // x to the power of `code`; `p` holds a general power.
 __device__ __forceinline__ double takePower(double x, uint32_t code, const double* p) {
     if (code == 1) return x;
-    if (code == 2) return x * x;
-    if (code == 3) return x * x * x;
-    if (code == 4) {
+    if (code <= 4) {
+        keepBranch();
         const double y = x * x;
-        return y * y;
+        if (code == 2) return y;
+        keepBranch();
+        return y * (code == 4 ? y : x);
     }
     if (lessThan(0.0, x)) return exp(*p * log(x));
     return 0.0;

@@ -21,14 +21,21 @@
 
 namespace hsg {
 
-__device__ __forceinline__ uint32_t hiOf(double x) { return (uint32_t)__double2hiint(x); }
-__device__ __forceinline__ uint32_t loOf(double x) { return (uint32_t)__double2loint(x); }
+// A double's bits, by a move that the compiler does not see through: it would
+// turn integer tests on them (for a NaN, say) back into FP64 instructions.
+__device__ __forceinline__ long long bitsOf(double x) {
+    long long b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+    return b;
+}
+__device__ __forceinline__ uint32_t hiOf(double x) { return (uint32_t)((unsigned long long)bitsOf(x) >> 32); }
+__device__ __forceinline__ uint32_t loOf(double x) { return (uint32_t)bitsOf(x); }
 __device__ __forceinline__ double fromWords(uint32_t hi, uint32_t lo) { return __hiloint2double((int)hi, (int)lo); }
 
 // a < b and a <= b as IEEE has them: false with a NaN, -0 equal to +0.
 __device__ __forceinline__ bool compareKeys(double a, double b, long long& x, long long& y) {
-    x = __double_as_longlong(a);
-    y = __double_as_longlong(b);
+    x = bitsOf(a);
+    y = bitsOf(b);
     const long long top = 0x7FFFFFFFFFFFFFFFll;
     const bool ordered = (x & top) <= 0x7FF0000000000000ll && (y & top) <= 0x7FF0000000000000ll;
     if (x < 0) x = -(x & top);      // -0 and +0 both 0
@@ -51,18 +58,32 @@ __device__ __forceinline__ bool isZero(double x) { return ((hiOf(x) << 1) | loOf
 // quotient() does not take.
 static __device__ __noinline__ double plainQuotient(double a, double d) { return a / d; }
 
+// q if it is RN(a / d), else the plain division's result.  q is next to the
+// quotient, so a - d q is exact, and q is right if that is less than |d| half
+// a last place of q (a quarter on the lower side of a power of two, where
+// places are half as large; never equal).
+static __device__ __noinline__ double checkedQuotient(double a, double d, double q) {
+    const double r = __fma_rn(-d, q, a);
+    const unsigned long long top = 0x7FFFFFFFFFFFFFFFull, R = bitsOf(r) & top;
+    const bool below = ((bitsOf(r) ^ bitsOf(a)) >> 63) && ((unsigned long long)bitsOf(q) << 12) == 0ull;
+    const unsigned long long e = ((unsigned long long)bitsOf(q) & 0x7FF0000000000000ull) >> 52;
+    const unsigned long long half = (bitsOf(d) & top) - ((1023ull + 53ull + (below ? 1ull : 0ull) - e) << 52);
+    return R < half ? q : plainQuotient(a, d);
+}
+
 // RN(a / d).  With mantissas a', d' in [1, 2):
 //   y0 + y1 ~ 1 / d', qh + ql ~ a' / d' as sums of two floats, from the FP32
-//   reciprocal and the exact FP32 residual (relative error < 2^-44);
+//   reciprocal and the FP32 residual (relative error < 2^-43);
 //   Q = qh + ql as a double (integer addition of the low part),
 //   r = a - d Q, one fused operation: the remainder to 53 bits,
 //   q = RN(Q + r y0): before rounding off by less than 2^-13 of q's last
 //   place, so q is the correctly rounded quotient unless the sum lies within
 //   that of a midpoint between two doubles.
 // That case (the fraction of r / d in last places within 2^-10 of 1/2, about
-// one division in 500), a quotient next to a power of two (whose last place
-// changes there), a sum Q that leaves qh's binade, zeros, infinities, NaNs and exponents beyond +-383 take the
-// plain division.  The remainder test needs no exact tie: a quotient of two
+// one division in 500) and a quotient next to a power of two (whose last place
+// changes there; a saturated gate's is next to 1 at every step) are checked by
+// their remainder.  A sum Q that leaves qh's binade, zeros, infinities, NaNs
+// and exponents beyond +-383 take the plain division.  The remainder test needs no exact tie: a quotient of two
 // doubles is never halfway between two doubles of normal range.
 struct Recip {          // what a division needs of its divisor
     float y0, y1;
@@ -72,8 +93,9 @@ struct Recip {          // what a division needs of its divisor
 __device__ __forceinline__ float mantissa(uint32_t hi, uint32_t lo) {
     return __uint_as_float((__funnelshift_l(lo, hi, 3) & 0x007FFFFFu) | 0x3F800000u);
 }
+// the 29 bits below the mantissa's 24, cut to 23, at their weight
 __device__ __forceinline__ float mantissaTail(uint32_t lo) {
-    return (float)(int)(lo & 0x1FFFFFFFu) * 0x1p-52f;
+    return (__uint_as_float(((lo >> 6) & 0x007FFFFFu) | 0x3F800000u) - 1.0f) * 0x1p-23f;
 }
 
 __device__ __forceinline__ Recip recip(double d) {
@@ -97,8 +119,10 @@ __device__ __forceinline__ double quotient(double a, double d, const Recip& R) {
     ql = fmaf(fa, R.y1, ql);
     ql = fmaf(ta, R.y0, ql);
     const uint32_t qb = __float_as_uint(qh);
-    // ql in units of the last place of qh's double: 2^52 / 2^exponent(qh)
-    const int k = __float2int_rn(ql * __uint_as_float((306u << 23) - (qb & 0xFF800000u)));
+    // ql (below 2^-21.2 of qh) in units of 2^9 last places of qh's double, that
+    // is of 2^(exponent(qh) - 43): rounded to an integer by adding 1.5 * 2^23
+    const float kf = fmaf(ql, __uint_as_float((297u << 23) - (qb & 0xFF800000u)), 12582912.0f);
+    const int k = (__float_as_int(kf) - 0x4B400000) * 512;
     const uint32_t ea = ha & 0x7FF00000u, ed = hd & 0x7FF00000u, sgn = (ha ^ hd) & 0x80000000u;
     unsigned long long Qb = ((unsigned long long)((qb >> 3) + 0x38000000u) << 32) | (qb << 29);
     Qb += (long long)k;
@@ -120,7 +144,8 @@ __device__ __forceinline__ double quotient(double a, double d, const Recip& R) {
     const bool edge = lq < 2048u && ((hiOf(q) + (lq < 1024u ? 1u : 0u)) & 0xFFFFFu) == 0u;
     // the integer sum crossed into another binade, whose last places differ
     const bool cross = (((uint32_t)(Qb >> 32) ^ ((qb >> 3) + 0x38000000u)) & 0x7FF00000u) != 0u;
-    if (!ok || near || edge || cross) return plainQuotient(a, d);
+    if (!ok || cross) return plainQuotient(a, d);
+    if (near || edge) return checkedQuotient(a, d, q);
     return q;
 }
 

@@ -217,12 +217,12 @@ __device__ __forceinline__ double depValue(uint32_t dep, double vm, double c1, d
     return dep == 0 ? vm : dep == 1 ? c1 : dep == 2 ? c2 : 0.0;
 }
 
-__device__ __forceinline__ void chan2dStep(const DevCell& c, uint32_t k) {
+// HHChannel2D k on the inputs vm, c1, c2; its Gk.
+__device__ __forceinline__ double chan2dStep(const DevCell& c, uint32_t k, double vm, double c1, double c2) {
     double g = c.c2dGbar[k];
     const uint32_t a = c.c2dA[k];
     if (a & 15u) {
         const int gi = c.c2dGate[k];
-        const double vm = c.c2dVm[k], c1 = c.c2dC1[k], c2 = c.c2dC2[k];
         const double x = depValue((a >> 4) & 15u, vm, c1, c2);
         const double y = depValue((a >> 8) & 15u, vm, c1, c2);
         double A, B;
@@ -241,16 +241,26 @@ __device__ __forceinline__ void chan2dStep(const DevCell& c, uint32_t k) {
         g *= takePower(X, a & 15u, c.c2dXpow + k);
     }
     const double mod = c.c2dMod[k];
-    c.c2dGk[k] = isOne(mod) ? g : g * mod;
+    if (!isOne(mod)) {
+        keepBranch();
+        g *= mod;
+    }
+    c.c2dGk[k] = g;
+    return g;
 }
 
 // ---- tick 6, per compartment: channels + matrix row -----------------------
 // Bound by the FP64 pipe (76 cycles per warp instruction and sub-partition):
 // the gates run in one loop over X, Y, Z, and what is not an operation of the
 // reference's arithmetic (compares, row indices, powers of 1, factors of 1)
-// is kept off that pipe.
-__device__ __forceinline__ void comptStep(const DevCell& c, uint32_t ic) {
-    double V = c.V[ic];
+// is kept off that pipe.  `first`: the launch's first step, the only one
+// with conductances and currents sent between process calls and with
+// HHChannel2D inputs that may differ from V and Ca (a field written since
+// they were sent).  `own2d`: the HHChannel2Ds of the compartment are stepped
+// here.  The row goes to M (diagonal at ic, right-hand side at N + ic).
+__device__ __forceinline__ void rowStep(const DevCell& c, uint32_t ic, double hdt, bool own2d, bool first, bool last,
+                                        double* M) {
+    const double V = c.V[ic];
     const Row vRow = tableRow(V, c.vMin, c.vMax, c.vDx, c.vRdx, c.vRows);
     double GkSum = 0.0, GkEkSum = 0.0;
     for (uint32_t q = c.chanPtr[ic]; q < c.chanPtr[ic + 1]; ++q) {
@@ -278,10 +288,14 @@ __device__ __forceinline__ void comptStep(const DevCell& c, uint32_t ic) {
                 }
                 double C1, C2;
                 tableLookup(T, nCol, col, r, C1, C2);
-                const double x = gateStep(c.state[s], C1, C2, c.dt, inst & (1 << g));
+                const double x = gateStep(c.state[s], C1, C2, c.dt, hdt, inst & (1 << g));
                 c.state[s++] = x;
-                const double pw = takePower(x, code, (g == 0 ? c.Xpow : g == 1 ? c.Ypow : c.Zpow) + q);
-                fraction = one ? pw : fraction * pw;
+                double pw = takePower(x, code, (g == 0 ? c.Xpow : g == 1 ? c.Ypow : c.Zpow) + q);
+                if (!one) {
+                    keepBranch();
+                    pw = fraction * pw;
+                }
+                fraction = pw;
                 one = false;
             }
             col = (int32_t)A.w;
@@ -292,253 +306,65 @@ __device__ __forceinline__ void comptStep(const DevCell& c, uint32_t ic) {
         GkEkSum += gk * c.Ek[q];
     }
     // external conductances in tick-4 send order (HSolve::addGkEk)
-    double eg = c.ext[2 * ic], ege = c.ext[2 * ic + 1];
+    double eg = 0.0, ege = 0.0, inj = 0.0;
+    if (first) {
+        eg = c.ext[2 * ic];
+        ege = c.ext[2 * ic + 1];
+        inj = c.injVarying[ic];
+        c.ext[2 * ic] = 0.0;
+        c.ext[2 * ic + 1] = 0.0;
+        c.injVarying[ic] = 0.0;
+    }
     for (uint32_t k = c.extPtr[ic]; k < c.extPtr[ic + 1]; ++k) {
-        int32_t code = c.extList[k];
-        double gk = code >= 0 ? c.c2dGk[code] : c.synGk[-code - 1];
-        double ek = code >= 0 ? c.c2dEk[code] : c.synEk[-code - 1];
+        const int32_t code = c.extList[k];
+        double gk, ek;
+        if (code >= 0) {
+            ek = c.c2dEk[code];
+            if (!own2d) {
+                gk = c.c2dGk[code];
+            } else {
+                const int32_t p1 = c.c2dConc1[code], p2 = c.c2dConc2[code];
+                const bool sent = first;
+                gk = chan2dStep(c, code, sent ? c.c2dVm[code] : V, sent || p1 < 0 ? c.c2dC1[code] : c.ca[p1],
+                                sent || p2 < 0 ? c.c2dC2[code] : c.ca[p2]);
+            }
+        } else {
+            gk = c.synGk[-code - 1];
+            ek = c.synEk[-code - 1];
+        }
         eg += gk;
         ege += gk * ek;
     }
-    c.prevExt[2 * ic] = eg;
-    c.prevExt[2 * ic + 1] = ege;
+    if (last) {
+        c.prevExt[2 * ic] = eg;
+        c.prevExt[2 * ic + 1] = ege;
+    }
     // HSolveActive::updateMatrix
-    const uint32_t N = c.N;
     double diag = c.HS2[ic] + GkSum;
     double rhs = V * c.CmByDt[ic] + c.EmByRm[ic] + GkEkSum;
-    if (c.injPresent[ic]) rhs += c.injVarying[ic] + c.injBasal[ic];
+    if (c.injPresent[ic]) {
+        keepBranch();
+        rhs += inj + c.injBasal[ic];
+    }
     diag += eg;
     rhs += ege;
-    c.M[ic] = diag;
-    c.M[N + ic] = rhs;
-}
-
-// ---- elimination -------------------------------------------------------------
-// A level costs the eliminating warp ~150 instructions of index loads and
-// loop control around its few FP64 operations, all on one dependency chain.
-// A run of cable rows (one row per level, see CellPlan::fRun/bRun) is walked
-// by lane 0 alone with the pivot's values carried in registers, the row
-// indices computed (row r: diagonal M[r], right-hand side M[N + r],
-// off-diagonal to r + 1 at M[2N + H + r]) and the next row's operands loaded
-// ahead; the operations and their order are those of the general loop.
-__device__ __forceinline__ void forwardCableRun(const DevCell& c, uint32_t r, uint32_t run) {
-    double* M = c.M;
-    const uint32_t N = c.N, offBase = 2 * N + c.H;
-    double d = M[r - 1], rhs = M[N + r - 1];
-    double off = M[offBase + r - 1], dNext = M[r], rNext = M[N + r];
-    for (uint32_t i = 0; i < run; ++i, ++r) {
-        const double o = off, dr = dNext, rr = rNext;
-        if (i + 1 < run) {
-            off = M[offBase + r];
-            dNext = M[r + 1];
-            rNext = M[N + r + 1];
-        }
-        const double q = quotient(o, d);
-        d = dr - q * o;
-        rhs = rr - q * rhs;
-        M[r] = d;
-        M[N + r] = rhs;
-    }
-}
-
-__device__ __forceinline__ void backwardCableRun(const DevCell& c, uint32_t i, uint32_t run) {
-    const double* M = c.M;
-    const uint32_t N = c.N, offBase = 2 * N + c.H;
-    double vNext = c.VMid[i + 1];
-    double rhs = M[N + i], off = M[offBase + i], diag = M[i], vOld = c.V[i];
-    for (uint32_t j = 0; j < run; ++j, --i) {
-        const double r = rhs, o = off, dg = diag, vo = vOld;
-        if (j + 1 < run) {
-            rhs = M[N + i - 1];
-            off = M[offBase + i - 1];
-            diag = M[i - 1];
-            vOld = c.V[i - 1];
-        }
-        double v = r;
-        v -= o * vNext;
-        v = quotient(v, dg);
-        c.VMid[i] = v;
-        c.V[i] = __fma_rn(2.0, v, -vo);     // 2 v is exact
-        vNext = v;
-    }
-}
-
-template <bool WARP>
-__device__ __forceinline__ void levelSync() {
-    if (WARP) __syncwarp();
-    else __syncthreads();
-}
-
-// Forward elimination and back substitution by a group of `nth` threads:
-// one warp per cell in the FP64 batch, the whole CTA in the drop-in (the
-// rows of a level are independent, so a wide level of a branched cell is
-// shared by all warps instead of walked by one; a barrier per level).
-template <bool WARP>
-__device__ __forceinline__ void eliminate(const DevCell& c, uint32_t tid, uint32_t nth) {
-    double* M = c.M;
-    // Waves (CellPlan::fWavePtr): the level programs' updates, each wave's
-    // on disjoint entries, so the group shares a wave update by update
-    // instead of walking a row's chain per thread.  With a whole CTA, a
-    // thread's first update of the next wave (read-only descriptors) is
-    // loaded before the barrier.
-    if (WARP) {
-        for (uint32_t w = 0; w < c.fWaves; ++w) {
-            for (uint32_t k = c.fWavePtr[w] + tid; k < c.fWavePtr[w + 1]; k += nth) {
-                const int4 x = c.fWaveOps[2 * k], y = c.fWaveOps[2 * k + 1];
-                const double q = quotient(M[y.x], M[y.y]);
-                M[x.x] -= q * M[x.y];
-                if (x.z >= 0) M[x.z] -= q * M[x.w];
-            }
-            levelSync<WARP>();
-        }
-    } else if (c.fWaves) {
-        uint32_t kb = c.fWavePtr[0] + tid, ke = c.fWavePtr[1];
-        int4 xn = make_int4(0, 0, -1, 0), yn = make_int4(0, 0, 0, 0);
-        if (kb < ke) {
-            xn = c.fWaveOps[2 * kb];
-            yn = c.fWaveOps[2 * kb + 1];
-        }
-        for (uint32_t w = 0; w < c.fWaves; ++w) {
-            const uint32_t k0 = kb, e = ke;
-            const int4 x0 = xn, y0 = yn;
-            if (w + 1 < c.fWaves) {
-                kb = c.fWavePtr[w + 1] + tid;
-                ke = c.fWavePtr[w + 2];
-                if (kb < ke) {
-                    xn = c.fWaveOps[2 * kb];
-                    yn = c.fWaveOps[2 * kb + 1];
-                }
-            }
-            if (k0 < e) {
-                const double q = quotient(M[y0.x], M[y0.y]);
-                M[x0.x] -= q * M[x0.y];
-                if (x0.z >= 0) M[x0.z] -= q * M[x0.w];
-            }
-            for (uint32_t k = k0 + nth; k < e; k += nth) {
-                const int4 x = c.fWaveOps[2 * k], y = c.fWaveOps[2 * k + 1];
-                const double q = quotient(M[y.x], M[y.y]);
-                M[x.x] -= q * M[x.y];
-                if (x.z >= 0) M[x.z] -= q * M[x.w];
-            }
-            levelSync<WARP>();
-        }
-    }
-    for (uint32_t l = 0; l < (c.fWaves ? 0u : c.fLevels); ++l) {
-        if (const uint32_t run = c.fRun[l]) {
-            if (tid == 0) forwardCableRun(c, c.fRunRow[l], run);
-            levelSync<WARP>();
-            l += run - 1;
-            continue;
-        }
-        for (uint32_t k = c.fLevelPtr[l] + tid; k < c.fLevelPtr[l + 1]; k += nth) {
-            // t -= l / pivot * a.  A row's consecutive updates by one pivot
-            // (its diagonal and right-hand side: the reference computes
-            // HS[4i+1] / HS[4i] for both) share the quotient: it is computed
-            // once, the same IEEE division of the same operands, which takes
-            // one FP64 division off each level of the dependency chain.
-            int32_t ql = -1, qp = -1;
-            double q = 0.0;
-            for (uint32_t o = c.fOpPtr[k]; o < c.fOpPtr[k + 1]; ++o) {
-                int4 op = c.fOps[o];
-                if (op.y != ql || op.w != qp) {
-                    q = quotient(M[op.y], M[op.w]);
-                    ql = op.y;
-                    qp = op.w;
-                }
-                M[op.x] -= q * M[op.z];
-                if (op.x == ql || op.x == qp) ql = -1;   // an operand changed
-            }
-        }
-        levelSync<WARP>();
-    }
-    // Back substitution.  With a whole CTA, a thread's first row of the next
-    // level has its index, right-hand side, diagonal, old V and term range
-    // (none of which this level writes) loaded before the barrier; the level
-    // then waits only on the VMid values its terms read.
-    const uint32_t N = c.N;
-    if (WARP) {
-        for (uint32_t l = 0; l < c.bLevels; ++l) {
-            if (const uint32_t run = c.bRun[l]) {
-                if (tid == 0) backwardCableRun(c, c.bRunRow[l], run);
-                levelSync<WARP>();
-                l += run - 1;
-                continue;
-            }
-            for (uint32_t k = c.bLevelPtr[l] + tid; k < c.bLevelPtr[l + 1]; k += nth) {
-                uint32_t i = c.bRows[k];
-                double v = M[N + i];
-                for (uint32_t t = c.bTermPtr[k]; t < c.bTermPtr[k + 1]; ++t) {
-                    int2 term = c.bTerms[t];
-                    v -= M[term.x] * c.VMid[term.y];
-                }
-                v = quotient(v, M[i]);
-                c.VMid[i] = v;
-                c.V[i] = __fma_rn(2.0, v, -c.V[i]);
-            }
-            levelSync<WARP>();
-        }
-        return;
-    }
-    uint32_t nk = 0, ne = 0, ni = 0, nt0 = 0, nt1 = 0;
-    double nr = 0.0, nd = 1.0, nv = 0.0;
-    auto preload = [&](uint32_t l) {
-        nk = c.bLevelPtr[l] + tid;
-        ne = c.bLevelPtr[l + 1];
-        if (nk < ne) {
-            ni = c.bRows[nk];
-            nr = M[N + ni];
-            nd = M[ni];
-            nv = c.V[ni];
-            nt0 = c.bTermPtr[nk];
-            nt1 = c.bTermPtr[nk + 1];
-        }
-    };
-    bool ahead = false;
-    for (uint32_t l = 0; l < c.bLevels; ++l) {
-        if (const uint32_t run = c.bRun[l]) {
-            if (tid == 0) backwardCableRun(c, c.bRunRow[l], run);
-            levelSync<WARP>();
-            l += run - 1;
-            ahead = false;
-            continue;
-        }
-        if (!ahead) preload(l);
-        const uint32_t k0 = nk, e = ne, i0 = ni, t0 = nt0, t1 = nt1;
-        const double r0 = nr, d0 = nd, v0 = nv;
-        ahead = l + 1 < c.bLevels && !c.bRun[l + 1];
-        if (ahead) preload(l + 1);
-        if (k0 < e) {
-            double v = r0;
-            for (uint32_t t = t0; t < t1; ++t) {
-                int2 term = c.bTerms[t];
-                v -= M[term.x] * c.VMid[term.y];
-            }
-            v = quotient(v, d0);
-            c.VMid[i0] = v;
-            c.V[i0] = __fma_rn(2.0, v, -v0);
-        }
-        for (uint32_t k = k0 + nth; k < e; k += nth) {
-            uint32_t i = c.bRows[k];
-            double v = M[N + i];
-            for (uint32_t t = c.bTermPtr[k]; t < c.bTermPtr[k + 1]; ++t) {
-                int2 term = c.bTerms[t];
-                v -= M[term.x] * c.VMid[term.y];
-            }
-            v = quotient(v, M[i]);
-            c.VMid[i] = v;
-            c.V[i] = __fma_rn(2.0, v, -c.V[i]);
-        }
-        levelSync<WARP>();
-    }
+    M[ic] = diag;
+    M[c.N + ic] = rhs;
 }
 
 // ---- advanceCalcium, per pool ----------------------------------------------
-__device__ __forceinline__ void poolStep(const DevCell& c, uint32_t p) {
-    double act = c.iCa[p];
+// V already holds the step's new value.  `first`: a current sent by `iCa`
+// since the last process call may be waiting.
+__device__ __forceinline__ void poolStep(const DevCell& c, uint32_t p, const double* VMid, bool first) {
+    double act = 0.0;
+    if (first) {
+        act = c.iCa[p];
+        c.iCa[p] = 0.0;
+    }
     for (uint32_t f = c.feedPtr[p]; f < c.feedPtr[p + 1]; ++f) {
         uint32_t q = c.feedChan[f];
         uint32_t ic = c.chanCompt[q];
-        const double v = c.caAdvance == 1 ? c.VMid[ic] : __fma_rn(2.0, c.VMid[ic], -c.V[ic]);
+        const double v = c.caAdvance == 1 ? VMid[ic] : __fma_rn(2.0, VMid[ic], -c.V[ic]);
         act += c.Gk[q] * (c.Ek[q] - v);
     }
     double cc = c.f1[p] * c.c[p] + c.f2[p] * act;
@@ -553,106 +379,289 @@ __device__ __forceinline__ void poolStep(const DevCell& c, uint32_t p) {
     }
     c.c[p] = cc;
     c.ca[p] = ca;
-    c.iCa[p] = 0.0;
 }
 
-// One cell, `nsteps` steps, executed by a group of `nth` threads (a whole
-// CTA for the drop-in, one warp for the batch).  `barrier` orders the phases.
-template <bool WARP>
-__device__ __forceinline__ void groupSync() {
-    if (WARP) __syncwarp();
-    else __syncthreads();
+// The end of a step of compartment ic: V = 2 VMid - V (2 VMid is exact) and
+// its pools.
+__device__ __forceinline__ void finishCompt(const DevCell& c, uint32_t ic, const double* VMid, bool first) {
+    c.V[ic] = __fma_rn(2.0, VMid[ic], -c.V[ic]);
+    for (uint32_t p = c.poolPtr[ic]; p < c.poolPtr[ic + 1]; ++p) poolStep(c, p, VMid, first);
 }
 
-template <bool WARP>
-__device__ void stepCell(const DevCell& c, uint32_t nsteps, uint32_t tid, uint32_t nth) {
-    unsigned long long step = c.ctl->nSteps;
-    uint32_t stimPtr = c.ctl->stimPtr, nSpikes = c.ctl->nSpikes, nSamples = c.ctl->nSamples;
-    groupSync<WARP>();
-    for (uint32_t s = 0; s < nsteps; ++s, ++step) {
-        const double currTime = c.dt * (double)(step + 1);   // Clock: dt_ * endStep
-        if (tid == 0) {
-            while (stimPtr < c.nStim && c.stimStep[stimPtr] <= step) {
-                uint32_t h = c.stimCompt[stimPtr];
-                c.injPresent[h] = 1;
-                c.injBasal[h] = c.stimValue[stimPtr];
-                ++stimPtr;
+// ---- elimination -------------------------------------------------------------
+// Threads that step a cell together: a CTA, or a part of one with its own
+// named barrier.
+struct Team {
+    uint32_t tid, nth, bar;
+};
+__device__ __forceinline__ void teamSync(const Team& t) {
+    asm volatile("bar.sync %0, %1;" ::"r"(t.bar), "r"(t.nth) : "memory");
+}
+
+// A run of cable rows (one row per level, see CellPlan::fRun/bRun) is walked
+// by one lane with the pivot's values carried in registers, the row
+// indices computed (row r: diagonal M[r], right-hand side M[N + r],
+// off-diagonal to r + 1 at off[r]) and the next row's operands loaded
+// ahead; the operations and their order are those of the general loop.
+__device__ __forceinline__ void forwardCableRun(double* M, const double* off, uint32_t N, uint32_t r, uint32_t run) {
+    double d = M[r - 1], rhs = M[N + r - 1];
+    double o1 = off[r - 1], dNext = M[r], rNext = M[N + r];
+    for (uint32_t i = 0; i < run; ++i, ++r) {
+        const double o = o1, dr = dNext, rr = rNext;
+        if (i + 1 < run) {
+            o1 = off[r];
+            dNext = M[r + 1];
+            rNext = M[N + r + 1];
+        }
+        const double q = quotient(o, d);
+        d = dr - q * o;
+        rhs = rr - q * rhs;
+        M[r] = d;
+        M[N + r] = rhs;
+    }
+}
+
+__device__ __forceinline__ void backwardCableRun(const double* M, const double* off, double* VMid, uint32_t N,
+                                                 uint32_t i, uint32_t run) {
+    double vNext = VMid[i + 1];
+    double rhs = M[N + i], o1 = off[i], diag = M[i];
+    for (uint32_t j = 0; j < run; ++j, --i) {
+        const double r = rhs, o = o1, dg = diag;
+        if (j + 1 < run) {
+            rhs = M[N + i - 1];
+            o1 = off[i - 1];
+            diag = M[i - 1];
+        }
+        double v = r;
+        v -= o * vNext;
+        v = quotient(v, dg);
+        VMid[i] = v;
+        vNext = v;
+    }
+}
+
+// The level program of the forward sweep, for cells without waves (cables):
+// a row's updates in order, the rows of a level shared by the team.
+__device__ __forceinline__ void forwardLevels(const DevCell& c, double* M, const Team& t) {
+    const uint32_t N = c.N, offBase = 2 * N + c.H;
+    const double* off = c.M + offBase;
+    auto at = [&](int32_t e) { return (uint32_t)e >= offBase ? off[e - offBase] : M[e]; };
+    for (uint32_t l = 0; l < c.fLevels; ++l) {
+        if (const uint32_t run = c.fRun[l]) {
+            if (t.tid == 0) forwardCableRun(M, off, N, c.fRunRow[l], run);
+            teamSync(t);
+            l += run - 1;
+            continue;
+        }
+        for (uint32_t k = c.fLevelPtr[l] + t.tid; k < c.fLevelPtr[l + 1]; k += t.nth) {
+            // t -= l / pivot * a.  A row's consecutive updates by one pivot
+            // (its diagonal and right-hand side: the reference computes
+            // HS[4i+1] / HS[4i] for both) share the quotient: it is computed
+            // once, the same IEEE division of the same operands.
+            int32_t ql = -1, qp = -1;
+            double q = 0.0;
+            for (uint32_t o = c.fOpPtr[k]; o < c.fOpPtr[k + 1]; ++o) {
+                int4 op = c.fOps[o];
+                if (op.y != ql || op.w != qp) {
+                    q = quotient(at(op.y), M[op.w]);
+                    ql = op.y;
+                    qp = op.w;
+                }
+                M[op.x] -= q * at(op.z);
+                if (op.x == ql || op.x == qp) ql = -1;   // an operand changed
             }
-            if (c.nDif) difProcess(c);     // tick 1, before the gates read extCa
         }
-        for (uint32_t k = tid; k < c.S; k += nth) synchanStep(c, k, currTime);
-        for (uint32_t k = tid; k < c.K2; k += nth) chan2dStep(c, k);
-        groupSync<WARP>();
-        for (uint32_t h = tid; h < c.H; h += nth) c.M[2 * c.N + h] = c.HJ0[h];
-        for (uint32_t ic = tid; ic < c.N; ic += nth) comptStep(c, ic);
-        groupSync<WARP>();
-        eliminate<WARP>(c, tid, nth);
-        groupSync<WARP>();
-        for (uint32_t p = tid; p < c.P; p += nth) poolStep(c, p);
-        groupSync<WARP>();
-        if (tid == 0 && c.nDif) difSendIk(c);
-        // sendValues for the next step's tick-4 objects; SpikeGens; traces
-        for (uint32_t k = tid; k < c.K2; k += nth) {
-            c.c2dVm[k] = c.V[c.c2dCompt[k]];
-            if (c.c2dConc1[k] >= 0) c.c2dC1[k] = c.ca[c.c2dConc1[k]];
-            if (c.c2dConc2[k] >= 0) c.c2dC2[k] = c.ca[c.c2dConc2[k]];
+        teamSync(t);
+    }
+}
+
+// Forward elimination and back substitution in shared memory: M holds the
+// diagonal [0, N), the right-hand side [N, 2N), which becomes VMid, and the
+// junction entries [2N, 2N + H); the off-diagonals, which never change, come
+// with the updates' descriptors.
+// A wave or level is one dependent chain: loads, a division, a product and a
+// difference, a store, a barrier.  Two things follow.  A warp alone issues an
+// instruction every ~4 cycles of it, so the narrow ones -- at most 16 updates
+// or 32 rows, most of a cell's -- have a program of one record per lane, laid
+// out wave after wave: no bounds, no loop, no branch but the division's rare
+// one, and each of the two entries an update changes on a lane of its own
+// (each with the quotient).  The first warp walks them without a barrier;
+// the others call `idle` once meanwhile.  And a warp issues in order, so a
+// load whose address waits for another load would hold up the chain: records
+// are read one ahead from an address that is known.
+// 500 branched compartments, one CTA, cycles per wave or level: ~2,300 in
+// global memory, ~1,600 with per-wave bounds in shared memory.
+constexpr uint32_t kNoIndex = 0xFFFFu;      // no second entry, no update or row for this lane
+constexpr uint32_t kOffIndex = 0xFFFEu;     // the update's (row's) off-diagonal
+
+struct ProgOp {
+    uint4 d;        // the DevCell::fW or bW entry
+    double off;     // its off-diagonal
+    uint32_t t3;    // bW: the fourth term
+};
+__device__ __forceinline__ ProgOp progOp(const uint4* prog, uint32_t k) {
+    ProgOp w;
+    w.d = __ldg(prog + 2 * k);
+    const uint4 o = __ldg(prog + 2 * k + 1);
+    w.off = fromWords(o.y, o.x);
+    w.t3 = o.z;
+    return w;
+}
+__device__ __forceinline__ void waveEntry(double* M, uint32_t ta, double q, double off) {
+    const uint32_t t = ta & 0xFFFFu, a = ta >> 16;
+    if (t != kNoIndex) M[t] -= q * (a == kOffIndex ? off : M[a]);
+}
+__device__ __forceinline__ double waveQuotient(const double* M, const ProgOp& u) {
+    const uint32_t l = u.d.z & 0xFFFFu;
+    return quotient(l == kOffIndex ? u.off : M[l], M[u.d.z >> 16]);
+}
+// One entry of an update: {t | a << 16, l | p << 16, off-diagonal}.
+__device__ __forceinline__ void laneUpdate(double* M, const uint4& r) {
+    const uint32_t t = r.x & 0xFFFFu, a = r.x >> 16, l = r.y & 0xFFFFu;
+    if (t == kNoIndex) return;
+    const double off = fromWords(r.w, r.z), x = M[t];
+    const double av = a == kOffIndex ? off : M[a], lv = l == kOffIndex ? off : M[l];
+    M[t] = x - quotient(lv, M[r.y >> 16]) * av;
+}
+// A row: {row | terms << 16, the first three terms}, {off-diagonal, fourth
+// term, first of the others in bX}.
+__device__ __forceinline__ void substitute(const DevCell& c, double* M, const uint4* prog, uint32_t k, const ProgOp& b) {
+    const uint32_t N = c.N, i = b.d.x & 0xFFFFu, n = b.d.x >> 16, co = b.d.y & 0xFFFFu;
+    double v = M[N + i];
+    const double d = M[i];
+    if (n) {
+        v -= (co == kOffIndex ? b.off : M[co]) * M[N + (b.d.y >> 16)];
+        if (n > 1) v -= M[b.d.z & 0xFFFFu] * M[N + (b.d.z >> 16)];
+        if (n > 2) v -= M[b.d.w & 0xFFFFu] * M[N + (b.d.w >> 16)];
+        if (n > 3) v -= M[b.t3 & 0xFFFFu] * M[N + (b.t3 >> 16)];
+        if (n > 4) {
+            const uint32_t x0 = __ldg(prog + 2 * k + 1).w;
+            for (uint32_t t = 4; t < n; ++t) {
+                const uint32_t x = __ldg(c.bX + x0 + t - 4);
+                v -= M[x & 0xFFFFu] * M[N + (x >> 16)];
+            }
         }
-        if (tid == 0) {
-            for (uint32_t k = 0; k < c.SG; ++k) {
-                double V = c.V[c.sgCompt[k]];
-                if (V > c.sgThreshold[k]) {
-                    if ((currTime + c.dt / 2.0) >= (c.sgLast[k] + c.sgRefract[k])) {
-                        if (!(c.sgEdge[k] && c.sgFired[k])) {
-                            if (nSpikes < c.spikeCap) {
-                                c.spikeGen[nSpikes] = k;
-                                c.spikeTime[nSpikes] = currTime;
-                            }
-                            ++nSpikes;
-                            c.sgLast[k] = currTime;
-                            c.sgFired[k] = 1;
-                        }
-                    }
-                } else {
-                    c.sgFired[k] = 0;
+    }
+    M[N + i] = quotient(v, d);
+}
+
+template <class Idle>
+__device__ __forceinline__ void eliminateShared(const DevCell& c, double* M, const Team& t, Idle idle) {
+    const uint32_t N = c.N, lane = t.tid & 31u;
+    const bool w0 = t.tid < 32;
+    bool idled = false, pend = false;      // pend: the first warp wrote since the last barrier
+    auto others = [&]() {
+        if (!idled) idle();
+        idled = true;
+    };
+    // Segments of consecutive narrow or wide waves {count | kind, first}.
+    for (uint32_t sg = 0; sg < c.nfSeg; ++sg) {
+        const uint2 S = __ldg(c.fSeg + sg);
+        const uint32_t n = S.x & ~kSegKind;
+        if (S.x & kSegNarrow) {
+            pend = true;
+            if (!w0) {
+                others();
+                continue;
+            }
+            const uint4* r = c.fLane + S.y + lane;
+            uint4 next = __ldg(r);
+            for (uint32_t w = 0; w < n; ++w) {
+                const uint4 u = next;
+                r += 32;
+                if (w + 1 < n) next = __ldg(r);
+                laneUpdate(M, u);
+                __syncwarp();
+            }
+            continue;
+        }
+        if (pend) teamSync(t);
+        pend = false;
+        const uint32_t* ptr = c.fWavePtr + S.y;
+        uint32_t b = ptr[0], e = ptr[1], e1 = ptr[min(2u, n)], k;
+        bool two;
+        auto mine = [&]() {
+            two = c.fSplit && 2 * (e - b) <= t.nth;
+            k = b + (two ? t.tid >> 1 : t.tid);
+        };
+        mine();
+        ProgOp next;
+        if (k < e) next = progOp(c.fW, k);
+        for (uint32_t w = 0; w < n; ++w) {
+            const uint32_t k0 = k, e0 = e;
+            const bool two0 = two;
+            ProgOp u = next;
+            if (w + 1 < n) {
+                b = e;
+                e = e1;
+                e1 = ptr[min(w + 3, n)];
+                mine();
+                if (k < e) next = progOp(c.fW, k);
+            }
+            if (two0) {
+                if (k0 < e0) waveEntry(M, (t.tid & 1u) ? u.d.y : u.d.x, waveQuotient(M, u), u.off);
+            } else {
+                for (uint32_t j = k0; j < e0; j += t.nth) {
+                    if (j != k0) u = progOp(c.fW, j);
+                    const double q = waveQuotient(M, u);
+                    waveEntry(M, u.d.x, q, u.off);
+                    waveEntry(M, u.d.y, q, u.off);
                 }
             }
+            teamSync(t);
         }
-        if (c.nRec && ((step + 1) % c.recStride) == 0) {
-            if (nSamples < c.recCap)
-                for (uint32_t r = tid; r < c.nRec; r += nth)
-                    c.recBuf[(size_t)nSamples * c.recLd + r] = recValue(c, c.recCompt[r]);
-            ++nSamples;
-        }
-        for (uint32_t ic = tid; ic < c.N; ic += nth) {
-            c.injVarying[ic] = 0.0;
-            c.ext[2 * ic] = 0.0;
-            c.ext[2 * ic + 1] = 0.0;
-        }
-        groupSync<WARP>();
     }
-    if (tid == 0) {
-        c.ctl->nSteps = step;
-        c.ctl->stimPtr = stimPtr;
-        c.ctl->nSpikes = nSpikes;
-        c.ctl->nSamples = nSamples;
+    if (!c.fWaves) forwardLevels(c, M, t);
+    // back substitution: narrow levels and cable runs by the first warp
+    for (uint32_t sg = 0; sg < c.nbSeg; ++sg) {
+        const uint2 S = __ldg(c.bSeg + sg);
+        const uint32_t n = S.x & ~kSegKind;
+        if (S.x & kSegKind) {
+            pend = true;
+            if (!w0) {
+                others();
+                continue;
+            }
+            if (S.x & kSegRun) {
+                if (t.tid == 0) backwardCableRun(M, c.M + 2 * N + c.H, M + N, N, S.y, n);
+                __syncwarp();
+                continue;
+            }
+            uint32_t k = S.y + lane;
+            ProgOp next = progOp(c.bLane, k);
+            for (uint32_t l = 0; l < n; ++l, k += 32) {
+                const ProgOp r = next;
+                if (l + 1 < n) next = progOp(c.bLane, k + 32);
+                if ((r.d.x & 0xFFFFu) != kNoIndex) substitute(c, M, c.bLane, k, r);
+                __syncwarp();
+            }
+            continue;
+        }
+        if (pend) teamSync(t);
+        pend = false;
+        const uint32_t* ptr = c.bLevelPtr + S.y;
+        uint32_t e = ptr[1], e1 = ptr[min(2u, n)], k = ptr[0] + t.tid;
+        ProgOp next;
+        if (k < e) next = progOp(c.bW, k);
+        for (uint32_t l = 0; l < n; ++l) {
+            const uint32_t k0 = k, e0 = e;
+            const ProgOp r = next;
+            if (l + 1 < n) {
+                k = e + t.tid;
+                e = e1;
+                e1 = ptr[min(l + 3, n)];
+                if (k < e) next = progOp(c.bW, k);
+            }
+            if (k0 < e0) substitute(c, M, c.bW, k0, r);
+            for (uint32_t j = k0 + t.nth; j < e0; j += t.nth) substitute(c, M, c.bW, j, progOp(c.bW, j));
+            teamSync(t);
+        }
     }
+    if (pend) teamSync(t);
 }
 
-__global__ void __launch_bounds__(256, 1) hsStepFp64(DevCell c, uint32_t nsteps) {
-    stepCell<false>(c, nsteps, threadIdx.x, blockDim.x);
-}
-
-// One cell stepped by a thread-block cluster.  On one SM a large cell's step
-// is bound by the FP64 work of its channels and matrix rows (one SM's FP64
-// pipe); the cluster's CTAs share that work -- object k goes to thread k of
-// the cluster -- and the wide waves and levels of the elimination
-// (eliminateCluster), while rank 0's CTA walks the narrow ones.
-// Every object's arithmetic is unchanged and the phases keep their order,
-// so the results are bit-identical to stepCell.  The hardware cluster
-// barrier (release/acquire at cluster scope) orders the phases; all data
-// stays in the cell's global arena.
-// One fused forward update and one back-substitution row, as eliminate does
-// them.
+// The same sweeps in global memory by one CTA, for a cell whose matrix does
+// not fit in shared memory (above ~5,000 branched compartments).
 __device__ __forceinline__ void waveUpdate(const DevCell& c, double* M, uint32_t k) {
     const int4 x = c.fWaveOps[2 * k], y = c.fWaveOps[2 * k + 1];
     const double q = quotient(M[y.x], M[y.y]);
@@ -660,40 +669,52 @@ __device__ __forceinline__ void waveUpdate(const DevCell& c, double* M, uint32_t
     if (x.z >= 0) M[x.z] -= q * M[x.w];
 }
 
-__device__ __forceinline__ void backRow(const DevCell& c, const double* M, uint32_t N, uint32_t k) {
-    uint32_t i = c.bRows[k];
+__device__ __forceinline__ void backRowGlobal(const DevCell& c, const double* M, uint32_t k) {
+    const uint32_t N = c.N, i = c.bRows[k];
     double v = M[N + i];
     for (uint32_t t = c.bTermPtr[k]; t < c.bTermPtr[k + 1]; ++t) {
         int2 term = c.bTerms[t];
         v -= M[term.x] * c.VMid[term.y];
     }
-    v = quotient(v, M[i]);
-    c.VMid[i] = v;
-    c.V[i] = __fma_rn(2.0, v, -c.V[i]);
+    c.VMid[i] = quotient(v, M[i]);
 }
 
-// The elimination of a cell stepped by a cluster.  A forward wave or a
+__device__ void eliminateGlobal(const DevCell& c, const Team& t) {
+    double* M = c.M;
+    const uint32_t N = c.N;
+    const double* off = M + 2 * N + c.H;
+    for (uint32_t w = 0; w < c.fWaves; ++w) {
+        for (uint32_t k = c.fWavePtr[w] + t.tid; k < c.fWavePtr[w + 1]; k += t.nth) waveUpdate(c, M, k);
+        teamSync(t);
+    }
+    if (!c.fWaves) forwardLevels(c, M, t);
+    for (uint32_t l = 0; l < c.bLevels; ++l) {
+        if (const uint32_t run = c.bRun[l]) {
+            if (t.tid == 0) backwardCableRun(M, off, c.VMid, N, c.bRunRow[l], run);
+            l += run - 1;
+        } else {
+            for (uint32_t k = c.bLevelPtr[l] + t.tid; k < c.bLevelPtr[l + 1]; k += t.nth) backRowGlobal(c, M, k);
+        }
+        teamSync(t);
+    }
+}
+
+// Of a cell stepped by a cluster, still in global memory: a forward wave or a
 // back-substitution level of at least kClusterWide updates or rows is
 // shared by all the cluster's CTAs, a cluster barrier after it (and before
 // it, when rank 0 wrote alone since the last one); narrower ones are
-// walked by rank 0's CTA with a CTA barrier, as eliminate walks them.  The
+// walked by rank 0's CTA with a CTA barrier.  The
 // updates of a wave, and the rows of a level, are independent, so which
-// thread of which CTA does one changes nothing: bit-identical to
-// eliminate.  Every CTA takes the same branches (they depend on the sizes
-// alone), so all meet at every cluster barrier.  Cells without waves (the
-// cable runs' level programs) and cells below kClusterElimRows compartments
-// are eliminated by rank 0 alone, as eliminate does it: sharing pays from
-// ~4,000 compartments on (one GB300, 8 CTAs: 5,000 compartments 407 -> 378
-// us per step, 10,000: 631 -> 498), and costs below (1,000: 171 -> 190,
-// 2,000: 231 -> 244; the shared waves' cluster barriers and the L2 reads
-// after them outweigh the work they split).
+// thread of which CTA does one changes nothing: bit-identical.  Every CTA
+// takes the same branches (they depend on the sizes
+// alone), so all meet at every cluster barrier.  (One GB300, 8 CTAs, against
+// rank 0 alone in global memory: 10,000 compartments 631 -> 498 us per step.)
 constexpr uint32_t kClusterWide = 1024;
-constexpr uint32_t kClusterElimRows = 4096;
 
-__device__ void eliminateCluster(const DevCell& c, cooperative_groups::cluster_group& cl, uint32_t rank,
-                                 uint32_t tid, uint32_t nth, uint32_t g, uint32_t G) {
-    if (!c.fWaves || c.N < kClusterElimRows) {
-        if (rank == 0) eliminate<false>(c, tid, nth);
+__device__ void eliminateGlobalCluster(const DevCell& c, cooperative_groups::cluster_group& cl, uint32_t rank,
+                                       const Team& t, uint32_t g, uint32_t G) {
+    if (!c.fWaves) {
+        if (rank == 0) eliminateGlobal(c, t);
         return;
     }
     double* M = c.M;
@@ -707,8 +728,8 @@ __device__ void eliminateCluster(const DevCell& c, cooperative_groups::cluster_g
             cl.sync();
         } else {
             if (rank == 0) {
-                for (uint32_t k = b0 + tid; k < e; k += nth) waveUpdate(c, M, k);
-                __syncthreads();
+                for (uint32_t k = b0 + t.tid; k < e; k += t.nth) waveUpdate(c, M, k);
+                teamSync(t);
             }
             alone = true;
         }
@@ -717,8 +738,8 @@ __device__ void eliminateCluster(const DevCell& c, cooperative_groups::cluster_g
     for (uint32_t l = 0; l < c.bLevels; ++l) {
         if (const uint32_t run = c.bRun[l]) {
             if (rank == 0) {
-                if (tid == 0) backwardCableRun(c, c.bRunRow[l], run);
-                __syncthreads();
+                if (t.tid == 0) backwardCableRun(M, M + 2 * N + c.H, c.VMid, N, c.bRunRow[l], run);
+                teamSync(t);
             }
             alone = true;
             l += run - 1;
@@ -728,88 +749,152 @@ __device__ void eliminateCluster(const DevCell& c, cooperative_groups::cluster_g
         if (e - b0 >= kClusterWide) {
             if (alone) cl.sync();
             alone = false;
-            for (uint32_t k = b0 + g; k < e; k += G) backRow(c, M, N, k);
+            for (uint32_t k = b0 + g; k < e; k += G) backRowGlobal(c, M, k);
             cl.sync();
         } else {
             if (rank == 0) {
-                for (uint32_t k = b0 + tid; k < e; k += nth) backRow(c, M, N, k);
-                __syncthreads();
+                for (uint32_t k = b0 + t.tid; k < e; k += t.nth) backRowGlobal(c, M, k);
+                teamSync(t);
             }
             alone = true;
         }
     }
 }
 
-__device__ void stepCellCluster(const DevCell& c, uint32_t nsteps) {
+// ---- outputs of a step ---------------------------------------------------------
+// SpikeGens (one thread), with V and Ca at the end of step `step`.
+__device__ __forceinline__ void spikeGens(const DevCell& c, unsigned long long step, uint32_t& nSpikes) {
+    const double currTime = c.dt * (double)(step + 1);
+    for (uint32_t k = 0; k < c.SG; ++k) {
+        if (lessThan(c.sgThreshold[k], c.V[c.sgCompt[k]])) {
+            if (atMost(c.sgLast[k] + c.sgRefract[k], currTime + c.dt / 2.0) && !(c.sgEdge[k] && c.sgFired[k])) {
+                if (nSpikes < c.spikeCap) {
+                    c.spikeGen[nSpikes] = k;
+                    c.spikeTime[nSpikes] = currTime;
+                }
+                ++nSpikes;
+                c.sgLast[k] = currTime;
+                c.sgFired[k] = 1;
+            }
+        } else {
+            c.sgFired[k] = 0;
+        }
+    }
+}
+
+__device__ __forceinline__ void stimulus(const DevCell& c, unsigned long long step, uint32_t& stimPtr) {
+    while (stimPtr < c.nStim && c.stimStep[stimPtr] <= step) {
+        uint32_t h = c.stimCompt[stimPtr];
+        c.injPresent[h] = 1;
+        c.injBasal[h] = c.stimValue[stimPtr];
+        ++stimPtr;
+    }
+}
+
+// What the tick-4 objects of compartment ic are sent (HSolveActive::sendValues).
+__device__ __forceinline__ void sendCompt(const DevCell& c, uint32_t k) {
+    c.c2dVm[k] = c.V[c.c2dCompt[k]];
+    if (c.c2dConc1[k] >= 0) c.c2dC1[k] = c.ca[c.c2dConc1[k]];
+    if (c.c2dConc2[k] >= 0) c.c2dC2[k] = c.ca[c.c2dConc2[k]];
+}
+
+// One cell, `nsteps` steps, by team `t` or, with CL, by the cluster whose
+// rank `rank` CTA this is.  Object k goes to thread k of the G threads
+// (this one is g).  The matrix Mr is in shared memory (`own`; of a cluster in
+// rank 0's, which the others reach through distributed shared memory) or,
+// unless `shared`, the cell's in global memory.
+// Fused steps (c.local: every pool and HHChannel2D reads and feeds its own
+// compartment; no tick-1 objects, no recorded Gk or Ik): the end of a
+// compartment's step (V, pools), its HHChannel2Ds and its next row are one
+// pass of one thread, so a step has two barriers besides the elimination's;
+// the outputs of a step, and the next step's SynChans and stimulus, which
+// need nothing that the elimination writes, run while it does.
+// Otherwise the phases run one after the other.
+template <bool CL>
+__device__ __forceinline__ void stepCell(const DevCell& c, uint32_t nsteps, const Team& t, bool shared, double* own,
+                                         double* Mr, uint32_t rank, uint32_t g, uint32_t G) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
-    const uint32_t rank = cl.block_rank();
-    const uint32_t tid = threadIdx.x, nth = blockDim.x;
-    const uint32_t g = rank * nth + tid, G = cl.num_blocks() * nth;
+    auto phase = [&]() {
+        if (CL) cl.sync();
+        else teamSync(t);
+    };
+    const uint32_t N = c.N;
+    const double hdt = c.dt / 2.0;
+    const bool fused = c.local && !c.nDif && !(c.nRec && c.recChan);
+    const bool aux = g == (G > 32 ? G - 32 : 0);      // stimulus and SpikeGens: a thread of the last warp
+    double* VMid = shared ? Mr + N : c.VMid;
     unsigned long long step = c.ctl->nSteps;
     uint32_t stimPtr = c.ctl->stimPtr, nSpikes = c.ctl->nSpikes, nSamples = c.ctl->nSamples;
-    cl.sync();
-    for (uint32_t s = 0; s < nsteps; ++s, ++step) {
-        const double currTime = c.dt * (double)(step + 1);
-        if (g == 0) {
-            while (stimPtr < c.nStim && c.stimStep[stimPtr] <= step) {
-                uint32_t h = c.stimCompt[stimPtr];
-                c.injPresent[h] = 1;
-                c.injBasal[h] = c.stimValue[stimPtr];
-                ++stimPtr;
-            }
-            if (c.nDif) difProcess(c);
-        }
-        for (uint32_t k = g; k < c.S; k += G) synchanStep(c, k, currTime);
-        for (uint32_t k = g; k < c.K2; k += G) chan2dStep(c, k);
-        cl.sync();
-        for (uint32_t h = g; h < c.H; h += G) c.M[2 * c.N + h] = c.HJ0[h];
-        for (uint32_t ic = g; ic < c.N; ic += G) comptStep(c, ic);
-        cl.sync();
-        eliminateCluster(c, cl, rank, tid, nth, g, G);
-        cl.sync();
-        for (uint32_t p = g; p < c.P; p += G) poolStep(c, p);
-        cl.sync();
-        if (g == 0 && c.nDif) difSendIk(c);
-        for (uint32_t k = g; k < c.K2; k += G) {
-            c.c2dVm[k] = c.V[c.c2dCompt[k]];
-            if (c.c2dConc1[k] >= 0) c.c2dC1[k] = c.ca[c.c2dConc1[k]];
-            if (c.c2dConc2[k] >= 0) c.c2dC2[k] = c.ca[c.c2dConc2[k]];
-        }
-        if (g == 0) {
-            for (uint32_t k = 0; k < c.SG; ++k) {
-                double V = c.V[c.sgCompt[k]];
-                if (V > c.sgThreshold[k]) {
-                    if ((currTime + c.dt / 2.0) >= (c.sgLast[k] + c.sgRefract[k])) {
-                        if (!(c.sgEdge[k] && c.sgFired[k])) {
-                            if (nSpikes < c.spikeCap) {
-                                c.spikeGen[nSpikes] = k;
-                                c.spikeTime[nSpikes] = currTime;
-                            }
-                            ++nSpikes;
-                            c.sgLast[k] = currTime;
-                            c.sgFired[k] = 1;
-                        }
-                    }
-                } else {
-                    c.sgFired[k] = 0;
-                }
-            }
-        }
-        if (c.nRec && ((step + 1) % c.recStride) == 0) {
+    phase();
+    auto record = [&](unsigned long long st) {
+        if (c.nRec && ((st + 1) % c.recStride) == 0) {
             if (nSamples < c.recCap)
                 for (uint32_t r = g; r < c.nRec; r += G)
                     c.recBuf[(size_t)nSamples * c.recLd + r] = recValue(c, c.recCompt[r]);
             ++nSamples;
         }
-        for (uint32_t ic = g; ic < c.N; ic += G) {
-            c.injVarying[ic] = 0.0;
-            c.ext[2 * ic] = 0.0;
-            c.ext[2 * ic + 1] = 0.0;
+    };
+    for (uint32_t s = 0; s < nsteps; ++s, ++step) {
+        const bool first = s == 0, last = s + 1 == nsteps;
+        if (first || !fused) {
+            const double currTime = c.dt * (double)(step + 1);   // Clock: dt_ * endStep
+            if (aux) stimulus(c, step, stimPtr);
+            if (g == 0 && c.nDif) difProcess(c);                  // tick 1, before the gates read extCa
+            for (uint32_t k = g; k < c.S; k += G) synchanStep(c, k, currTime);
+            if (!fused)
+                for (uint32_t k = g; k < c.K2; k += G) chan2dStep(c, k, c.c2dVm[k], c.c2dC1[k], c.c2dC2[k]);
+            phase();
         }
-        cl.sync();
+        for (uint32_t h = g; h < c.H; h += G) Mr[2 * N + h] = c.HJ0[h];
+        for (uint32_t ic = g; ic < N; ic += G) {
+            if (fused && !first) finishCompt(c, ic, VMid, s == 1);
+            rowStep(c, ic, hdt, fused, first, last, Mr);
+        }
+        phase();
+        auto aside = [&](uint32_t a, uint32_t nA) {
+            if (!fused) return;
+            if (!first && aux) spikeGens(c, step - 1, nSpikes);
+            if (last) return;
+            if (aux) stimulus(c, step + 1, stimPtr);
+            const double nextTime = c.dt * (double)(step + 2);
+            for (uint32_t k = a; k < c.S; k += nA) synchanStep(c, k, nextTime);
+        };
+        if (fused && !first) record(step - 1);
+        if (!shared) {
+            aside(g, G);
+            if (CL) eliminateGlobalCluster(c, cl, rank, t, g, G);
+            else eliminateGlobal(c, t);
+        } else if (CL) {
+            if (rank) aside((rank - 1) * t.nth + t.tid, G - t.nth);
+            else eliminateShared(c, own, t, [&]() {});
+        } else if (t.nth > 32) {
+            eliminateShared(c, own, t, [&]() { aside(t.tid - 32, t.nth - 32); });
+        } else {
+            aside(g, G);
+            eliminateShared(c, own, t, [&]() {});
+        }
+        if (CL || !shared) phase();
+        if (!fused) {
+            for (uint32_t ic = g; ic < N; ic += G) c.V[ic] = __fma_rn(2.0, VMid[ic], -c.V[ic]);
+            phase();
+            for (uint32_t p = g; p < c.P; p += G) poolStep(c, p, VMid, first);
+            phase();
+            if (g == 0 && c.nDif) difSendIk(c);
+            for (uint32_t k = g; k < c.K2; k += G) sendCompt(c, k);
+            if (aux) spikeGens(c, step, nSpikes);
+            record(step);
+            phase();
+        }
     }
-    if (g == 0) {
+    if (fused && nsteps) {
+        for (uint32_t ic = g; ic < N; ic += G) finishCompt(c, ic, VMid, nsteps == 1);
+        phase();
+        for (uint32_t k = g; k < c.K2; k += G) sendCompt(c, k);
+        if (aux) spikeGens(c, step - 1, nSpikes);
+        record(step - 1);
+    }
+    if (aux) {
         c.ctl->nSteps = step;
         c.ctl->stimPtr = stimPtr;
         c.ctl->nSpikes = nSpikes;
@@ -817,43 +902,108 @@ __device__ void stepCellCluster(const DevCell& c, uint32_t nsteps) {
     }
 }
 
-__global__ void __launch_bounds__(256, 1) hsStepFp64Cluster(DevCell c, uint32_t nsteps) {
-    stepCellCluster(c, nsteps);
+// The drop-in, one CTA.  `words`: the matrix is in shared memory (that many
+// doubles), 0: in global memory.
+__global__ void __launch_bounds__(512, 1) hsStepFp64(DevCell c, uint32_t words, uint32_t nsteps) {
+    extern __shared__ double sMatrix[];
+    const Team t{threadIdx.x, blockDim.x, 0};
+    stepCell<false>(c, nsteps, t, words != 0, sMatrix, words ? sMatrix : c.M, 0, t.tid, t.nth);
 }
+
+// One cell stepped by a thread-block cluster.  On one SM a large cell's step
+// is bound by the FP64 work of its channels and matrix rows (one SM's FP64
+// pipe); the cluster's CTAs share that work -- object k goes to thread k of
+// the cluster -- and write the rows into rank 0's shared memory, whose CTA
+// eliminates.  Every object's arithmetic is unchanged and the phases keep
+// their order, so the results are bit-identical to one CTA's.  The hardware
+// cluster barrier (release/acquire at cluster scope) orders the phases.
+__device__ __forceinline__ void stepCellCluster(const DevCell& c, uint32_t words, uint32_t nsteps, double* sm) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const Team t{threadIdx.x, blockDim.x, 0};
+    const uint32_t rank = cl.block_rank();
+    // warps of the cluster in turn over its CTAs: a few warps of objects
+    // reach as many sub-partitions as there are
+    const uint32_t nb = cl.num_blocks(), g = ((t.tid >> 5) * nb + rank) * 32 + (t.tid & 31u);
+    stepCell<true>(c, nsteps, t, words != 0, sm, words ? cl.map_shared_rank(sm, 0) : c.M, rank, g, nb * t.nth);
+    if (words) cl.sync();        // rank 0's shared memory outlives every access
+}
+
+__global__ void __launch_bounds__(256, 1) hsStepFp64Cluster(DevCell c, uint32_t words, uint32_t nsteps) {
+    extern __shared__ double sMatrix[];
+    stepCellCluster(c, words, nsteps, sMatrix);
+}
+
+// The cell descriptions are read from shared memory: a pointer per array, used
+// all through the step.
+__device__ __forceinline__ void copyCell(DevCell* dst, const DevCell* src, uint32_t tid, uint32_t nth) {
+    const uint32_t n = sizeof(DevCell) / 8;
+    const unsigned long long* a = reinterpret_cast<const unsigned long long*>(src);
+    unsigned long long* b = reinterpret_cast<unsigned long long*>(dst);
+    for (uint32_t i = tid; i < n; i += nth) b[i] = a[i];
+}
+static_assert(sizeof(DevCell) % 8 == 0, "DevCell is copied in 8-byte words");
 
 // Separate drop-in solvers stepped in one launch (hs_process_group): CTA k
 // steps solver k exactly as hsStepFp64 steps it alone; in the cluster form
-// cluster k steps solver k exactly as hsStepFp64Cluster does.
-__global__ void __launch_bounds__(256) hsGroupStepFp64(const DevCell* __restrict__ cells, uint32_t nsteps) {
-    stepCell<false>(cells[blockIdx.x], nsteps, threadIdx.x, blockDim.x);
+// cluster k steps solver k exactly as hsStepFp64Cluster does.  `words`: doubles
+// of shared memory a CTA has for its matrix.
+__global__ void __launch_bounds__(256, 2) hsGroupStepFp64(const DevCell* __restrict__ cells, uint32_t words,
+                                                          uint32_t nsteps) {
+    extern __shared__ double sMatrix[];
+    __shared__ DevCell c;
+    copyCell(&c, cells + blockIdx.x, threadIdx.x, blockDim.x);
+    __syncthreads();
+    const Team t{threadIdx.x, blockDim.x, 0};
+    const bool shared = c.smWords && c.smWords <= words;
+    stepCell<false>(c, nsteps, t, shared, sMatrix, shared ? sMatrix : c.M, 0, t.tid, t.nth);
 }
 
-__global__ void __launch_bounds__(256) hsGroupStepFp64Cluster(const DevCell* __restrict__ cells, uint32_t nsteps) {
-    stepCellCluster(cells[blockIdx.x / cooperative_groups::this_cluster().num_blocks()], nsteps);
+__global__ void __launch_bounds__(256) hsGroupStepFp64Cluster(const DevCell* __restrict__ cells, uint32_t words,
+                                                              uint32_t nsteps) {
+    extern __shared__ double sMatrix[];
+    __shared__ DevCell c;
+    copyCell(&c, cells + blockIdx.x / cooperative_groups::this_cluster().num_blocks(), threadIdx.x, blockDim.x);
+    __syncthreads();
+    stepCellCluster(c, c.smWords <= words ? c.smWords : 0, nsteps, sMatrix);
 }
 
-// Batched FP64.  A CTA either steps its cells one after the other with all
-// its threads, as the drop-in steps one cell (ctaCellPtr gives it a
-// non-empty list: the largest cells, whose chains would otherwise bound the
-// step), or runs one warp per cell on the cells listed per warp.  Both
-// forms do the drop-in's arithmetic in its order: results are bit-identical
-// whichever form steps a cell.
-__global__ void __launch_bounds__(256) hsBatchStepFp64(const DevCell* __restrict__ cells,
-                                                       const uint32_t* __restrict__ warpCellPtr,
-                                                       const uint32_t* __restrict__ warpCells,
-                                                       uint32_t nWarps, const uint32_t* __restrict__ ctaCellPtr,
-                                                       const uint32_t* __restrict__ ctaCells, uint32_t nsteps) {
-    const uint32_t c0 = ctaCellPtr[blockIdx.x], c1 = ctaCellPtr[blockIdx.x + 1];
-    if (c0 < c1) {      // uniform over the CTA
-        for (uint32_t k = c0; k < c1; ++k) stepCell<false>(cells[ctaCells[k]], nsteps, threadIdx.x, blockDim.x);
-        return;
-    }
-    uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    uint32_t lane = threadIdx.x & 31;
-    if (w >= nWarps) return;
-    for (uint32_t k = warpCellPtr[w]; k < warpCellPtr[w + 1]; ++k) {
-        const DevCell& c = cells[warpCells[k]];
-        stepCell<true>(c, nsteps, lane, 32);
+// Batched FP64: one CTA per SM, in teams of `teamThreads` threads.  The CTA
+// steps the cells of its own list (wholePtr) one after the other with all its
+// threads, as the drop-in steps one cell; then each team steps its list
+// (teamPtr), so that the elimination's latency of one cell overlaps the FP64
+// work of the others.  Both forms do the drop-in's arithmetic in its order:
+// results are bit-identical whichever form steps a cell.  `words`: doubles of
+// shared memory for a whole-CTA cell's matrix; a team has its share.
+__global__ void __launch_bounds__(512, 1) hsBatchStepFp64(const DevCell* __restrict__ cells,
+                                                          const uint32_t* __restrict__ wholePtr,
+                                                          const uint32_t* __restrict__ wholeCells,
+                                                          const uint32_t* __restrict__ teamPtr,
+                                                          const uint32_t* __restrict__ teamCells,
+                                                          uint32_t teamThreads, uint32_t words, uint32_t nsteps) {
+    extern __shared__ double sm[];
+    const uint32_t nTeams = blockDim.x / teamThreads, team = threadIdx.x / teamThreads;
+    DevCell* sCells = reinterpret_cast<DevCell*>(sm);
+    double* sMatrix = sm + nTeams * (sizeof(DevCell) / 8);
+    const uint32_t n0 = wholePtr[blockIdx.x + 1] - wholePtr[blockIdx.x];
+    const uint32_t t0 = blockIdx.x * nTeams + team;
+    const uint32_t n1 = teamPtr[t0 + 1] - teamPtr[t0];
+    const uint32_t share = words / nTeams;
+    for (uint32_t k = 0;; ++k) {
+        if (k == n0 && n0) __syncthreads();     // the whole CTA's last cell is done everywhere
+        if (k >= n0 + n1) break;
+        const bool whole = k < n0;
+        const Team t{whole ? threadIdx.x : threadIdx.x - team * teamThreads, whole ? blockDim.x : teamThreads,
+                     whole ? 0 : team};
+        const uint32_t cell = whole ? wholeCells[wholePtr[blockIdx.x] + k] : teamCells[teamPtr[t0] + k - n0];
+        DevCell* c = sCells + (whole ? 0 : team);
+        teamSync(t);                            // the team's last cell is done
+        copyCell(c, cells + cell, t.tid, t.nth);
+        teamSync(t);
+        const uint32_t room = whole ? words : share;
+        const bool shared = c->smWords && c->smWords <= room;
+        double* M = sMatrix + (whole ? 0 : team * share);
+        stepCell<false>(*c, nsteps, t, shared, M, shared ? M : c->M, 0, t.tid, t.nth);
     }
 }
 
@@ -1027,63 +1177,95 @@ cudaError_t launchScatterFields(const FieldWrite* w, uint32_t n, cudaStream_t st
     return cudaGetLastError();
 }
 
+namespace {
+
+// Doubles of shared memory that a kernel with `statics` bytes of its own can
+// have, on the current device.
+uint32_t roomWords(size_t statics) {
+    int dev = 0, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return 0;
+    return (size_t)optin > statics ? (uint32_t)(((size_t)optin - statics) / 8) : 0;
+}
+
+template <class K>
+cudaError_t allowShared(K kernel, size_t bytes) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+cudaLaunchConfig_t clusterConfig(cudaLaunchAttribute* attr, uint32_t grid, uint32_t ctas, size_t smem,
+                                 cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+}  // namespace
+
+uint32_t fp64MatrixRoom() { return roomWords(sizeof(DevCell)); }
+
 cudaError_t launchStepFp64(const DevCell& c, uint32_t nsteps, cudaStream_t st) {
-    hsStepFp64<<<1, 256, 0, st>>>(c, nsteps);
+    const uint32_t words = c.smWords <= fp64MatrixRoom() ? c.smWords : 0;
+    cudaError_t e = allowShared(hsStepFp64, 8 * (size_t)words);
+    if (e != cudaSuccess) return e;
+    hsStepFp64<<<1, c.N > 256 ? 512 : 256, 8 * (size_t)words, st>>>(c, words, nsteps);
     return cudaGetLastError();
 }
 
 cudaError_t launchStepFp64Cluster(const DevCell& c, uint32_t ctas, uint32_t nsteps, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
+    const uint32_t words = c.smWords <= fp64MatrixRoom() ? c.smWords : 0;
+    cudaError_t e = allowShared(hsStepFp64Cluster, 8 * (size_t)words);
+    if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, hsStepFp64Cluster, c, nsteps);
+    const cudaLaunchConfig_t cfg = clusterConfig(attr, ctas, ctas, 8 * (size_t)words, st);
+    return cudaLaunchKernelEx(&cfg, hsStepFp64Cluster, c, words, nsteps);
 }
 
-// `ctas` CTAs per solver: 1 = one CTA each (no cluster), 2..8 = a cluster each
-cudaError_t launchGroupStepFp64(const DevCell* cells, uint32_t n, uint32_t ctas, uint32_t nsteps,
+// `ctas` CTAs per solver: 1 = one CTA each (no cluster), 2..8 = a cluster
+// each; `words`: doubles of shared memory per CTA, the most that a member's
+// matrix needs (members that need more use global memory)
+cudaError_t launchGroupStepFp64(const DevCell* cells, uint32_t n, uint32_t ctas, uint32_t words, uint32_t nsteps,
                                 cudaStream_t st) {
     if (!n) return cudaSuccess;
+    const size_t smem = 8 * (size_t)words;
     if (ctas <= 1) {
-        hsGroupStepFp64<<<n, 256, 0, st>>>(cells, nsteps);
+        cudaError_t e = allowShared(hsGroupStepFp64, smem);
+        if (e != cudaSuccess) return e;
+        hsGroupStepFp64<<<n, 256, smem, st>>>(cells, words, nsteps);
         return cudaGetLastError();
     }
-    cudaLaunchConfig_t cfg = {};
+    cudaError_t e = allowShared(hsGroupStepFp64Cluster, smem);
+    if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(n * ctas);
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, hsGroupStepFp64Cluster, cells, nsteps);
+    const cudaLaunchConfig_t cfg = clusterConfig(attr, n * ctas, ctas, smem, st);
+    return cudaLaunchKernelEx(&cfg, hsGroupStepFp64Cluster, cells, words, nsteps);
 }
 
-cudaError_t launchBatchStepFp64(const DevCell* cells, const uint32_t* warpCellPtr,
-                                const uint32_t* warpCells, uint32_t nWarps, const uint32_t* ctaCellPtr,
-                                const uint32_t* ctaCells, uint32_t nsteps, uint32_t threadsPerCta,
+// Doubles of shared memory that the FP64 batch's CTA of `teams` teams has for
+// matrices.
+uint32_t fp64BatchWords(uint32_t teams) { return roomWords(teams * sizeof(DevCell)); }
+
+cudaError_t launchBatchStepFp64(const DevCell* cells, const uint32_t* wholePtr, const uint32_t* wholeCells,
+                                const uint32_t* teamPtr, const uint32_t* teamCells, uint32_t nBlocks,
+                                uint32_t teams, uint32_t teamThreads, uint32_t words, uint32_t nsteps,
                                 cudaStream_t st) {
-    uint32_t blocks = (nWarps * 32 + threadsPerCta - 1) / threadsPerCta;
-    hsBatchStepFp64<<<blocks, threadsPerCta, 0, st>>>(cells, warpCellPtr, warpCells, nWarps, ctaCellPtr, ctaCells,
-                                                      nsteps);
+    const size_t smem = teams * sizeof(DevCell) + 8 * (size_t)words;
+    cudaError_t e = allowShared(hsBatchStepFp64, smem);
+    if (e != cudaSuccess) return e;
+    hsBatchStepFp64<<<nBlocks, teams * teamThreads, smem, st>>>(cells, wholePtr, wholeCells, teamPtr, teamCells,
+                                                                teamThreads, words, nsteps);
     return cudaGetLastError();
-}
-
-int fp64BatchCtasPerSm(uint32_t threadsPerCta) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, hsBatchStepFp64, (int)threadsPerCta, 0) != cudaSuccess)
-        return 0;
-    return n;
 }
 
 cudaError_t launchReinitFp64(const DevCell* cells, uint32_t nCells, cudaStream_t st) {
