@@ -305,7 +305,7 @@ int repack(HsBatch* b) {
         const uint32_t n = (uint32_t)cells.size();
         uint32_t least = 0;
         for (uint32_t i = 0; i < n; ++i)
-            if (2 * (uint64_t)b->plans[cells[i]].N + b->plans[cells[i]].H > share) least = i + 1;
+            if (b->dcs[cells[i]].smWords > share) least = i + 1;
         // the cells after the first `k0` to the teams, longest first; estimated time
         std::vector<std::vector<uint32_t>> best, lists;
         double bestT = 0;

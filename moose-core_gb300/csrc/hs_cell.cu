@@ -1,4 +1,5 @@
 // hs_cell.cu -- upload of a CellPlan into a device arena (see hs_cell.h).
+#include <algorithm>
 #include <cstring>
 
 #include "hs_cell.h"
@@ -213,7 +214,12 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         Compact C;
         const bool compact = compactPrograms(P, C);
         if (!compact) C = Compact();
-        c.smWords = compact ? 2 * N + H : 0;
+        uint32_t longest = 0;      // runs walked as runs: forward only without waves
+        for (uint32_t r : P.bRun) longest = std::max(longest, r);
+        if (P.fWavePtr.empty())
+            for (uint32_t r : P.fRun) longest = std::max(longest, r);
+        c.runRows = longest >= kWarpRun ? longest : 0;
+        c.smWords = compact ? 2 * N + H + 2 * c.runRows : 0;
         c.fSplit = C.split;
         c.fW = u.put(C.fW);
         c.bW = u.put(C.bW);

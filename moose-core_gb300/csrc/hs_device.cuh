@@ -30,6 +30,7 @@ constexpr uint32_t kRecShift = 28;
 constexpr uint32_t kRecVm = 0, kRecIk = 1, kRecGk = 2, kRecCa = 3;
 
 // kinds of segments of the sweeps (DevCell::fSeg, bSeg)
+constexpr uint32_t kWarpRun = 64;       // rows from which a cable run is shared by a warp
 constexpr uint32_t kSegNarrow = 0x80000000u, kSegRun = 0x40000000u, kSegKind = kSegNarrow | kSegRun;
 
 struct DevCtl {
@@ -57,8 +58,8 @@ struct DevCell {
     const uint32_t *bLevelPtr, *bRows, *bTermPtr;
     const int2* bTerms;
     const uint32_t *fRun, *fRunRow, *bRun, *bRunRow;   // cable runs per level
-    // the sweeps in shared memory (16-bit entries; smWords = 2N + H doubles, 0:
-    // not built).  fW, two uint4 per fused update: {t1 | a1 << 16, t2 | a2 << 16,
+    // the sweeps in shared memory (16-bit entries; smWords = 2N + H doubles and
+    // the runs' scratch, 0: not built).  fW, two uint4 per fused update: {t1 | a1 << 16, t2 | a2 << 16,
     // l | p << 16, -}, {off-diagonal, -}.  bW, two per row of bRows: {row |
     // terms << 16, coefficient | source << 16 of the first three terms},
     // {off-diagonal, fourth term, first of the others in bX}.  fLane, bLane:
@@ -73,6 +74,7 @@ struct DevCell {
     const uint4 *fW, *bW, *fLane, *bLane;
     const uint2 *fSeg, *bSeg;
     uint32_t nfSeg, nbSeg;
+    uint32_t runRows;            // rows of the longest cable run a warp shares (0: none); 2 runRows doubles of smWords
     const uint32_t* bX;
     const uint32_t* fWavePtr;
     const int4* fWaveOps;        // per fused update: {t1, a1, t2, a2}, {l, p, -, -}

@@ -440,15 +440,166 @@ __device__ __forceinline__ void backwardCableRun(const double* M, const double* 
     }
 }
 
+// A long run shared by the lanes of a warp, with the serial walk's results.
+// Each lane walks a piece of the run from a guess of the value that enters
+// it, with the reference's operations; then every lane whose entry value is
+// not, bit for bit, the one its left neighbour came out with walks again
+// from that, until none is left.  By induction the first k pieces are final
+// after k rounds (the first starts from the given value), so the result is
+// the serial walk's whatever the guesses, in at most as many rounds as there
+// are pieces.  It takes few because a cable's sweeps forget: an error in a
+// pivot shrinks by q^2 per row, in a right-hand side or a voltage by q (the
+// quotient, ~0.67 on the 201-compartment cable), and once it is below half a
+// last place the two walks coincide.
+// A lone lane's row is bound by latency (~670 cycles forward, ~490 back) and an
+// FP64 instruction costs the same for one lane or 32: the 201-compartment
+// cable's sweeps take 134k + 98k cycles per step row by row, 32k + 21k shared.
+// From 64 rows: below that a piece is two rows or fewer.
+constexpr uint32_t kWarmRows = 20;      // rows before a piece that its FP32 guess of the pivot walks
+
+// Value of x as a float, cut; 0 outside the float range.
+__device__ __forceinline__ float cutFloat(double x) {
+    const uint32_t h = hiOf(x), e = (h >> 20) & 0x7FFu;
+    const uint32_t b = ((h & 0x7FFFFFFFu) - 0x38000000u) << 3 | loOf(x) >> 29;
+    return e - 897u < 253u ? __uint_as_float(b | (h & 0x80000000u)) : 0.f;
+}
+
+// Rounds of `walk(entry) -> exit` over the lanes' pieces; `active`: the lane
+// has one.  Returns with every piece walked from its left neighbour's exit.
+template <class Walk>
+__device__ __forceinline__ void settle(double entry, bool active, Walk walk) {
+    const uint32_t lane = threadIdx.x & 31u;
+    double out = entry;
+    bool go = active;
+    for (uint32_t round = 0; round < 33; ++round) {
+        if (go) out = walk(entry);
+        const double left = __shfl_up_sync(0xFFFFFFFFu, out, 1);
+        go = active && lane && bitsOf(left) != bitsOf(entry);
+        if (go) entry = left;
+        if (!__any_sync(0xFFFFFFFFu, go)) break;
+    }
+}
+
+// Entry values of the pieces from their affine maps x -> a x + b, x0 entering
+// the first (guesses, in plain FP64).
+__device__ __forceinline__ double affineEntry(double a, double b, double x0) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k = 1; k < 32; k <<= 1) {
+        const double pa = __shfl_up_sync(0xFFFFFFFFu, a, k), pb = __shfl_up_sync(0xFFFFFFFFu, b, k);
+        if (lane >= k) {
+            b = __fma_rn(a, pb, b);
+            a = a * pa;
+        }
+    }
+    const double end = __fma_rn(a, x0, b), left = __shfl_up_sync(0xFFFFFFFFu, end, 1);
+    return lane ? left : x0;
+}
+
+// Rows r .. r + run - 1 forward; `S`: scratch of 2 run doubles.
+__device__ __forceinline__ void forwardWarpRun(double* M, const double* off, uint32_t N, uint32_t r, uint32_t run,
+                                               double* S) {
+    const uint32_t lane = threadIdx.x & 31u, m = ((run + 31) / 32) | 1u;      // odd: no bank conflicts
+    const uint32_t s = min(lane * m, run), e = min(s + m, run);
+    const bool active = s < e;
+    const double d0 = M[r - 1];
+    double guess = d0;
+    if (lane && active) {
+        const uint32_t w = s > kWarmRows ? s - kWarmRows : 0u;
+        float x = w ? cutFloat(M[r + w - 1]) : cutFloat(d0);
+        for (uint32_t i = w; i < s; ++i) {
+            const float o = cutFloat(off[r + i - 1]);
+            x = cutFloat(M[r + i]) - __fdividef(o * o, x);
+        }
+        const uint32_t b = __float_as_uint(x);
+        guess = fromWords((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + 0x38000000u), b << 29);
+    }
+    double* Q = S + run;
+    settle(guess, active, [&](double d) {
+        double oNext = off[r + s - 1], dNext = M[r + s];
+        for (uint32_t i = s; i < e; ++i) {
+            const double o = oNext, dr = dNext;
+            if (i + 1 < e) {
+                oNext = off[r + i];
+                dNext = M[r + i + 1];
+            }
+            const double q = quotient(o, d);
+            d = dr - q * o;
+            S[i] = d;
+            Q[i] = q;
+        }
+        return d;
+    });
+    for (uint32_t i = s; i < e; ++i) M[r + i] = S[i];
+    // right-hand sides, with the quotients at hand
+    double a = 1.0, b = 0.0;
+    for (uint32_t i = s; i < e; ++i) {
+        b = __fma_rn(-Q[i], b, M[N + r + i]);
+        a = -Q[i] * a;
+    }
+    settle(affineEntry(a, b, M[N + r - 1]), active, [&](double x) {
+        double qNext = Q[s], rNext = M[N + r + s];
+        for (uint32_t i = s; i < e; ++i) {
+            const double q = qNext, rr = rNext;
+            if (i + 1 < e) {
+                qNext = Q[i + 1];
+                rNext = M[N + r + i + 1];
+            }
+            x = rr - q * x;
+            S[i] = x;
+        }
+        return x;
+    });
+    for (uint32_t i = s; i < e; ++i) M[N + r + i] = S[i];
+    __syncwarp();
+}
+
+// Rows i0, i0 - 1, .. (run of them) back; VMid over the right-hand sides.
+__device__ __forceinline__ void backwardWarpRun(double* M, const double* off, uint32_t N, uint32_t i0, uint32_t run,
+                                                double* S) {
+    const uint32_t lane = threadIdx.x & 31u, m = ((run + 31) / 32) | 1u;
+    const uint32_t s = min(lane * m, run), e = min(s + m, run);
+    const bool active = s < e;
+    double* R = M + N;
+    double a = 1.0, b = 0.0;
+    for (uint32_t j = s; j < e; ++j) {
+        const double d = M[i0 - j];
+        const Recip y = recip(d);
+        const double q = quotient(off[i0 - j], d, y);
+        b = __fma_rn(-q, b, quotient(R[i0 - j], d, y));
+        a = -q * a;
+    }
+    settle(affineEntry(a, b, R[i0 + 1]), active, [&](double x) {
+        double rNext = R[i0 - s], oNext = off[i0 - s], dNext = M[i0 - s];
+        for (uint32_t j = s; j < e; ++j) {
+            const double rr = rNext, o = oNext, d = dNext;
+            if (j + 1 < e) {
+                rNext = R[i0 - j - 1];
+                oNext = off[i0 - j - 1];
+                dNext = M[i0 - j - 1];
+            }
+            x = quotient(rr - o * x, d);
+            S[j] = x;
+        }
+        return x;
+    });
+    for (uint32_t j = s; j < e; ++j) R[i0 - j] = S[j];
+    __syncwarp();
+}
+
 // The level program of the forward sweep, for cells without waves (cables):
 // a row's updates in order, the rows of a level shared by the team.
-__device__ __forceinline__ void forwardLevels(const DevCell& c, double* M, const Team& t) {
+// `S`: scratch of the cell's runs in shared memory (DevCell::runRows), or null.
+__device__ __forceinline__ void forwardLevels(const DevCell& c, double* M, const Team& t, double* S) {
     const uint32_t N = c.N, offBase = 2 * N + c.H;
     const double* off = c.M + offBase;
     auto at = [&](int32_t e) { return (uint32_t)e >= offBase ? off[e - offBase] : M[e]; };
     for (uint32_t l = 0; l < c.fLevels; ++l) {
         if (const uint32_t run = c.fRun[l]) {
-            if (t.tid == 0) forwardCableRun(M, off, N, c.fRunRow[l], run);
+            if (S && run >= kWarpRun) {
+                if (t.tid < 32) forwardWarpRun(M, off, N, c.fRunRow[l], run, S);
+            } else if (t.tid == 0) {
+                forwardCableRun(M, off, N, c.fRunRow[l], run);
+            }
             teamSync(t);
             l += run - 1;
             continue;
@@ -611,23 +762,26 @@ __device__ __forceinline__ void eliminateShared(const DevCell& c, double* M, con
             teamSync(t);
         }
     }
-    if (!c.fWaves) forwardLevels(c, M, t);
+    double* S = c.runRows ? M + 2 * N + c.H : nullptr;
+    if (!c.fWaves) forwardLevels(c, M, t, S);
     // back substitution: narrow levels and cable runs by the first warp
     for (uint32_t sg = 0; sg < c.nbSeg; ++sg) {
-        const uint2 S = __ldg(c.bSeg + sg);
-        const uint32_t n = S.x & ~kSegKind;
-        if (S.x & kSegKind) {
+        const uint2 sgm = __ldg(c.bSeg + sg);
+        const uint32_t n = sgm.x & ~kSegKind;
+        if (sgm.x & kSegKind) {
             pend = true;
             if (!w0) {
                 others();
                 continue;
             }
-            if (S.x & kSegRun) {
-                if (t.tid == 0) backwardCableRun(M, c.M + 2 * N + c.H, M + N, N, S.y, n);
+            if (sgm.x & kSegRun) {
+                const double* off = c.M + 2 * N + c.H;
+                if (S && n >= kWarpRun) backwardWarpRun(M, off, N, sgm.y, n, S);
+                else if (t.tid == 0) backwardCableRun(M, off, M + N, N, sgm.y, n);
                 __syncwarp();
                 continue;
             }
-            uint32_t k = S.y + lane;
+            uint32_t k = sgm.y + lane;
             ProgOp next = progOp(c.bLane, k);
             for (uint32_t l = 0; l < n; ++l, k += 32) {
                 const ProgOp r = next;
@@ -639,7 +793,7 @@ __device__ __forceinline__ void eliminateShared(const DevCell& c, double* M, con
         }
         if (pend) teamSync(t);
         pend = false;
-        const uint32_t* ptr = c.bLevelPtr + S.y;
+        const uint32_t* ptr = c.bLevelPtr + sgm.y;
         uint32_t e = ptr[1], e1 = ptr[min(2u, n)], k = ptr[0] + t.tid;
         ProgOp next;
         if (k < e) next = progOp(c.bW, k);
@@ -687,7 +841,7 @@ __device__ void eliminateGlobal(const DevCell& c, const Team& t) {
         for (uint32_t k = c.fWavePtr[w] + t.tid; k < c.fWavePtr[w + 1]; k += t.nth) waveUpdate(c, M, k);
         teamSync(t);
     }
-    if (!c.fWaves) forwardLevels(c, M, t);
+    if (!c.fWaves) forwardLevels(c, M, t, nullptr);
     for (uint32_t l = 0; l < c.bLevels; ++l) {
         if (const uint32_t run = c.bRun[l]) {
             if (t.tid == 0) backwardCableRun(M, off, c.VMid, N, c.bRunRow[l], run);
@@ -959,7 +1113,7 @@ __global__ void __launch_bounds__(256, 2) hsGroupStepFp64(const DevCell* __restr
     stepCell<false>(c, nsteps, t, shared, sMatrix, shared ? sMatrix : c.M, 0, t.tid, t.nth);
 }
 
-__global__ void __launch_bounds__(256) hsGroupStepFp64Cluster(const DevCell* __restrict__ cells, uint32_t words,
+__global__ void __launch_bounds__(256, 2) hsGroupStepFp64Cluster(const DevCell* __restrict__ cells, uint32_t words,
                                                               uint32_t nsteps) {
     extern __shared__ double sMatrix[];
     __shared__ DevCell c;
