@@ -395,18 +395,21 @@ int hs_read_spikes(HsSolver* s, uint32_t* gen, double* time, uint32_t capacity,
 typedef struct HsBatch HsBatch;
 
 /* Launch shape of the batched kernel (0 keeps the current value).
- * FP64: one wave of ctas_per_sm x SM-count CTAs (fewer per SM if the
- * kernel's registers do not fit that many); a warp steps its cells one after
- * the other, and the cells too large to share a warp's load with others are
- * stepped by a whole CTA each.  Mixed: one CTA steps a forest of cells at a time; a forest
+ * FP64: one block per SM, of up to ctas_per_sm teams of threads_per_cta
+ * threads (512 threads in all); a team steps its cells one after the other,
+ * and a cell too large for a team's share is stepped by the whole block.  Mixed: one CTA steps a forest of cells at a time; a forest
  * holds its elimination arrays in the CTA's shared memory (30 B per node),
- * so ctas_per_sm and forest_nodes set the forest size.  Changing either (or
+ * so ctas_per_sm and forest_nodes set the forest size.  Cells of a CTA that do
+ * not fit one such forest are stepped as pairs of forests that keep 16 B per
+ * node there (CTAs of 640 threads or more, with eliminator warps), or else as
+ * several forests, the largest cells in global memory.  Changing either (or
  * max_ctas) on a mixed batch renumbers its nodes: its state, recording and
  * inject targets start over and hs_batch_reinit must follow. */
 typedef struct HsBatchTuning {
     uint32_t threads_per_cta;   /* multiple of 32; FP64 <= 256 (default 128),
                                    mixed <= 1024 (default 1024) */
-    uint32_t ctas_per_sm;       /* CTAs per SM (default 4 FP64, 1 mixed) */
+    uint32_t ctas_per_sm;       /* FP64: teams per SM (default 4);
+                                   mixed: CTAs per SM (default 1) */
     uint32_t steps_per_launch;  /* dt steps per kernel launch (default 100) */
     uint32_t use_graph;         /* capture a process() call as a CUDA graph */
     uint32_t forest_nodes;      /* mixed: most nodes per shared-memory forest
@@ -415,7 +418,9 @@ typedef struct HsBatchTuning {
                                    CTAs (0: ctas_per_sm x SM count); fewer,
                                    fuller forests leave SMs to other batches */
     uint32_t elim_warps;        /* mixed: warps of a CTA that eliminate while the
-                                   others assemble (default 4; 0 keeps the
+                                   others assemble (default 4 to 8 by forest size;
+                                   of a pair, warps per forest, at most a fifth
+                                   of the CTA, the default; 0 keeps the
                                    current value, 0xFFFFFFFF turns the split off) */
     uint32_t wait_rounds;       /* mixed: most sleep rounds (~128 ns each) an
                                    eliminator waits for one level's assembly
@@ -543,7 +548,8 @@ int hs_batch_stream(HsBatch* b, void** stream);
 int hs_batch_info(HsBatch* b, uint64_t* n_compt, uint32_t* n_ctas,
                   uint32_t* threads_per_cta, uint32_t* steps_per_launch);
 /* Mixed batch: how many elimination forests the packing made and how many
- * of them are eliminated in shared memory (the others in global memory);
+ * of them are eliminated in shared memory, in whole or with their pivots and
+ * right-hand sides (the others in global memory);
  * 0 and 0 for an FP64 batch. */
 int hs_batch_forests(HsBatch* b, uint32_t* n_forests, uint32_t* n_shared);
 /* Average duration (ms) of the stepping kernel launches timed with CUDA

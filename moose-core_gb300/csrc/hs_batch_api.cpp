@@ -36,11 +36,12 @@ namespace hsg {
 int setLastError(int code, const std::string& msg);
 cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, const uint32_t* ctaForests,
                                   uint32_t nCtas, uint32_t threadsPerCta, uint32_t smemBytes, uint32_t cap,
-                                  uint32_t elimWarps, uint32_t nsteps, cudaStream_t st);
+                                  uint32_t deep, uint32_t pairWarps, uint32_t elimWarps, uint32_t minLevels,
+                                  uint32_t maxLevels, uint32_t modes, uint32_t nsteps, cudaStream_t st);
 cudaError_t launchForestStepMixedCluster(const MixBatch& b, const uint32_t* ctaPtr, const uint32_t* ctaForests,
                                          uint32_t nClusters, uint32_t kC, uint32_t threadsPerCta,
                                          uint32_t smemBytes, uint32_t cap, uint32_t stageCap, uint32_t elimWarps,
-                                         uint32_t nsteps, cudaStream_t st);
+                                         uint32_t modes, uint32_t nsteps, cudaStream_t st);
 cudaError_t launchBatchReinitMixed(const MixBatch& b, uint32_t nNodes, const double* initVm, const float* c2dX0,
                                    const uint32_t* evStart, cudaStream_t st);
 cudaError_t launchScatterInject(double* const* addr, uint8_t* const* flag, const double* val, uint32_t n,
@@ -155,6 +156,12 @@ struct HsBatch {
     // mixed: forests per CTA, shared-memory forest capacity
     uint32_t *dCtaPtr = nullptr, *dCtaForests = nullptr;
     uint32_t mixCap = 0, mixSmem = 0;
+    uint32_t mixHalf = 0;               // nodes of the half-shared arrays
+    uint32_t mixDeep = 0;               // doubles of shared memory for deep forests' level offsets
+    uint32_t mixMinLevels = 0, mixLevels = 0, mixMaxNodes = 0;      // of the forests
+    uint32_t mixModes = 0;              // bits 1 << MixForest::shared (a cluster's: staged or not)
+    bool mixPairs = false;              // forests stepped in pairs
+    bool elimSet = false;               // elimWarps was asked for
     unsigned long long* dStopStep = nullptr;    // mixed: per-cell stop steps
     unsigned long long* dForestStop = nullptr;  // mixed: per-forest largest stop step
     std::vector<uint32_t> forestCellPtr, forestCellIdx;   // mixed: cells of each forest (host)
@@ -236,18 +243,29 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
     if (b->precision == HS_PREC_FP64)
         return launchBatchStepFp64(b->dDcs, b->dWholePtr, b->dWholeCells, b->dTeamPtr, b->dTeamCells, b->nBlocks,
                                    b->nTeams, b->threadsPerCta, b->batchWords, k, b->st);
-    const uint32_t ew = b->elimWarps && b->threadsPerCta > 32 * b->elimWarps ? b->elimWarps : 0;
+    uint32_t ew = b->elimWarps && b->threadsPerCta > 32 * b->elimWarps ? b->elimWarps : 0;
+    // Unless asked for a number, more eliminators for forests of wider levels:
+    // 4 up to 1,279 nodes, 8 from 2,048 (us per step with 4 / 6 / 8: 203 nodes
+    // 19.1 / 19.4 / 19.9, ~1,700 45.3 / 43.7 / 44.3, ~6,500 93.7 / 89.6 / 85.8).
+    if (ew && !b->elimSet && b->mixModes == 1u << kRowsShared)
+        ew = std::max<uint32_t>(4, std::min(b->mixMaxNodes / 256, b->threadsPerCta / 128));
     b->mb.waitRounds = b->waitRounds;
     if (b->clusterCtas > 1) {
-        // every forest is in global memory: twice the eliminator warps, as
+        // the cluster's forests are large: twice the eliminator warps, as
         // the one-CTA serving kernel gives its global forests
         const uint32_t ce = std::min<uint32_t>(2 * (ew ? ew : 4), std::min<uint32_t>(16, b->threadsPerCta / 64));
         return launchForestStepMixedCluster(b->mb, b->dCtaPtr, b->dCtaForests, b->nCtas, b->clusterCtas,
-                                            b->threadsPerCta, b->mixSmem, b->mixCap, b->mixStageCap, ce, k,
-                                            b->st);
+                                            b->threadsPerCta, b->mixSmem, b->mixCap, b->mixStageCap, ce,
+                                            b->mixModes, k, b->st);
     }
+    // Eliminators of each forest of a pair: 3/16 of the CTA (of 32 warps 6 each;
+    // a population of 1,024 cells: 4 124, 6 112, 8 125 us per step), fewer if
+    // asked for; none (split off, or too few threads): forest after forest.
+    const uint32_t pw = b->threadsPerCta / 160;
+    const uint32_t pairWarps = !b->mixPairs || !b->elimWarps ? 0 : b->elimSet ? std::min(b->elimWarps, pw) : pw;
     return launchForestStepMixed(b->mb, b->dCtaPtr, b->dCtaForests, b->nCtas, b->threadsPerCta, b->mixSmem,
-                                 b->mixCap, ew, k, b->st);
+                                 b->mixPairs ? b->mixHalf : b->mixCap, b->mixDeep, pairWarps, ew, b->mixMinLevels,
+                                 b->mixLevels, b->mixModes, k, b->st);
 }
 
 // Packing of the FP64 batch: one block per SM, in teams (hsBatchStepFp64).
@@ -545,9 +563,7 @@ int starTree(const CellPlan& P, StarTree& S) {
     return HS_OK;
 }
 
-// Shared-memory bytes per forest node: D, R, OFF (8 B), TOPO (4 B), PAR (2 B);
-// the kernel also keeps kSmemLevels level offsets and kWsLevels level
-// counters (4 B each) there.
+// Shared-memory bytes per forest node: D, R, OFF (8 B), TOPO (4 B), PAR (2 B).
 constexpr uint32_t kForestNodeBytes = 30;
 
 // The rate tables of a mixed batch: one V table and one Ca table for all
@@ -616,6 +632,30 @@ int unionTables(HsBatch* b, bool ca, UnionTable& U) {
     return HS_OK;
 }
 
+// Levels of a star tree.
+uint32_t treeLevels(const StarTree& S) {
+    uint32_t n = 0;
+    for (std::vector<uint32_t> cur{S.root}, next; !cur.empty(); cur.swap(next), ++n) {
+        next.clear();
+        for (uint32_t i : cur) next.insert(next.end(), S.ch.begin() + S.chPtr[i], S.ch.begin() + S.chPtr[i + 1]);
+    }
+    return n;
+}
+
+// The FP32 rate table as the mixed kernel reads it (MixBatch::vTab): per row
+// and species {A, B, dA, dB}, the differences to the next row rounded as the
+// interpolation would round them.
+std::vector<float> rowPairs(const UnionTable& U) {
+    std::vector<float> out;
+    for (uint32_t r = 0; r + 1 < U.nPts; ++r)
+        for (uint32_t k = 0; k < U.nCol; k += 2) {
+            const double* a = U.data.data() + (size_t)r * U.nCol + k;
+            const float A = (float)a[0], B = (float)a[1], A1 = (float)a[U.nCol], B1 = (float)a[U.nCol + 1];
+            out.insert(out.end(), {A, B, A1 - A, B1 - B});
+        }
+    return out;
+}
+
 int buildMixed(HsBatch* b) {
     const uint32_t nC = b->nCells;
     for (const CellPlan& P : b->plans)
@@ -636,20 +676,23 @@ int buildMixed(HsBatch* b) {
     if (ce != cudaSuccess) return cerr(ce, "shared memory size");
     const uint32_t perCta =
         std::min<uint32_t>((uint32_t)optin, (uint32_t)perSm / std::max<uint32_t>(1, b->ctasPerSm) - 1024) / 256 * 256;
-    const uint32_t reserve = (kSmemLevels + kWsLevels) * 4;
+    // (a cluster's forests have fewer than kWsLevels levels; small CTAs get
+    // room for no more either)
+    b->mixDeep = b->clusterCtas > 1 || perCta < 65536 ? 0 : kDeepDoubles;
+    const uint32_t reserve = kAreaBytes + b->mixDeep * 8;
     if (perCta < reserve + 8 * kForestNodeBytes) return berr(HS_EINVAL, "too many CTAs per SM");
     uint32_t cap = std::min<uint32_t>(kMaxForestNodes, (perCta - reserve) / kForestNodeBytes) / 8 * 8;
     // a cluster keeps only D and R (16 B a node) of its forest in rank 0's
     // shared memory, after the level offsets, counters and barrier word
-    const uint32_t reserveCl = (kSmemLevels + kWsLevels + 4) * 4;
-    if (b->clusterCtas > 1) cap = std::min<uint32_t>(kMaxForestNodes, (perCta - reserveCl) / 16) / 8 * 8;
+    if (b->clusterCtas > 1) cap = std::min<uint32_t>(kMaxForestNodes, (perCta - reserve) / 16) / 8 * 8;
     if (b->forestNodes) cap = std::min(cap, b->forestNodes / 8 * 8);
     if (cap < 8) return berr(HS_EINVAL, "forest_nodes too small");
     b->mixCap = cap;
     b->mixSmem = (reserve + cap * kForestNodeBytes + 15) / 16 * 16;
+    const uint32_t half = (perCta - reserve) / 16 / 2 * 2;     // nodes of half-shared forests
     if (b->clusterCtas > 1) {
-        b->mixSmem = reserveCl + 16 * cap;
-        b->mixStageCap = (b->mixSmem - reserveCl) / kForestNodeBytes / 8 * 8;
+        b->mixSmem = reserve + 16 * cap;
+        b->mixStageCap = (b->mixSmem - reserve) / kForestNodeBytes / 8 * 8;
         if (b->threadsPerCta <= 32 * (b->elimWarps ? b->elimWarps : 4))
             return berr(HS_EINVAL, "cluster_ctas: threads_per_cta must exceed the eliminator warps");
     }
@@ -686,24 +729,77 @@ int buildMixed(HsBatch* b) {
     }
     struct ForestPlan {
         std::vector<uint32_t> cells;
-        uint32_t nodes = 0;
-        bool shared = true;
+        uint32_t nodes = 0, rows = kRowsShared, mate = 0, slot = 0;
     };
+    // The cells of a CTA (in order of size) as pairs of forests, of at most
+    // `lim` nodes a pair: as few pairs as hold them, the cells spread evenly,
+    // the largest forest with the smallest.  Empty if a cell does not fit.
+    auto pairForests = [&](const std::vector<uint32_t>& cells, uint32_t lim) {
+        uint64_t total = 0;
+        for (uint32_t c : cells) total += trees[c].T;
+        auto fewer = [](const ForestPlan& x, const ForestPlan& y) { return x.nodes < y.nodes; };
+        for (size_t n = (total + lim - 1) / lim; 2 * n <= cells.size() + 1; ++n) {
+            std::vector<ForestPlan> bins(2 * n), out;
+            for (uint32_t c : cells) {
+                ForestPlan& f = *std::min_element(bins.begin(), bins.end(), fewer);
+                f.cells.push_back(c);
+                f.nodes += trees[c].T;
+            }
+            std::stable_sort(bins.rbegin(), bins.rend(), fewer);
+            bool fits = true;
+            for (size_t k = 0; k < n; ++k) {
+                ForestPlan &x = bins[k], &y = bins[2 * n - 1 - k];
+                x.rows = y.rows = kRowsHalf;
+                x.mate = y.nodes > 0;
+                y.slot = (x.nodes + 1) & ~1u;
+                fits = fits && y.slot + y.nodes <= lim;
+                out.push_back(std::move(x));
+                if (out.back().mate) out.push_back(std::move(y));
+            }
+            if (fits) return out;
+        }
+        return std::vector<ForestPlan>();
+    };
+    // Pairs where a CTA's cells do not fit one shared forest (1,024 cells, about
+    // 8,850 nodes a CTA: 112 us per step, 140 in two shared forests one after
+    // the other; 2,048 cells 223 and 250) or forest_nodes keeps them out of
+    // one (the 1,024 cells 112 and 156); a population that fits is as fast in
+    // a shared forest (7,000 nodes: 90 and 86 to 89), and forests of no more
+    // nodes than the CTA has threads, one pass of assembly with nothing to
+    // overlap, lose (250 nodes: 34 and 30).
+    std::vector<std::vector<ForestPlan>> pairsOf;
+    b->mixPairs = false;
+    if (b->mixDeep && b->elimWarps && b->threadsPerCta >= 640) {
+        for (uint32_t k = 0; k < nCtas; ++k) {
+            uint64_t total = 0;
+            for (uint32_t c : ctaCells[k]) total += trees[c].T;
+            b->mixPairs = b->mixPairs || total > std::max(cap, b->threadsPerCta);
+        }
+        for (uint32_t c = 0; b->mixPairs && c < nC; ++c) b->mixPairs = treeLevels(trees[c]) < kWsLevels;
+        for (uint32_t k = 0; b->mixPairs && k < nCtas; ++k) {
+            pairsOf.push_back(pairForests(ctaCells[k], half));
+            b->mixPairs = !pairsOf.back().empty() || ctaCells[k].empty();
+        }
+    }
     std::vector<ForestPlan> forests;
     std::vector<uint32_t> ctaPtr(nCtas + 1, 0), ctaForests;
     for (uint32_t k = 0; k < nCtas; ++k) {
         std::vector<ForestPlan> fs;
+        if (b->mixPairs) {
+            fs.swap(pairsOf[k]);
+            ctaCells[k].clear();
+        }
         for (uint32_t c : ctaCells[k]) {      // decreasing size
             const uint32_t T = trees[c].T;
-            const bool sh = T <= cap;
-            if (clustered && !sh)
+            const uint32_t rows = T <= cap ? kRowsShared : kRowsGlobal;
+            if (clustered && rows != kRowsShared)
                 return berr(HS_ENOTSUP, "mixed batch: a cell too large for a cluster's shared-memory forest");
-            const uint32_t lim = sh ? cap : kMaxForestNodes;
+            const uint32_t lim = rows == kRowsShared ? cap : kMaxForestNodes;
             size_t f = 0;
-            while (f < fs.size() && (fs[f].shared != sh || fs[f].nodes + T > lim)) ++f;
+            while (f < fs.size() && (fs[f].rows != rows || fs[f].nodes + T > lim)) ++f;
             if (f == fs.size()) {
                 fs.emplace_back();
-                fs.back().shared = sh;
+                fs.back().rows = rows;
             }
             fs[f].cells.push_back(c);
             fs[f].nodes += T;
@@ -728,6 +824,7 @@ int buildMixed(HsBatch* b) {
     std::vector<std::pair<uint32_t, uint32_t>> nodeCT;    // (cell, tree node) of each global node
     std::vector<uint8_t> nodeLevel;                       // forest level, capped at 255
     std::vector<MixForest> fdev(forests.size());
+    b->mixLevels = b->mixModes = b->mixHalf = b->mixMaxNodes = 0;
     std::vector<uint32_t> levelPtr, forestCells;
     for (size_t fi = 0; fi < forests.size(); ++fi) {
         const ForestPlan& FP = forests[fi];
@@ -738,7 +835,10 @@ int buildMixed(HsBatch* b) {
         F.level0 = (uint32_t)levelPtr.size();
         F.cell0 = (uint32_t)forestCells.size();
         F.nCells = (uint32_t)FP.cells.size();
-        F.shared = FP.shared ? 1 : 0;
+        F.shared = FP.rows;
+        F.mate = FP.mate;
+        F.slot = FP.slot;
+        if (FP.rows == kRowsHalf) b->mixHalf = std::max(b->mixHalf, (FP.slot + FP.nodes + 1) & ~1u);
         forestCells.insert(forestCells.end(), FP.cells.begin(), FP.cells.end());
         std::vector<std::pair<uint32_t, uint32_t>> cur, next;
         for (uint32_t c : FP.cells) {
@@ -766,10 +866,15 @@ int buildMixed(HsBatch* b) {
             cur.swap(next);
         }
         F.nLevels = (uint32_t)(levelPtr.size() - F.level0 - 1);
+        b->mixMinLevels = fi ? std::min(b->mixMinLevels, F.nLevels) : F.nLevels;
+        b->mixLevels = std::max(b->mixLevels, F.nLevels);
+        b->mixMaxNodes = std::max(b->mixMaxNodes, F.nNodes);
+        b->mixModes |= 1u << (!clustered ? F.shared : F.nNodes <= b->mixStageCap ? kRowsShared : kRowsHalf);
         if (nodeCT.size() - F.node0 != F.nNodes) return berr(HS_EINVAL, "mixed batch: forest layout failed");
         if (clustered && F.nLevels > kWsLevels - 1)
             return berr(HS_ENOTSUP, "mixed batch: a forest stepped by a cluster has more than 255 tree levels");
     }
+    if (b->mixPairs) b->mixSmem = reserve + 16 * b->mixHalf;
     const uint32_t nN = (uint32_t)nodeCT.size();
     // 4. per-cell lists: inject entries, stimulus, SpikeGens; model maps
     H.cells.resize(nC);
@@ -842,11 +947,10 @@ int buildMixed(HsBatch* b) {
         for (uint32_t k = 0; k < P.S; ++k) synIdx[ci][fill[P.synCompt[k]]++] = k;   // creation order per compartment
     }
     // 5. per-node arrays in global node order
-    std::vector<float> vtab(V0.data.begin(), V0.data.end()), catab(C0.data.begin(), C0.data.end());
+    const std::vector<float> vtab = rowPairs(V0), catab = rowPairs(C0);
     std::map<std::tuple<const double*, const double*, uint32_t, uint32_t>, int> g2dIndex;
-    std::vector<float> g2d, g2dGeom;
+    std::vector<float> g2d;
     std::vector<uint64_t> g2dOff;
-    std::vector<uint32_t> g2dN;
     struct ChanKey {          // a channel type with its general powers (for dedup)
         ChanType t;
         ChanPow p;
@@ -880,7 +984,7 @@ int buildMixed(HsBatch* b) {
             for (uint32_t k = S.chPtr[t]; k < S.chPtr[t + 1]; ++k) par[posOf[ci][S.ch[k]]] = (uint16_t)(g - F.node0);
             off[g] = S.off[t];
             HS2[g] = S.diag[t];
-            uint32_t info = (center ? kNodeCenter : 0) | ((uint32_t)kNoType << 8);
+            uint32_t info = (center ? kNodeCenter : 0) | kNoK2 << 8;
             uint32_t types = 0xFFFFFFFFu;
             syn0.push_back((uint32_t)synTypeV.size());
             if (!center) {
@@ -961,7 +1065,7 @@ int buildMixed(HsBatch* b) {
                     auto it = g2dIndex.find(key);
                     if (it == g2dIndex.end()) {
                         if (g2dIndex.size() >= 127) return berr(HS_ENOTSUP, "mixed batch: too many 2-D tables");
-                        const int gi = (int)g2dN.size() / 2;
+                        const int gi = (int)g2dOff.size();
                         const size_t nn = (size_t)G.nx * G.ny;
                         g2dOff.push_back(g2d.size());
                         const size_t o = g2d.size();
@@ -970,10 +1074,6 @@ int buildMixed(HsBatch* b) {
                             g2d[o + 2 * i] = (float)G.srcA[i];
                             g2d[o + 2 * i + 1] = (float)G.srcB[i];
                         }
-                        g2dGeom.insert(g2dGeom.end(), {(float)G.xmin, (float)G.ymin, (float)G.invDx, (float)G.invDy,
-                                                       (float)G.xmax, (float)G.ymax});
-                        g2dN.push_back(G.nx);
-                        g2dN.push_back(G.ny);
                         it = g2dIndex.emplace(key, gi).first;
                     }
                     C2dType ky;
@@ -988,10 +1088,18 @@ int buildMixed(HsBatch* b) {
                     ky.dep0 = dep(P.c2dDep0[kk]);
                     ky.dep1 = dep(P.c2dDep1[kk]);
                     ky.instant = (int8_t)P.c2dInstant[kk];
-                    ky.gate = (int8_t)it->second;
+                    ky.xmin = (float)G.xmin;
+                    ky.ymin = (float)G.ymin;
+                    ky.invDx = (float)G.invDx;
+                    ky.invDy = (float)G.invDy;
+                    ky.xmax = (float)G.xmax;
+                    ky.ymax = (float)G.ymax;
+                    ky.nx = G.nx;
+                    ky.ny = G.ny;
+                    ky.tab = g2dOff[it->second];
                     const int ti = typeIndex(ktypes, ky, kMaxC2dTypes - 1);
                     if (ti < 0) return berr(HS_ENOTSUP, "mixed batch: too many HHChannel2D types");
-                    info = (info & ~(0xFFu << 8)) | ((uint32_t)ti << 8);
+                    info = (info & ~(kNoK2 << 8)) | ((uint32_t)ti << 8);
                     k2gbar[g] = (float)(P.c2dGbar[kk] * P.c2dMod[kk]);
                     H.c2dNode[ci][kk] = g;
                     k2x0[g] = (float)P.c2dX0[kk];
@@ -1029,7 +1137,7 @@ int buildMixed(HsBatch* b) {
     H.c2dX0 = k2x0;
     H.nForests = (uint32_t)forests.size();
     H.nShared = 0;
-    for (const ForestPlan& f : forests) H.nShared += f.shared ? 1 : 0;
+    for (const ForestPlan& f : forests) H.nShared += f.rows != kRowsGlobal ? 1 : 0;
     trees.clear();
     // 6. upload
     DevBuf& D = b->buf;
@@ -1060,6 +1168,14 @@ int buildMixed(HsBatch* b) {
     m.nodeInfo = D.up(nodeInfo, st);
     m.ctype4 = D.up(ctype4, st);
     m.topo = D.up(topo, st);
+    std::vector<double2> offC(b->mixPairs || clustered ? nN : 0, make_double2(0.0, 0.0));
+    for (const MixForest& F : fdev)
+        for (uint32_t g = F.node0; !offC.empty() && g < F.node0 + F.nNodes; ++g) {
+            const uint32_t c0 = F.node0 + (topo[g] & 0xFFFF), nc = topo[g] >> 16 & 0xFF;
+            if (nc) offC[g].x = off[c0];
+            if (nc > 1) offC[g].y = off[c0 + 1];
+        }
+    m.offC = D.up(offC, st);
     m.par = D.up(par, st);
     m.injIdx = D.up(injIdx, st);
     m.off = D.up(off, st);
@@ -1067,7 +1183,7 @@ int buildMixed(HsBatch* b) {
     m.CmByDt = D.up(CmByDt, st);
     m.EmByRm = D.up(EmByRm, st);
     m.V = D.up(H.initVm, st);
-    if (H.nShared < H.nForests) {
+    if (b->mixModes & 1u << kRowsGlobal) {
         m.elimD = D.zeros<double>(nN, st);
         m.elimR = D.zeros<double>(nN, st);
     }
@@ -1085,9 +1201,6 @@ int buildMixed(HsBatch* b) {
     m.k2gbar = D.up(k2gbar, st);
     m.k2x = D.up(k2x0, st);
     m.g2d = D.up(g2d, st);
-    m.g2dOff = D.up(g2dOff, st);
-    m.g2dGeom = D.up(g2dGeom, st);
-    m.g2dN = D.up(g2dN, st);
     m.syn0 = D.up(syn0, st);
     m.synType = D.up(synTypeV, st);
     m.synX = D.zeros<float>(synTypeV.size(), st);
@@ -1145,11 +1258,11 @@ int buildMixed(HsBatch* b) {
     {
         uint32_t gateUse = 0, slotUse = 0, anyPool = 0, anyK2 = 0, anySyn = 0;
         for (uint32_t g = 0; g < nN; ++g) {
-            gateUse |= nodeInfo[g] >> kNodeGateShift;
+            gateUse |= (nodeInfo[g] >> kNodeGateShift) & 0xFFFu;
             for (int j = 0; j < kMaxChan; ++j)
                 if (((ctype4[g] >> (8 * j)) & 0xFF) != kNoType) slotUse |= 1u << j;
             anyPool |= nodeInfo[g] & kNodePool;
-            anyK2 |= ((nodeInfo[g] >> 8) & 0xFF) != kNoType;
+            anyK2 |= ((nodeInfo[g] >> 8) & kNoK2) != kNoK2;
             anySyn |= nodeInfo[g] & kNodeSyn;
         }
         auto add = [&](const void* p, uint32_t elem, uint64_t n) {
@@ -1179,11 +1292,20 @@ int buildMixed(HsBatch* b) {
             add(m.k2gbar, 4, nN);
         }
         if (anySyn) add(m.syn0, 4, nN + 1);
+        if (b->mixPairs) {
+            add(m.topo, 4, nN);
+            add(m.off, 8, nN);
+            add(m.offC, 16, nN);
+            add(m.par, 2, nN);
+        }
     }
     b->dCtaPtr = D.up(ctaPtr, st);
     b->dCtaForests = D.up(ctaForests, st);
     b->nCtas = busy;
     if (D.err != cudaSuccess) return cerr(D.err, "mixed batch upload");
+    // (whole tables: the kernel copies them into shared memory)
+    ktypes.resize(kMaxC2dTypes);
+    ctypes.resize(kMaxChanTypes);
     std::vector<ChanType> ctT;
     std::vector<ChanPow> ctP;
     for (const ChanKey& k : ctypes) {
@@ -1425,6 +1547,7 @@ int hs_batch_create(const HsCellDesc* cells, const uint32_t* seeds, uint32_t n_c
         if (tuning->steps_per_launch) b->stepsPerLaunch = tuning->steps_per_launch;
         b->forestNodes = tuning->forest_nodes;
         b->maxCtas = tuning->max_ctas;
+        b->elimSet = tuning->elim_warps != 0;
         if (tuning->elim_warps) b->elimWarps = tuning->elim_warps == 0xFFFFFFFFu ? 0 : tuning->elim_warps;
         if (tuning->wait_rounds) b->waitRounds = tuning->wait_rounds;
         if (tuning->cluster_ctas) b->clusterCtas = tuning->cluster_ctas;
@@ -1492,6 +1615,7 @@ int hs_batch_tune(HsBatch* b, const HsBatchTuning* t) {
     b->ctasPerSm = cps;
     b->forestNodes = t->forest_nodes;
     b->maxCtas = t->max_ctas;
+    if (t->elim_warps) b->elimSet = true;
     if (t->elim_warps) b->elimWarps = t->elim_warps == 0xFFFFFFFFu ? 0 : t->elim_warps;
     if (t->wait_rounds) b->waitRounds = t->wait_rounds;
     if (t->steps_per_launch) b->stepsPerLaunch = t->steps_per_launch;

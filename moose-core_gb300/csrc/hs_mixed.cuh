@@ -16,7 +16,10 @@
 // step of the elimination, so narrow levels of one cell fill up with the
 // levels of the others.  During elimination a forest keeps its pivots, right
 // hand sides and coupling topology in shared memory when it fits ("shared
-// forest"); otherwise in global scratch ("global forest").
+// forest", 30 B a node).  Where a CTA's cells do not fit one, it keeps pivots
+// and right hand sides there (16 B a node, "half-shared") and steps two
+// forests at once; what that does not hold is in global scratch ("global
+// forest").
 //
 // Per-node arrays: structure of arrays over all nodes (forest after forest),
 // with fixed "slots" so that a warp's loads are coalesced:
@@ -35,7 +38,7 @@
 namespace hsg {
 
 constexpr int kMaxChanTypes = 64;
-constexpr int kMaxC2dTypes = 16;
+constexpr int kMaxC2dTypes = 16;       // below kNoK2
 constexpr int kMaxSynTypes = 16;
 constexpr int kMaxChan = 4;            // channel slots per compartment
 constexpr uint8_t kNoType = 0xFF;
@@ -45,7 +48,8 @@ constexpr uint32_t kNodeCenter = 1u << 0;    // junction node, no membrane
 constexpr uint32_t kNodeInject = 1u << 1;    // has an inject entry
 constexpr uint32_t kNodePool = 1u << 2;      // has a Ca pool
 constexpr uint32_t kNodeSyn = 1u << 3;       // has SynChans
-// bits 8..15: HHChannel2D type (kNoType: none)
+// bits 8..12: HHChannel2D type (kNoK2: none)
+constexpr uint32_t kNoK2 = 31;
 // bits 16..27: gate present, bit kNodeGateShift + 3*slot + gate (X, Y, Z)
 constexpr uint32_t kNodeGateShift = 16;
 
@@ -71,10 +75,14 @@ struct C2dType {           // one HHChannel2D prototype
     int8_t xp;             // power 1..4, -1 general
     int8_t dep0, dep1;     // 0 Vm, 1 conc (the node's pool), -1 none
     int8_t instant;
-    int8_t gate;           // 2-D table
-    int8_t pad[3];
+    int8_t pad[4];
     float xpf;
+    // its 2-D table: bounds, 1 / spacing, points, first float of MixBatch::g2d
+    float xmin, ymin, invDx, invDy, xmax, ymax;
+    uint32_t nx, ny;
+    uint64_t tab;
 };
+static_assert(sizeof(C2dType) == 56 || sizeof(C2dType) == 64, "C2dType is copied in words");
 
 struct SynType {           // SynChan constants at the clock dt
     float xc1, xc2, yc1, yc2, ek;
@@ -82,8 +90,23 @@ struct SynType {           // SynChan constants at the clock dt
 
 constexpr uint32_t kNoParent = 0xFFFF;   // MixBatch::par of a root
 constexpr uint32_t kMaxForestNodes = 0xFFFF;
-constexpr uint32_t kSmemLevels = 1024;      // level offsets kept in shared memory
+constexpr uint32_t kTypeBytes = kMaxChanTypes * sizeof(ChanType) + kMaxC2dTypes * sizeof(C2dType) +
+                                kMaxSynTypes * sizeof(SynType);    // the prototypes, copied into shared memory
+constexpr uint32_t kSmemLevels = 1024;      // level offsets kept in shared memory where it is not short
 constexpr uint32_t kWsLevels = 256;         // per-level counters of the split step
+
+// Shared memory of the stepping kernels before a forest's arrays (hs_mixed.cu):
+// the prototypes, the words of the forests under way, level counters, the
+// cluster's barrier and kWsLevels level offsets; where there is room,
+// kDeepDoubles more hold up to kSmemLevels of them, or a pair's.
+constexpr uint32_t kCtlBytes = 128;
+constexpr uint32_t kAreaBytes = kTypeBytes + kCtlBytes + (2 * kWsLevels + 4) * 4;
+constexpr uint32_t kDeepDoubles = (kSmemLevels - kWsLevels) / 2;
+static_assert(kAreaBytes % 16 == 0 && kDeepDoubles % 2 == 0, "aligned arrays");
+
+// where a forest's elimination arrays are (MixForest::shared): in global memory;
+// all in shared memory; pivots and right-hand sides in shared memory ("half")
+constexpr uint32_t kRowsGlobal = 0, kRowsShared = 1, kRowsHalf = 2;
 
 // A forest: nodes [node0, node0 + nNodes), level offsets (forest-local)
 // levelPtr[level0 .. level0 + nLevels], cells forestCells[cell0 ..].
@@ -91,8 +114,9 @@ struct MixForest {
     uint32_t node0, nNodes;
     uint32_t level0, nLevels;
     uint32_t cell0, nCells;
-    uint32_t shared;             // 1: elimination arrays staged in shared memory
-    uint32_t pad;
+    uint32_t shared;             // kRowsGlobal, kRowsShared or kRowsHalf
+    uint32_t mate;               // 1: the CTA's next forest is stepped together with it
+    uint32_t slot;               // kRowsHalf: its first node's place in the shared arrays
 };
 
 // Per-cell entries of the inject, stimulus, SpikeGen and recording lists.
@@ -145,6 +169,7 @@ struct MixBatch {
     // per node (global index)
     const uint32_t* nodeInfo;    // flags, K(Ca) type, gate mask (bits above)
     const uint32_t* ctype4;      // 4 channel type bytes
+    const double2* offC;         // OFF of the first and second child (0 where there is none)
     const uint32_t* topo;        // forest-local first child | child count << 16 | level (<= 255) << 24
     const uint16_t* par;         // forest-local parent, kNoParent for a root
     uint32_t* err;               // set to 1 when a bounded wait gave up
@@ -163,9 +188,6 @@ struct MixBatch {
     const float* k2gbar;         // Gbar * modulation
     float* k2x;
     const float* g2d;            // interleaved (A,B) tables, FP32
-    const uint64_t* g2dOff;
-    const float* g2dGeom;        // xmin, ymin, invDx, invDy, xmax, ymax per table
-    const uint32_t* g2dN;        // nx, ny
     // SynChans
     const uint32_t* syn0;        // CSR (ld+1)
     const uint8_t* synType;
@@ -192,7 +214,8 @@ struct MixBatch {
     uint32_t* spikeCount;
     uint32_t* spikeGen;
     float* spikeTime;
-    // rate tables (FP32), A/B interleaved per species
+    // rate tables (FP32), per row and species {A, B, A of the next row - A, B
+    // of the next row - B}: one 16-byte read per gate
     const float* vTab;
     uint32_t vCol, vRows;
     float vMin, vMax, vInvDx;
