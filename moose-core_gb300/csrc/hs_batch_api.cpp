@@ -634,10 +634,13 @@ int unionTables(HsBatch* b, bool ca, UnionTable& U) {
 
 // Levels of a star tree.
 uint32_t treeLevels(const StarTree& S) {
+    std::vector<std::pair<uint32_t, uint32_t>> open{{S.root, 1}};     // node, its level + 1
     uint32_t n = 0;
-    for (std::vector<uint32_t> cur{S.root}, next; !cur.empty(); cur.swap(next), ++n) {
-        next.clear();
-        for (uint32_t i : cur) next.insert(next.end(), S.ch.begin() + S.chPtr[i], S.ch.begin() + S.chPtr[i + 1]);
+    while (!open.empty()) {
+        const auto [i, level] = open.back();
+        open.pop_back();
+        n = std::max(n, level);
+        for (uint32_t k = S.chPtr[i]; k < S.chPtr[i + 1]; ++k) open.push_back({S.ch[k], level + 1});
     }
     return n;
 }
@@ -647,6 +650,7 @@ uint32_t treeLevels(const StarTree& S) {
 // interpolation would round them.
 std::vector<float> rowPairs(const UnionTable& U) {
     std::vector<float> out;
+    out.reserve(2 * (size_t)U.nPts * U.nCol);
     for (uint32_t r = 0; r + 1 < U.nPts; ++r)
         for (uint32_t k = 0; k < U.nCol; k += 2) {
             const double* a = U.data.data() + (size_t)r * U.nCol + k;
