@@ -108,7 +108,11 @@ namespace {
 // must come before the solver's next group launch.
 cudaStream_t stOf(HsSolver* s) {
     if (s->group) {
-        cudaStreamWaitEvent(s->st, s->group->ev, 0);
+        // (a launch that is over needs no wait: of the reads after a group's
+        // step only the first waits, and 256 take 1 ms less)
+        const cudaError_t e = cudaEventQuery(s->group->ev);
+        if (e == cudaErrorNotReady) cudaGetLastError();
+        if (e != cudaSuccess) cudaStreamWaitEvent(s->st, s->group->ev, 0);
         s->group.reset();
     }
     s->queued = true;
@@ -874,8 +878,8 @@ int hs_read_vm(HsSolver* s, double* out, uint32_t n) {
     if (n != s->P.hinesOf.size()) return setErr(HS_EINVAL, "n must equal the model's compartment count");
     if (int rc = flushWrites(s)) return rc;
     std::vector<double> v(s->P.N);
+    // (a copy to pageable memory is done when the call returns)
     cudaError_t e = cudaMemcpyAsync(v.data(), s->dc.V, v.size() * 8, cudaMemcpyDeviceToHost, stOf(s));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stOf(s));
     if (e != cudaSuccess) return cudaErr(e, "read vm");
     for (uint32_t m = 0; m < n; ++m) out[m] = s->P.hinesOf[m] < 0 ? NAN : v[s->P.hinesOf[m]];
     return HS_OK;
@@ -887,7 +891,6 @@ int hs_read_ca(HsSolver* s, double* out, uint32_t n) {
     if (int rc = flushWrites(s)) return rc;
     std::vector<double> v(s->P.P + 1);
     cudaError_t e = cudaMemcpyAsync(v.data(), s->dc.ca, s->P.P * 8, cudaMemcpyDeviceToHost, stOf(s));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stOf(s));
     if (e != cudaSuccess) return cudaErr(e, "read ca");
     for (uint32_t m = 0; m < n; ++m) out[m] = s->P.poolSolverOf[m] < 0 ? NAN : v[s->P.poolSolverOf[m]];
     return HS_OK;

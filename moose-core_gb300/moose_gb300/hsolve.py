@@ -206,13 +206,13 @@ class HSolve:
 
     def vm(self):
         out = np.empty(self.model.n_compt)
-        _native.check(_native.load().hs_read_vm(self._h, out.ctypes.data_as(C.POINTER(C.c_double)), len(out)))
+        _native.check(_native.load().hs_read_vm(self._h, C.byref(C.c_double.from_buffer(out)), len(out)))
         return out
 
     def ca(self):
         out = np.empty(len(self.model.pool_compt))
         if len(out):
-            _native.check(_native.load().hs_read_ca(self._h, out.ctypes.data_as(C.POINTER(C.c_double)), len(out)))
+            _native.check(_native.load().hs_read_ca(self._h, C.byref(C.c_double.from_buffer(out)), len(out)))
         return out
 
     def dif(self):
