@@ -19,7 +19,7 @@ The JSON line carries:
              each) on a sample of the same cells, and the ratio to `value`;
   single_cell the FP64 drop-in on the single-cell case (soma + 200-compartment
              HH cable, 0.5 s), next to the same cell on one host core;
-  fp64_batch the FP64 batch (one warp per cell, the drop-in's arithmetic,
+  fp64_batch the FP64 batch (teams of threads, the drop-in's arithmetic,
              bit-identical results) on all cells of the workload;
   accuracy   max |dVm| (soma every dt step, every compartment every 1,000
              steps) and spike-time shift of the mixed batch against the FP64
@@ -603,7 +603,7 @@ def run_ours(args, rank, world, cpu_pool):
                                 "value": nc * args.dropin_steps / wall_g}}
             for h in hs:
                 h.close()
-        # the FP64 batch (warp per cell, the drop-in's arithmetic) on the same workload
+        # the FP64 batch (the drop-in's arithmetic) on the same workload
         fp64b = None
         if not args.skip_fp64_batch:
             f = Batch(cells, DT, HS_PREC_FP64, steps_per_launch=100)

@@ -413,7 +413,8 @@ typedef struct HsBatchTuning {
     uint32_t steps_per_launch;  /* dt steps per kernel launch (default 100) */
     uint32_t use_graph;         /* capture a process() call as a CUDA graph */
     uint32_t forest_nodes;      /* mixed: most nodes per shared-memory forest
-                                   (0: as many as shared memory holds) */
+                                   (0: as many as shared memory holds); a CTA's
+                                   larger cells are merged into one forest */
     uint32_t max_ctas;          /* mixed: pack the cells into at most this many
                                    CTAs (0: ctas_per_sm x SM count); fewer,
                                    fuller forests leave SMs to other batches */

@@ -689,6 +689,7 @@ int buildMixed(HsBatch* b) {
     // a cluster keeps only D and R (16 B a node) of its forest in rank 0's
     // shared memory, after the level offsets, counters and barrier word
     if (b->clusterCtas > 1) cap = std::min<uint32_t>(kMaxForestNodes, (perCta - reserve) / 16) / 8 * 8;
+    const uint32_t room = cap;                  // nodes of the largest shared forest
     if (b->forestNodes) cap = std::min(cap, b->forestNodes / 8 * 8);
     if (cap < 8) return berr(HS_EINVAL, "forest_nodes too small");
     b->mixCap = cap;
@@ -766,18 +767,16 @@ int buildMixed(HsBatch* b) {
     };
     // Pairs where a CTA's cells do not fit one shared forest (1,024 cells, about
     // 8,850 nodes a CTA: 112 us per step, 140 in two shared forests one after
-    // the other; 2,048 cells 223 and 250) or forest_nodes keeps them out of
-    // one (the 1,024 cells 112 and 156); a population that fits is as fast in
-    // a shared forest (7,000 nodes: 90 and 86 to 89), and forests of no more
-    // nodes than the CTA has threads, one pass of assembly with nothing to
-    // overlap, lose (250 nodes: 34 and 30).
+    // the other, 156 in one in global memory; 2,048 cells 223, 250 and 242).  A
+    // population that fits is as fast or faster in a shared forest (about
+    // 7,000 nodes: 86 us, 93 in pairs; 250 nodes: 27 and 34).
     std::vector<std::vector<ForestPlan>> pairsOf;
     b->mixPairs = false;
     if (b->mixDeep && b->elimWarps && b->threadsPerCta >= 640) {
         for (uint32_t k = 0; k < nCtas; ++k) {
             uint64_t total = 0;
             for (uint32_t c : ctaCells[k]) total += trees[c].T;
-            b->mixPairs = b->mixPairs || total > std::max(cap, b->threadsPerCta);
+            b->mixPairs = b->mixPairs || total > room;
         }
         for (uint32_t c = 0; b->mixPairs && c < nC; ++c) b->mixPairs = treeLevels(trees[c]) < kWsLevels;
         for (uint32_t k = 0; b->mixPairs && k < nCtas; ++k) {
@@ -809,6 +808,8 @@ int buildMixed(HsBatch* b) {
             fs[f].nodes += T;
         }
         for (ForestPlan& f : fs) {
+            // (cells that forest_nodes left out of shared forests, now merged)
+            if (f.rows == kRowsGlobal && f.nodes <= room) f.rows = kRowsShared;
             ctaForests.push_back((uint32_t)forests.size());
             forests.push_back(std::move(f));
         }
@@ -878,7 +879,25 @@ int buildMixed(HsBatch* b) {
         if (clustered && F.nLevels > kWsLevels - 1)
             return berr(HS_ENOTSUP, "mixed batch: a forest stepped by a cluster has more than 255 tree levels");
     }
-    if (b->mixPairs) b->mixSmem = reserve + 16 * b->mixHalf;
+    // No more shared memory than the forests need: the rest is L1, where the
+    // assembly's table rows and states are found again (one cell of 203
+    // compartments 17.3 us per step, 19.1 with all of it taken; 608 cells,
+    // about 5,700 nodes a CTA, 75 and 86).
+    uint32_t most[3] = {0, 8, 8};       // nodes by where the rows are
+    for (const MixForest& F : fdev) {
+        const uint32_t rows = !clustered ? F.shared : F.nNodes <= b->mixStageCap ? kRowsShared : kRowsHalf;
+        most[rows] = std::max(most[rows], (F.nNodes + 7) / 8 * 8);
+    }
+    if (b->mixPairs) {
+        b->mixSmem = reserve + 16 * b->mixHalf;
+    } else if (clustered) {
+        b->mixStageCap = most[kRowsShared];
+        b->mixCap = most[kRowsHalf];
+        b->mixSmem = reserve + (std::max(b->mixCap * 16, b->mixStageCap * kForestNodeBytes) + 15) / 16 * 16;
+    } else {
+        b->mixCap = most[kRowsShared];
+        b->mixSmem = reserve + (b->mixCap * kForestNodeBytes + 15) / 16 * 16;
+    }
     const uint32_t nN = (uint32_t)nodeCT.size();
     // 4. per-cell lists: inject entries, stimulus, SpikeGens; model maps
     H.cells.resize(nC);

@@ -219,7 +219,6 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.extPtr = u.put(P.extPtr);
     c.extList = u.put(P.extList);
     c.fLevelPtr = u.put(P.fLevelPtr);
-    c.fRows = u.put(P.fRows);
     c.fOpPtr = u.put(P.fOpPtr);
     c.fOps = reinterpret_cast<const int4*>(u.put(P.fOps));
     c.bLevelPtr = u.put(P.bLevelPtr);
@@ -352,7 +351,6 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.c2dVm = u.zeros<double>(P.K2);
     c.c2dC1 = u.zeros<double>(P.K2);
     c.c2dC2 = u.zeros<double>(P.K2);
-    c.synCompt = u.put(P.synCompt);
     c.synEk = u.put(P.synEk);
     c.synMod = u.put(P.synMod);
     c.synX = u.zeros<double>(P.S);

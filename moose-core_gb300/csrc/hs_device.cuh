@@ -53,7 +53,7 @@ struct DevCell {
     const uint32_t *chanPtr, *poolPtr, *extPtr;
     const int32_t* extList;
     // elimination programs
-    const uint32_t *fLevelPtr, *fRows, *fOpPtr;
+    const uint32_t *fLevelPtr, *fOpPtr;
     const int4* fOps;
     const uint32_t *bLevelPtr, *bRows, *bTermPtr;
     const int2* bTerms;
@@ -106,7 +106,6 @@ struct DevCell {
     double *c2dGbar, *c2dEk, *c2dXpow, *c2dMod, *c2dX, *c2dGk, *c2dVm, *c2dC1, *c2dC2;
     const double* c2dX0;         // X at reinit
     // SynChans
-    const uint32_t* synCompt;
     double *synEk, *synMod, *synX, *synY, *synAct, *synGk, *synXc1, *synXc2, *synYc1, *synYc2, *synNorm;
     const double* synConst;      // per SynChan: xc1, xc2, yc1, yc2, norm at the clock dt
     const uint32_t* evPtr;

@@ -51,11 +51,11 @@ def _run(cells, stops, tune=None, **tuning):
 
 # sizes (negative: a cable), forests of the paired layout
 LAYOUTS = [
-    ((1100,), 1),                           # a lone forest
-    ((900, 700), 2),
-    ((1500, 40, 25, 3), 2),                 # the second far smaller, narrower than a warp
+    ((8000,), 1),                           # a lone forest
+    ((5000, 4000), 2),
+    ((8000, 40, 25, 3), 2),                 # the second far smaller, narrower than a warp
     ((9000, 6000, 2000), 3),                # more than one pair's shared memory: a pair, then a lone forest
-    ((1200, -260), 1),                      # 256 levels or more: no pairs
+    ((8000, -260), 1),                      # 256 levels or more: no pairs
 ]
 
 
@@ -70,7 +70,7 @@ def test_paired_forests_bit_identical_to_global_forests(sizes, forests, stops):
 @pytest.mark.parametrize("tune", [dict(threads_per_cta=640), dict(threads_per_cta=160), dict(threads_per_cta=64),
                                   dict(elim_warps=1), dict(elim_warps=OFF)])
 def test_paired_layout_steps_with_any_tuning(tune):
-    cells = _cells((900, 700, 20))
+    cells = _cells((5000, 4000, 20))
     _same(_run(cells, True, tune=tune), _run(cells, True, elim_warps=OFF), 2)
 
 
