@@ -358,6 +358,13 @@ int repack(HsBatch* b) {
             teamPtr.push_back((uint32_t)teamCells.size());
         }
     }
+    // no more shared memory than these cells need: the rest is L1 (1,024 cells
+    // of 50 to 400 compartments 156 us per step, 166 with all of it taken)
+    uint32_t whole = 0, team = 0;
+    for (uint32_t c : wholeCells)
+        if (b->dcs[c].smWords <= b->batchWords) whole = std::max(whole, b->dcs[c].smWords);
+    for (uint32_t c : teamCells) team = std::max(team, b->dcs[c].smWords);
+    b->batchWords = std::max(whole, team * b->nTeams);
     b->dWholePtr = b->packBuf.up(wholePtr, b->st);
     b->dWholeCells = b->packBuf.up(wholeCells, b->st);
     b->dTeamPtr = b->packBuf.up(teamPtr, b->st);
