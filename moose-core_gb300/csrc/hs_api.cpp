@@ -61,7 +61,7 @@ struct HsSolver {
     bool queued = true;
     cudaEvent_t evQueued = nullptr;
     CellPlan P;
-    Arena arena;
+    Arena arena, spikes;
     DevCell dc;
     DevCell* dcDev = nullptr;    // device copy of dc (for the reinit kernel)
     double dt_ = 0;          // HSolve::dt_ (setup dt, clock dt after reinit)
@@ -312,13 +312,16 @@ int hs_create(const HsCellDesc* cell, uint32_t seed, double dt, int precision, H
         return cudaErr(e, "stream");
     }
     const uint32_t spikeCap = 1u << 16;
-    Arena dry;
-    layoutCell(s->P, dry, s->dc, spikeCap, stOf(s));
+    Arena dry, drySpikes;
+    layoutCell(s->P, dry, s->dc, spikeCap, stOf(s), nullptr, &drySpikes);
     dry.take<DevCell>(1);
     s->arena.size = dry.used + 256;
+    s->spikes.size = drySpikes.used;
     e = cudaMalloc(&s->arena.base, s->arena.size);
+    if (e == cudaSuccess) e = cudaMalloc(&s->spikes.base, s->spikes.size);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->arena.base, 0, s->arena.size, stOf(s));
-    if (e == cudaSuccess) e = layoutCell(s->P, s->arena, s->dc, spikeCap, stOf(s));
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->spikes.base, 0, s->spikes.size, stOf(s));
+    if (e == cudaSuccess) e = layoutCell(s->P, s->arena, s->dc, spikeCap, stOf(s), nullptr, &s->spikes);
     s->dcDev = s->arena.take<DevCell>(1);
     s->descPtr = s->dc.evPtr;
     s->descCur = s->dc.evCur;
@@ -344,6 +347,7 @@ int hs_destroy(HsSolver* s) {
     if (!s) return HS_OK;
     if (s->st) cudaStreamSynchronize(stOf(s));
     if (s->arena.base) cudaFree(s->arena.base);
+    if (s->spikes.base) cudaFree(s->spikes.base);
     if (s->recCompt) cudaFree(s->recCompt);
     if (s->recBuf) cudaFree(s->recBuf);
     if (s->ownIdx) cudaFree(s->ownIdx);

@@ -185,7 +185,7 @@ bool compactPrograms(const CellPlan& P, Compact& C) {
 }  // namespace
 
 cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCap,
-                       cudaStream_t st, const CellShared* sh) {
+                       cudaStream_t st, const CellShared* sh, Arena* spikes) {
     Uploader u{a, st};
     const uint32_t N = P.N, H = P.H;
     std::memset(&c, 0, sizeof(c));
@@ -373,8 +373,9 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.sgEdge = u.put(P.sgEdge);
     c.sgFired = u.zeros<int32_t>(P.SG);
     c.spikeCap = spikeCap;
-    c.spikeGen = u.zeros<uint32_t>(spikeCap);
-    c.spikeTime = u.zeros<double>(spikeCap);
+    Arena& sa = spikes ? *spikes : a;
+    c.spikeGen = sa.take<uint32_t>(spikeCap);
+    c.spikeTime = sa.take<double>(spikeCap);
     c.stimStep = u.put(P.stimStep);
     c.stimCompt = u.put(P.stimCompt);
     c.stimValue = u.put(P.stimValue);

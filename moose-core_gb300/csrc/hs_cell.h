@@ -28,7 +28,9 @@ struct Arena {
 // cell; fills `dc`.  Static arrays are copied with cudaMemcpyAsync on `st`.
 // A batch passes `shared`: device arrays it owns (initVm and SynChan
 // constants of all cells contiguous, for one-copy reinit) and rate tables
-// shared by the cells that have identical ones.
+// shared by the cells that have identical ones.  `spikes`: where the spike
+// buffers go, if not into `a` (a drop-in solver's: an allocation of more than
+// 1 MiB costs 57 us to make and free, two smaller ones 4).
 std::vector<double> pairTable(const Table& t);   // rate table as the FP64 kernels read it (DevCell::vTab)
 struct CellShared {
     double* initVm = nullptr;
@@ -39,7 +41,7 @@ struct CellShared {
     std::vector<uint64_t> g2dOff;    // per gate2d of the cell, offset from g2dBase
 };
 cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& dc, uint32_t spikeCap,
-                       cudaStream_t st, const CellShared* shared = nullptr);
+                       cudaStream_t st, const CellShared* shared = nullptr, Arena* spikes = nullptr);
 
 // SynChan reinit constants of one cell at the clock dt, 5 per SynChan
 // (xc1, xc2, yc1, yc2, norm), computed with the host libm as the reference does.
