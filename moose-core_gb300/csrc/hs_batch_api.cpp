@@ -157,7 +157,7 @@ struct HsBatch {
     uint32_t *dCtaPtr = nullptr, *dCtaForests = nullptr;
     uint32_t mixCap = 0, mixSmem = 0;
     uint32_t mixHalf = 0;               // nodes of the half-shared arrays
-    uint32_t mixPairNodes = 0;          // nodes of the largest pair of forests
+    uint32_t mixPairNodes = 0;          // nodes of a pair of forests, on average
     uint32_t mixDeep = 0;               // doubles of shared memory for deep forests' level offsets
     uint32_t mixMinLevels = 0, mixLevels = 0, mixMaxNodes = 0;      // of the forests
     uint32_t mixModes = 0;              // bits 1 << MixForest::shared (a cluster's: staged or not)
@@ -261,11 +261,11 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
     }
     // Eliminators of each forest of a pair: 3/16 of the CTA (of 32 warps 6 each;
     // a population of 1,024 cells, 8,850 nodes a pair: 4 124, 5 117, 6 112, 8
-    // 125 us per step; 2,048 cells 5 227, 6 222), of pairs of more than 12,288
-    // nodes, with their wider levels, one less (4,096 cells, up to 13,900 nodes: 5
-    // 406, 6 425); fewer if asked for; none (split off, or too few threads):
+    // 125 us per step; 2,048 cells 5 227, 6 222), of pairs of more than 10,240
+    // nodes, with their wider levels, one less (4,096 cells, 11,700 nodes: 5 406,
+    // 6 425); fewer if asked for; none (split off, or too few threads):
     // forest after forest.
-    const uint32_t pw = b->threadsPerCta / (b->mixPairNodes > 12288 ? 192 : 160);
+    const uint32_t pw = b->threadsPerCta / (b->mixPairNodes > 10240 ? 192 : 160);
     const uint32_t pairWarps = !b->mixPairs || !b->elimWarps ? 0 : b->elimSet ? std::min(b->elimWarps, pw) : pw;
     return launchForestStepMixed(b->mb, b->dCtaPtr, b->dCtaForests, b->nCtas, b->threadsPerCta, b->mixSmem,
                                  b->mixPairs ? b->mixHalf : b->mixCap, b->mixDeep, pairWarps, ew, b->mixMinLevels,
@@ -840,7 +840,7 @@ int buildMixed(HsBatch* b) {
     std::vector<std::pair<uint32_t, uint32_t>> nodeCT;    // (cell, tree node) of each global node
     std::vector<uint8_t> nodeLevel;                       // forest level, capped at 255
     std::vector<MixForest> fdev(forests.size());
-    b->mixLevels = b->mixModes = b->mixHalf = b->mixMaxNodes = b->mixPairNodes = 0;
+    b->mixLevels = b->mixModes = b->mixHalf = b->mixMaxNodes = 0;
     std::vector<uint32_t> levelPtr, forestCells;
     for (size_t fi = 0; fi < forests.size(); ++fi) {
         const ForestPlan& FP = forests[fi];
@@ -854,7 +854,6 @@ int buildMixed(HsBatch* b) {
         F.shared = FP.rows;
         F.mate = FP.mate;
         F.slot = FP.slot;
-        if (FP.slot) b->mixPairNodes = std::max(b->mixPairNodes, FP.slot + FP.nodes);
         if (FP.rows == kRowsHalf) b->mixHalf = std::max(b->mixHalf, (FP.slot + FP.nodes + 1) & ~1u);
         forestCells.insert(forestCells.end(), FP.cells.begin(), FP.cells.end());
         std::vector<std::pair<uint32_t, uint32_t>> cur, next;
@@ -901,6 +900,9 @@ int buildMixed(HsBatch* b) {
         most[rows] = std::max(most[rows], (F.nNodes + 7) / 8 * 8);
     }
     if (b->mixPairs) {
+        uint32_t pairs = 0;
+        for (const MixForest& F : fdev) pairs += F.slot == 0;
+        b->mixPairNodes = (uint32_t)nodeCT.size() / pairs;
         b->mixSmem = reserve + 16 * b->mixHalf;
     } else if (clustered) {
         b->mixStageCap = most[kRowsShared];
