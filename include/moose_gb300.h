@@ -401,8 +401,9 @@ typedef struct HsBatch HsBatch;
  * holds its elimination arrays in the CTA's shared memory (30 B per node),
  * so ctas_per_sm and forest_nodes set the forest size.  Cells of a CTA that do
  * not fit one such forest are stepped as pairs of forests that keep 16 B per
- * node there (CTAs of 640 threads or more, with eliminator warps), or else as
- * several forests, the largest cells in global memory.  Changing either (or
+ * node there (CTAs of 640 threads or more, with eliminator warps), more than
+ * two such pairs as one forest in global memory, or else as several forests,
+ * the largest cells in global memory.  Changing either (or
  * max_ctas) on a mixed batch renumbers its nodes: its state, recording and
  * inject targets start over and hs_batch_reinit must follow. */
 typedef struct HsBatchTuning {

@@ -248,6 +248,8 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
     // Unless asked for a number, more eliminators for forests of wider levels:
     // 4 up to 1,279 nodes, 8 from 2,048 (us per step with 4 / 6 / 8: 203 nodes
     // 19.1 / 19.4 / 19.9, ~1,700 45.3 / 43.7 / 44.3, ~6,500 93.7 / 89.6 / 85.8).
+    if (ew && !b->elimSet && b->mixModes == 1u << kRowsGlobal && b->threadsPerCta >= 640)
+        ew = b->threadsPerCta * 10 / 1024;      // (4,096 cells merged: 6 487, 8 419, 10 396)
     if (ew && !b->elimSet && b->mixModes == 1u << kRowsShared)
         ew = std::max<uint32_t>(4, std::min(b->mixMaxNodes / 256, b->threadsPerCta / 128));
     b->mb.waitRounds = b->waitRounds;
@@ -781,6 +783,11 @@ int buildMixed(HsBatch* b) {
     // the other, 156 in one in global memory; 2,048 cells 223, 250 and 242).  A
     // population that fits is as fast or faster in a shared forest (about
     // 7,000 nodes: 86 us, 93 in pairs; 250 nodes: 27 and 34).
+    // From three pairs on, one forest of all of a CTA's cells in global memory:
+    // its tail and back substitution are a small part by then, and nothing
+    // waits between the pairs (4,096 cells: 396 us per step with ten eliminator
+    // warps, 415 in pairs; 2,048 cells, two pairs: 229 and 221).
+    bool merge = false;
     std::vector<std::vector<ForestPlan>> pairsOf;
     b->mixPairs = false;
     if (b->mixDeep && b->elimWarps && b->threadsPerCta >= 640) {
@@ -788,8 +795,11 @@ int buildMixed(HsBatch* b) {
             uint64_t total = 0;
             for (uint32_t c : ctaCells[k]) total += trees[c].T;
             b->mixPairs = b->mixPairs || total > room;
+            merge = merge || total > 2 * half;
         }
         for (uint32_t c = 0; b->mixPairs && c < nC; ++c) b->mixPairs = treeLevels(trees[c]) < kWsLevels;
+        merge = merge && b->mixPairs && (!b->elimSet || b->elimWarps >= 10);   // (with 8: 419)
+        if (merge) b->mixPairs = false;
         for (uint32_t k = 0; b->mixPairs && k < nCtas; ++k) {
             pairsOf.push_back(pairForests(ctaCells[k], half));
             b->mixPairs = !pairsOf.back().empty() || ctaCells[k].empty();
@@ -805,7 +815,7 @@ int buildMixed(HsBatch* b) {
         }
         for (uint32_t c : ctaCells[k]) {      // decreasing size
             const uint32_t T = trees[c].T;
-            const uint32_t rows = T <= cap ? kRowsShared : kRowsGlobal;
+            const uint32_t rows = T <= cap && !merge ? kRowsShared : kRowsGlobal;
             if (clustered && rows != kRowsShared)
                 return berr(HS_ENOTSUP, "mixed batch: a cell too large for a cluster's shared-memory forest");
             const uint32_t lim = rows == kRowsShared ? cap : kMaxForestNodes;
@@ -820,7 +830,7 @@ int buildMixed(HsBatch* b) {
         }
         for (ForestPlan& f : fs) {
             // (cells that forest_nodes left out of shared forests, now merged)
-            if (f.rows == kRowsGlobal && f.nodes <= room) f.rows = kRowsShared;
+            if (f.rows == kRowsGlobal && f.nodes <= room && !merge) f.rows = kRowsShared;
             ctaForests.push_back((uint32_t)forests.size());
             forests.push_back(std::move(f));
         }

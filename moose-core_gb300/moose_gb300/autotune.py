@@ -27,7 +27,7 @@ from .abi import HS_PREC_FP64
 
 MIXED_SPACE = {
     # (ctas_per_sm, forest_nodes[, elim_warps])
-    "packing": [(1, 0), (1, 8, 8), (1, 6000), (1, 4096), (2, 0)],
+    "packing": [(1, 0), (1, 8, 8), (1, 0, 10), (1, 6000), (1, 4096), (2, 0)],
     "threads_per_cta": [1024, 768, 512],
     "elim_warps": [4, 5, 3, 8],
     "steps_per_launch": [100, 50, 200],

@@ -55,6 +55,7 @@ LAYOUTS = [
     ((5000, 4000), 2),
     ((8000, 40, 25, 3), 2),                 # the second far smaller, narrower than a warp
     ((9000, 6000, 2000), 3),                # more than one pair's shared memory: a pair, then a lone forest
+    ((12000, 9000, 8000), 1),               # more than two pairs' nodes: one forest in global memory
     ((8000, -260), 1),                      # 256 levels or more: no pairs
 ]
 
