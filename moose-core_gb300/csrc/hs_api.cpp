@@ -892,8 +892,9 @@ int hs_read_vm(HsSolver* s, double* out, uint32_t n) {
     if (n != s->P.hinesOf.size()) return setErr(HS_EINVAL, "n must equal the model's compartment count");
     if (int rc = flushWrites(s)) return rc;
     std::vector<double> v(s->P.N);
-    // (a copy to pageable memory is done when the call returns)
     cudaError_t e = cudaMemcpyAsync(v.data(), s->dc.V, v.size() * 8, cudaMemcpyDeviceToHost, stOf(s));
+    // (a copy to pageable memory may be under way when its call returns)
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
     if (e != cudaSuccess) return cudaErr(e, "read vm");
     for (uint32_t m = 0; m < n; ++m) out[m] = s->P.hinesOf[m] < 0 ? NAN : v[s->P.hinesOf[m]];
     return HS_OK;
@@ -905,6 +906,7 @@ int hs_read_ca(HsSolver* s, double* out, uint32_t n) {
     if (int rc = flushWrites(s)) return rc;
     std::vector<double> v(s->P.P + 1);
     cudaError_t e = cudaMemcpyAsync(v.data(), s->dc.ca, s->P.P * 8, cudaMemcpyDeviceToHost, stOf(s));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
     if (e != cudaSuccess) return cudaErr(e, "read ca");
     for (uint32_t m = 0; m < n; ++m) out[m] = s->P.poolSolverOf[m] < 0 ? NAN : v[s->P.poolSolverOf[m]];
     return HS_OK;

@@ -33,6 +33,9 @@ constexpr uint32_t kRecVm = 0, kRecIk = 1, kRecGk = 2, kRecCa = 3;
 constexpr uint32_t kWarpRun = 64;       // rows from which a cable run is shared by a warp
 constexpr uint32_t kSegNarrow = 0x80000000u, kSegRun = 0x40000000u, kSegKind = kSegNarrow | kSegRun;
 
+// Power codes: 0 the gate is absent, 1..4 that power, kPowGeneral any other.
+constexpr uint32_t kPowGeneral = 5;
+
 struct DevCtl {
     unsigned long long nSteps;   // steps since reinit
     uint32_t stimPtr;
@@ -161,9 +164,6 @@ __device__ __forceinline__ double recValue(const DevCell& c, uint32_t e) {
 
 // ---------------------------------------------------------------------------
 // FP64 helpers, reference order
-
-// Power codes: 0 the gate is absent, 1..4 that power, kPowGeneral any other.
-constexpr uint32_t kPowGeneral = 5;
 
 struct Row {
     uint32_t i;       // table row

@@ -1,0 +1,157 @@
+// A stand-in for the CUDA runtime and the kernel launches, for tests of the
+// host code (hs_api.cpp, hs_batch_api.cpp, hs_cell.cu) without a GPU
+// (tests/fake_gpu.py).  Device memory is host memory and all streams are one
+// queue.  What CUDA leaves open is taken at its worst: a copy between device
+// and pageable host memory, which "might be synchronous", reads and writes the
+// host's memory only when something waits for it (fake_lazy).
+#include <cuda_runtime.h>
+
+#include <cstdlib>
+#include <cstring>
+#include <deque>
+#include <functional>
+
+#include "hs_cell.h"
+#include "hs_mixed.cuh"
+#include "hs_noalloc.h"
+
+namespace {
+
+std::deque<std::function<void()>> g_queue;
+bool g_lazyRead = false, g_lazyWrite = false;      // device to host, host to device
+void drain() {
+    while (!g_queue.empty()) {
+        g_queue.front()();
+        g_queue.pop_front();
+    }
+}
+cudaError_t push(std::function<void()> f) {
+    g_queue.push_back(std::move(f));
+    return cudaSuccess;
+}
+void* grab(size_t n) { return std::aligned_alloc(256, (n + 255) / 256 * 256); }
+
+constexpr int kShared = 232448, kSharedSm = 233472, kSms = 152;
+
+}  // namespace
+
+extern "C" {
+
+void fake_lazy(int reads, int writes) {
+    drain();
+    g_lazyRead = reads;
+    g_lazyWrite = writes;
+}
+
+const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
+    *v = a == cudaDevAttrMultiProcessorCount ? kSms : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? kShared : kSharedSm;
+    return cudaSuccess;
+}
+cudaError_t cudaDeviceGetDefaultMemPool(cudaMemPool_t* p, int) { *p = nullptr; return cudaSuccess; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) { *p = grab(n); return cudaSuccess; }
+cudaError_t cudaFree(void* p) { drain(); std::free(p); return cudaSuccess; }
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return push([=] { std::free(p); }); }
+cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) { return push([=] { std::memset(p, v, n); }); }
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
+    push([=] { std::memcpy(d, s, n); });
+    if (!(k == cudaMemcpyDeviceToHost ? g_lazyRead : k == cudaMemcpyHostToDevice && g_lazyWrite)) drain();
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) {
+    drain();
+    std::memcpy(d, s, n);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStream_t)grab(1); return cudaSuccess; }
+cudaError_t cudaStreamDestroy(cudaStream_t s) { drain(); std::free(s); return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { drain(); return cudaSuccess; }
+cudaError_t cudaStreamQuery(cudaStream_t) { return g_queue.empty() ? cudaSuccess : cudaErrorNotReady; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) { *g = nullptr; return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) { *x = nullptr; return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)grab(1); return cudaSuccess; }
+cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { std::free(e); return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventQuery(cudaEvent_t) { return g_queue.empty() ? cudaSuccess : cudaErrorNotReady; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0; return cudaSuccess; }
+
+}  // extern "C"
+
+namespace hsg {
+
+// ---- FP64: the steps change nothing ------------------------------------------
+uint32_t fp64MatrixRoom() { return (kShared - sizeof(DevCell)) / 8; }
+uint32_t fp64BatchWords(uint32_t teams) { return (kShared - teams * sizeof(DevCell)) / 8; }
+cudaError_t launchStepFp64(const DevCell&, uint32_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t launchStepFp64Cluster(const DevCell&, uint32_t, uint32_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t launchGroupStepFp64(const DevCell*, uint32_t, uint32_t, uint32_t, uint32_t, cudaStream_t) {
+    return cudaSuccess;
+}
+cudaError_t launchBatchStepFp64(const DevCell*, const uint32_t*, const uint32_t*, const uint32_t*, const uint32_t*,
+                                uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, cudaStream_t) {
+    return cudaSuccess;
+}
+cudaError_t launchReinitFp64(const DevCell* cells, uint32_t n, cudaStream_t) {
+    return push([=] {
+        for (const DevCell* c = cells; c < cells + n; ++c) {
+            std::memcpy(c->V, c->initVm, c->N * 8);
+            std::memcpy(c->ca, c->CaBasal, c->P * 8);
+        }
+    });
+}
+cudaError_t launchScatterFields(const FieldWrite* w, uint32_t n, cudaStream_t) {
+    return push([=] {
+        for (uint32_t i = 0; i < n; ++i) std::memcpy(w[i].addr, &w[i].bits, w[i].size);
+    });
+}
+cudaError_t launchGatherValues(const void* const* src, uint32_t f32, uint64_t n, double* out, cudaStream_t) {
+    return push([=] {
+        for (uint64_t k = 0; k < n; ++k)
+            out[k] = f32 ? *static_cast<const float*>(src[k]) : *static_cast<const double*>(src[k]);
+    });
+}
+cudaError_t launchSpikeCountsFp64(const DevCell*, uint32_t, uint32_t*, cudaStream_t) { return cudaSuccess; }
+cudaError_t launchGatherSpikes(const DevCell*, const uint32_t*, const float*, uint32_t, uint32_t, const uint32_t*,
+                               uint32_t*, double*, cudaStream_t) {
+    return cudaSuccess;
+}
+
+// ---- mixed ---------------------------------------------------------------------
+cudaError_t launchForestStepMixed(const MixBatch&, const uint32_t*, const uint32_t*, uint32_t, uint32_t, uint32_t,
+                                  uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t,
+                                  cudaStream_t) {
+    return cudaSuccess;
+}
+cudaError_t launchForestStepMixedCluster(const MixBatch&, const uint32_t*, const uint32_t*, uint32_t, uint32_t,
+                                         uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t,
+                                         cudaStream_t) {
+    return cudaSuccess;
+}
+cudaError_t launchBatchReinitMixed(const MixBatch&, uint32_t, const double*, const float*, const uint32_t*,
+                                   cudaStream_t) {
+    return cudaSuccess;
+}
+cudaError_t launchScatterInject(double* const*, uint8_t* const*, const double*, uint32_t, cudaStream_t) {
+    return cudaSuccess;
+}
+cudaError_t launchScatterValues(const ValueWrite*, uint32_t, cudaStream_t) { return cudaSuccess; }
+std::mutex& injectStaticLock() {
+    static std::mutex m;
+    return m;
+}
+InjectWrite* injectStaging() { return nullptr; }
+cudaError_t scatterInjectStatic(int, uint32_t, cudaStream_t) { return cudaSuccess; }
+
+}  // namespace hsg
