@@ -393,8 +393,9 @@ uint32_t deliveryStep(double t, double dt) {
 
 int buildFp64(HsBatch* b, const HsCellDesc* cells) {
     const uint32_t nC = b->nCells;
-    // shared V/Ca tables by content, 2-D tables by source identity
-    std::map<std::pair<uint64_t, size_t>, const double*> tabDev;
+    // shared V/Ca tables by content and columns (pairTable's differences
+    // depend on both), 2-D tables by source identity
+    std::map<std::tuple<uint64_t, size_t, uint32_t>, const double*> tabDev;
     std::map<std::tuple<const double*, const double*, uint32_t, uint32_t>, uint64_t> g2dIndex;
     std::vector<double> g2dHost;
     std::vector<std::vector<uint64_t>> g2dOffs(nC);
@@ -422,7 +423,7 @@ int buildFp64(HsBatch* b, const HsCellDesc* cells) {
     for (uint32_t c = 0; c < nC; ++c) {
         for (int pass = 0; pass < 2; ++pass) {
             const Table& T = pass ? b->plans[c].caTable : b->plans[c].vTable;
-            auto key = std::make_pair(fnv(T.data.data(), T.data.size() * 8), T.data.size());
+            auto key = std::make_tuple(fnv(T.data.data(), T.data.size() * 8), T.data.size(), T.nCol);
             auto it = tabDev.find(key);
             if (it == tabDev.end()) it = tabDev.emplace(key, b->buf.up(pairTable(T), b->st)).first;
             (pass ? catab : vtab)[c] = it->second;
@@ -609,7 +610,7 @@ int unionTables(HsBatch* b, bool ca, UnionTable& U) {
             return berr(HS_ENOTSUP, std::string("mixed batch: the cells' ") + (ca ? "Ca" : "V") +
                                         " rate tables lie on different grids (min, max, divisions)");
         }
-        const auto key = std::make_pair(fnv(T.data.data(), T.data.size() * 8), T.data.size());
+        const auto key = std::make_tuple(fnv(T.data.data(), T.data.size() * 8), T.data.size(), T.nCol);
         auto it = byTable.find(key);
         if (it == byTable.end()) {
             std::vector<int32_t> map(T.nCol, -1);

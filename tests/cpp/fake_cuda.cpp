@@ -31,6 +31,9 @@ cudaError_t push(std::function<void()> f) {
 }
 void* grab(size_t n) { return std::aligned_alloc(256, (n + 255) / 256 * 256); }
 
+const hsg::DevCell* g_cells = nullptr;      // of the last reinit
+uint32_t g_nCells = 0;
+
 constexpr int kShared = 232448, kSharedSm = 233472, kSms = 152;
 
 }  // namespace
@@ -41,6 +44,15 @@ void fake_lazy(int reads, int writes) {
     drain();
     g_lazyRead = reads;
     g_lazyWrite = writes;
+}
+
+// Cell k's rate table on Vm as the last reinit had it: {columns, rows} and its data.
+const double* fake_table(uint32_t k, uint32_t* shape) {
+    drain();
+    if (k >= g_nCells) return nullptr;
+    shape[0] = g_cells[k].vCol;
+    shape[1] = g_cells[k].vRows;
+    return g_cells[k].vTab;
 }
 
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
@@ -104,6 +116,8 @@ cudaError_t launchBatchStepFp64(const DevCell*, const uint32_t*, const uint32_t*
     return cudaSuccess;
 }
 cudaError_t launchReinitFp64(const DevCell* cells, uint32_t n, cudaStream_t) {
+    g_cells = cells;
+    g_nCells = n;
     return push([=] {
         for (const DevCell* c = cells; c < cells + n; ++c) {
             std::memcpy(c->V, c->initVm, c->N * 8);

@@ -44,6 +44,8 @@ def load():
     try:
         L = _native.load()
         L.fake_lazy.argtypes = [C.c_int, C.c_int]
+        L.fake_table.argtypes = [C.c_uint32, C.POINTER(C.c_uint32)]
+        L.fake_table.restype = C.POINTER(C.c_double)
         yield L
         L.fake_lazy(0, 0)
     finally:

@@ -1,10 +1,14 @@
 """The host code without a GPU, on a stand-in for the CUDA runtime that takes
 what CUDA leaves open at its worst (tests/cpp/fake_cuda.cpp)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 import fake_gpu
 from moose_gb300 import models
+from moose_gb300.abi import HS_PREC_FP64
+from moose_gb300.batch import Batch
 from moose_gb300.hsolve import HSolve
 
 DT = 25e-6
@@ -33,3 +37,29 @@ def test_reads_wait_for_their_copy(gpu):
     assert np.array_equal(h.vm(), m.initVm)
     assert np.array_equal(h.ca(), m.pool_CaBasal)
     h.close()
+
+
+def test_batch_shares_rate_tables_of_one_shape_only(gpu):
+    """Two cells of an FP64 batch whose rate tables hold the same numbers, in
+    30 rows of one gate and in 10 of three: each gets the rows and differences
+    of its own shape (in the other's, the last rows are out of range)."""
+    cells = []
+    for species, divs in ((1, 28), (3, 8)):
+        m = models.config1_cell(n_cable=3)          # Na (gates 0, 1) and K (gate 2) in turn
+        m.gates = [(models.VMIN, models.VMAX, np.full(divs + 1, 2.0), np.full(divs + 1, 4.0))] * 3
+        if species == 1:
+            for name in [a for a in vars(m) if a.startswith("chan_")]:
+                setattr(m, name, getattr(m, name)[1::2].copy())
+        cells.append(m)
+    b = Batch(cells, DT, HS_PREC_FP64)
+    b.reinit(DT)
+    shape = (C.c_uint32 * 2)()
+    at = []
+    for k, (cols, rows) in enumerate([(2, 30), (6, 10)]):
+        p = gpu.fake_table(k, shape)
+        assert tuple(shape) == (cols, rows)
+        got = np.ctypeslib.as_array(p, (rows - 1, cols, 2))
+        assert np.array_equal(got, np.tile([[2.0, 0.0], [4.0, 0.0]], (rows - 1, cols // 2, 1)))
+        at.append(C.addressof(p.contents))
+    assert at[0] != at[1]
+    b.close()
