@@ -610,7 +610,7 @@ int unionTables(HsBatch* b, bool ca, UnionTable& U) {
             return berr(HS_ENOTSUP, std::string("mixed batch: the cells' ") + (ca ? "Ca" : "V") +
                                         " rate tables lie on different grids (min, max, divisions)");
         }
-        const auto key = std::make_tuple(fnv(T.data.data(), T.data.size() * 8), T.data.size(), T.nCol);
+        const auto key = std::make_pair(fnv(T.data.data(), T.data.size() * 8), T.data.size());
         auto it = byTable.find(key);
         if (it == byTable.end()) {
             std::vector<int32_t> map(T.nCol, -1);
