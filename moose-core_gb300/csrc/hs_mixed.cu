@@ -621,10 +621,14 @@ __device__ __forceinline__ void groupSync(uint32_t id, uint32_t count) {
 
 // A counter in shared memory that orders what its threads wrote before
 // (release) and read after (acquire), within the CTA: a full fence would also
-// wait for the reads a thread has under way.
+// wait for the reads a thread has under way.  kCluster: threads of the
+// cluster's other CTAs add to it too.
+template <bool kCluster>
 __device__ __forceinline__ uint32_t loadAcquire(const uint32_t* p) {
     uint32_t v;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    if (kCluster) asm volatile("ld.acquire.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    else asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
 __device__ __forceinline__ void addRelease(uint32_t* p, uint32_t v) {
@@ -638,10 +642,11 @@ __device__ __forceinline__ void addRelease(uint32_t* p, uint32_t v) {
 // set by another CTA, waits no more in this launch: the launch then ends
 // after at most one bounded wait per eliminator thread, and its results are
 // marked invalid (hs_batch_sync returns HS_ETIMEOUT).
+template <bool kCluster = false>
 __device__ __forceinline__ bool waitLevel(const MixBatch& b, const uint32_t* done, uint32_t need, bool& gaveUp) {
     if (gaveUp) return false;
     uint32_t rounds = 0;
-    while (loadAcquire(done) < need) {
+    while (loadAcquire<kCluster>(done) < need) {
         ++rounds;
         if (rounds > b.waitRounds || ((rounds & 1023u) == 0 && *(volatile const uint32_t*)b.err)) {
             atomicExch(b.err, 1u);
@@ -875,7 +880,7 @@ __device__ __forceinline__ void forwardHalf(const MixBatch& b, const HalfRows& E
     if (i < e) q = pullIn(b, E.node0 + i);
     for (int L = (int)nL - 1; L >= 0; --L) {
         const bool narrow = 2 * (e - b0) <= nE;
-        waitLevel(b, &done[L], e - b0, gaveUp);
+        waitLevel<kCluster>(b, &done[L], e - b0, gaveUp);
         if (kCluster) fenceCluster();
         for (;; i += nE) {
             const bool last = i + nE >= e;       // of this level
@@ -1329,7 +1334,7 @@ __device__ __forceinline__ void stepForestCluster(const MixBatch& b, const MixFo
             } else {
                 for (int L = (int)F.nLevels - 1; L >= 0; --L) {
                     const uint32_t b0 = lp[L], e = lp[L + 1];
-                    waitLevel(b, &done[L], e - b0, waitGaveUp);
+                    waitLevel<true>(b, &done[L], e - b0, waitGaveUp);
                     fenceCluster();
                     if (2 * (e - b0) <= nE) {
                         pullNarrow(E, b0, e, tid);

@@ -57,6 +57,28 @@ def test_clustered_batch_bit_identical_to_one_cta(ctas):
     assert len(ref["spikes"][2]) > 0
 
 
+@pytest.mark.parametrize("n", [1800, 6000, 9001])
+@pytest.mark.parametrize("ctas", [2, 8])
+def test_lone_clustered_cell_bit_identical_to_one_cta(n, ctas):
+    """A batch of one kind of forest: with all its arrays in rank 0's shared
+    memory (up to ~7,490 nodes), and with pivots and right-hand sides only."""
+    rng = np.random.default_rng([43, n])
+    parent, d, L = models.branched_morphology(rng, n, 0.5, 4)
+    cell = models.active_cell(parent, d, L, inject=0.8e-9, n_syn=40, rng=rng, t_end=0.02, syn_rate=60.0,
+                              kca_tables=models.kca_2d_tables(vdivs=300, cadivs=300))
+    out = []
+    for kw in (dict(), dict(cluster_ctas=ctas)):
+        b = Batch([cell], DT, HS_PREC_MIXED, **kw)
+        b.reinit(DT)
+        for k in (1, 299):
+            b.process(k)
+        b.sync()
+        out.append((b.vm(0), b.ca(0), b.spikes()[2]))
+        b.close()
+    for x, y in zip(*out):
+        assert np.array_equal(x, y)
+
+
 def test_cluster_option_is_checked():
     cells = _cells()[:2]
     with pytest.raises(_native.HsError):
