@@ -20,6 +20,7 @@
 #include "../../include/moose_gb300.h"
 #include "hs_device.cuh"
 #include "hs_plan.h"
+#include "hs_shared.h"
 
 namespace hsg {
 
@@ -1343,12 +1344,6 @@ uint32_t roomWords(size_t statics) {
     return (size_t)optin > statics ? (uint32_t)(((size_t)optin - statics) / 8) : 0;
 }
 
-template <class K>
-cudaError_t allowShared(K kernel, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
-
 cudaLaunchConfig_t clusterConfig(cudaLaunchAttribute* attr, uint32_t grid, uint32_t ctas, size_t smem,
                                  cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
@@ -1371,7 +1366,7 @@ uint32_t fp64MatrixRoom() { return roomWords(sizeof(DevCell)); }
 
 cudaError_t launchStepFp64(const DevCell& c, uint32_t nsteps, cudaStream_t st) {
     const uint32_t words = c.smWords <= fp64MatrixRoom() ? c.smWords : 0;
-    cudaError_t e = allowShared(hsStepFp64, 8 * (size_t)words);
+    cudaError_t e = allowShared((const void*)hsStepFp64);
     if (e != cudaSuccess) return e;
     hsStepFp64<<<1, c.N > 256 ? 512 : 256, 8 * (size_t)words, st>>>(c, words, nsteps);
     return cudaGetLastError();
@@ -1379,7 +1374,7 @@ cudaError_t launchStepFp64(const DevCell& c, uint32_t nsteps, cudaStream_t st) {
 
 cudaError_t launchStepFp64Cluster(const DevCell& c, uint32_t ctas, uint32_t nsteps, cudaStream_t st) {
     const uint32_t words = c.smWords <= fp64MatrixRoom() ? c.smWords : 0;
-    cudaError_t e = allowShared(hsStepFp64Cluster, 8 * (size_t)words);
+    cudaError_t e = allowShared((const void*)hsStepFp64Cluster);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = clusterConfig(attr, ctas, ctas, 8 * (size_t)words, st);
@@ -1394,12 +1389,12 @@ cudaError_t launchGroupStepFp64(const DevCell* cells, uint32_t n, uint32_t ctas,
     if (!n) return cudaSuccess;
     const size_t smem = 8 * (size_t)words;
     if (ctas <= 1) {
-        cudaError_t e = allowShared(hsGroupStepFp64, smem);
+        cudaError_t e = allowShared((const void*)hsGroupStepFp64);
         if (e != cudaSuccess) return e;
         hsGroupStepFp64<<<n, 256, smem, st>>>(cells, words, nsteps);
         return cudaGetLastError();
     }
-    cudaError_t e = allowShared(hsGroupStepFp64Cluster, smem);
+    cudaError_t e = allowShared((const void*)hsGroupStepFp64Cluster);
     if (e != cudaSuccess) return e;
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg = clusterConfig(attr, n * ctas, ctas, smem, st);
@@ -1415,7 +1410,7 @@ cudaError_t launchBatchStepFp64(const DevCell* cells, const uint32_t* wholePtr, 
                                 uint32_t teams, uint32_t teamThreads, uint32_t words, uint32_t nsteps,
                                 cudaStream_t st) {
     const size_t smem = teams * sizeof(DevCell) + 8 * (size_t)words;
-    cudaError_t e = allowShared(hsBatchStepFp64, smem);
+    cudaError_t e = allowShared((const void*)hsBatchStepFp64);
     if (e != cudaSuccess) return e;
     hsBatchStepFp64<<<nBlocks, teams * teamThreads, smem, st>>>(cells, wholePtr, wholeCells, teamPtr, teamCells,
                                                                 teamThreads, words, nsteps);

@@ -27,6 +27,7 @@
 
 #include "hs_exact.cuh"
 #include "hs_mixed.cuh"
+#include "hs_shared.h"
 
 namespace hsg {
 
@@ -1453,7 +1454,7 @@ cudaError_t launchForestStepMixedCluster(const MixBatch& b, const uint32_t* ctaP
     constexpr uint32_t S = 1u << kRowsShared, H = 1u << kRowsHalf;
     auto kern = modes == S ? hsForestStepMixedCluster<S>
                            : modes == H ? hsForestStepMixedCluster<H> : hsForestStepMixedCluster<S | H>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemBytes);
+    cudaError_t e = allowShared((const void*)kern);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nClusters * kC);
@@ -1478,7 +1479,7 @@ cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, con
     // maxLevels: the deepest forest's levels; modes: bits 1 << MixForest::shared
     if (pairWarps) {
         auto kern = b.anyStop ? hsForestPairStepMixed<true> : hsForestPairStepMixed<false>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemBytes);
+        cudaError_t e = allowShared((const void*)kern);
         if (e != cudaSuccess) return e;
         kern<<<nCtas, threadsPerCta, smemBytes, st>>>(b, ctaPtr, ctaForests, cap, pairWarps, nsteps);
         return cudaGetLastError();
@@ -1494,7 +1495,7 @@ cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, con
         kern = modes == S ? hsForestStepMixed<true, kUnsplit, S> : hsForestStepMixed<true, kUnsplit, S | G>;
     }
     if (modes == 1u << kRowsHalf) kern = hsForestStepMixed<true, kUnsplit, 1u << kRowsHalf>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemBytes);
+    cudaError_t e = allowShared((const void*)kern);
     if (e != cudaSuccess) return e;
     kern<<<nCtas, threadsPerCta, smemBytes, st>>>(b, ctaPtr, ctaForests, cap, deep, elimWarps, nsteps);
     return cudaGetLastError();

@@ -10,10 +10,12 @@
 #include <cstring>
 #include <deque>
 #include <functional>
+#include <map>
 
 #include "hs_cell.h"
 #include "hs_mixed.cuh"
 #include "hs_noalloc.h"
+#include "hs_shared.h"
 
 namespace {
 
@@ -31,6 +33,8 @@ cudaError_t push(std::function<void()> f) {
 }
 void* grab(size_t n) { return std::aligned_alloc(256, (n + 255) / 256 * 256); }
 
+int g_device = 0;
+std::map<std::pair<int, const void*>, int> g_limit;      // dynamic shared memory each kernel may take, per device
 const hsg::DevCell* g_cells = nullptr;      // of the last reinit
 uint32_t g_nCells = 0;
 
@@ -55,10 +59,32 @@ const double* fake_table(uint32_t k, uint32_t* shape) {
     return g_cells[k].vTab;
 }
 
+// Readies a kernel for its launches on `device`, and what they may take there.
+int fake_allow(uint64_t id, int device) {
+    g_device = device;
+    const cudaError_t e = hsg::allowShared((const void*)id);
+    g_device = 0;
+    return e == cudaSuccess ? 0 : -1;
+}
+int fake_limit(uint64_t id, int device) {
+    auto it = g_limit.find({device, (const void*)id});
+    return it == g_limit.end() ? 48 * 1024 : it->second;
+}
+
 const char* cudaGetErrorString(cudaError_t) { return "fake error"; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
-cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaGetDevice(int* d) { *d = g_device; return cudaSuccess; }
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void* f) {      // kernel `id`: id & 0xFFFF bytes of its own
+    *a = {};
+    a->sharedSizeBytes = (size_t)f & 0xFFFF;
+    return cudaSuccess;
+}
+cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute, int v) {
+    if (v + (int)((size_t)f & 0xFFFF) > kShared) return cudaErrorInvalidValue;
+    g_limit[{g_device, f}] = v;
+    return cudaSuccess;
+}
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
     *v = a == cudaDevAttrMultiProcessorCount ? kSms : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? kShared : kSharedSm;

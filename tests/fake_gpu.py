@@ -46,6 +46,7 @@ def load():
         L.fake_lazy.argtypes = [C.c_int, C.c_int]
         L.fake_table.argtypes = [C.c_uint32, C.POINTER(C.c_uint32)]
         L.fake_table.restype = C.POINTER(C.c_double)
+        L.fake_allow.argtypes = L.fake_limit.argtypes = [C.c_uint64, C.c_int]
         yield L
         L.fake_lazy(0, 0)
     finally:

@@ -63,3 +63,16 @@ def test_batch_shares_rate_tables_of_one_shape_only(gpu):
         at.append(C.addressof(p.contents))
     assert at[0] != at[1]
     b.close()
+
+
+def test_shared_memory_limit_is_the_devices_and_stays(gpu):
+    """A kernel's limit of dynamic shared memory belongs to the function: it
+    is set to all that the device has beside the kernel's own arrays, per
+    kernel and device, and no later launch lowers it."""
+    room = 232448
+    for kernel in (0x10000, 0x20400):           # without and with 1,024 bytes of its own
+        for dev in (0, 1):
+            assert gpu.fake_limit(kernel, dev) == 48 * 1024
+            for _ in range(2):
+                assert gpu.fake_allow(kernel, dev) == 0
+                assert gpu.fake_limit(kernel, dev) == room - (kernel & 0xFFFF)
