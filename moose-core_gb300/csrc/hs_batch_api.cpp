@@ -17,6 +17,7 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <queue>
@@ -393,6 +394,7 @@ uint32_t deliveryStep(double t, double dt) {
 
 int buildFp64(HsBatch* b, const HsCellDesc* cells) {
     const uint32_t nC = b->nCells;
+    std::vector<std::shared_ptr<void>> sent;        // host copies under way to the device
     // shared V/Ca tables by content and columns (pairTable's differences
     // depend on both), 2-D tables by source identity
     std::map<std::tuple<uint64_t, size_t, uint32_t>, const double*> tabDev;
@@ -425,7 +427,11 @@ int buildFp64(HsBatch* b, const HsCellDesc* cells) {
             const Table& T = pass ? b->plans[c].caTable : b->plans[c].vTable;
             auto key = std::make_tuple(fnv(T.data.data(), T.data.size() * 8), T.data.size(), T.nCol);
             auto it = tabDev.find(key);
-            if (it == tabDev.end()) it = tabDev.emplace(key, b->buf.up(pairTable(T), b->st)).first;
+            if (it == tabDev.end()) {
+                auto pairs = std::make_shared<std::vector<double>>(pairTable(T));
+                it = tabDev.emplace(key, b->buf.up(*pairs, b->st)).first;
+                sent.push_back(pairs);
+            }
             (pass ? catab : vtab)[c] = it->second;
         }
     }
@@ -460,13 +466,22 @@ int buildFp64(HsBatch* b, const HsCellDesc* cells) {
         sh[c].caTab = catab[c];
         sh[c].g2dBase = g2dBase;
         sh[c].g2dOff = g2dOffs[c];
-        layoutCell(b->plans[c], dry, b->dcs[c], b->spikeCap, b->st, &sh[c]);
+        layoutCell(b->plans[c], dry, b->dcs[c], b->spikeCap, b->st, sent, &sh[c]);
     }
     b->arena.size = dry.used + 256;
     e = cudaMallocAsync(&b->arena.base, b->arena.size, b->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->arena.base, 0, b->arena.size, b->st);
-    for (uint32_t c = 0; c < nC && e == cudaSuccess; ++c)
-        e = layoutCell(b->plans[c], b->arena, b->dcs[c], b->spikeCap, b->st, &sh[c]);
+    size_t kept = 0;
+    for (uint32_t c = 0; c < nC && e == cudaSuccess; ++c) {
+        const size_t from = b->arena.used;
+        e = layoutCell(b->plans[c], b->arena, b->dcs[c], b->spikeCap, b->st, sent, &sh[c]);
+        kept += b->arena.used - from;
+        if (e == cudaSuccess && (kept > (64u << 20) || c + 1 == nC)) {
+            e = cudaStreamSynchronize(b->st);
+            sent.clear();
+            kept = 0;
+        }
+    }
     if (e != cudaSuccess) return cerr(e, "batch upload");
     b->dDcs = b->buf.alloc<DevCell>(nC);
     if (b->buf.err != cudaSuccess) return cerr(b->buf.err, "batch cells");

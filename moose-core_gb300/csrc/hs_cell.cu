@@ -16,14 +16,22 @@ namespace {
 struct Uploader {
     Arena& a;
     cudaStream_t st;
+    std::vector<std::shared_ptr<void>>& sent;
     cudaError_t err = cudaSuccess;
     std::vector<char> part = {};       // bytes [first, first + part.size()) of the arena, to be sent
     size_t first = 0;
     static constexpr size_t kDirect = 64 << 10;
+    // `v` outlives the copies, as the plan does
     template <class T>
     T* put(const std::vector<T>& v) {
         T* p = a.take<T>(v.empty() ? 1 : v.size());
         if (p && !v.empty() && err == cudaSuccess) add(reinterpret_cast<char*>(p) - a.base, v.data(), v.size() * sizeof(T));
+        return p;
+    }
+    template <class T>
+    T* put(std::vector<T>&& v) {
+        T* p = put(static_cast<const std::vector<T>&>(v));
+        if (p && v.size() * sizeof(T) >= kDirect) keep(std::move(v));
         return p;
     }
     template <class T>
@@ -46,11 +54,16 @@ struct Uploader {
         part.insert(part.end(), static_cast<const char*>(src), static_cast<const char*>(src) + bytes);
     }
     cudaError_t send() {
-        if (!part.empty() && err == cudaSuccess)
+        if (!part.empty() && err == cudaSuccess) {
             err = cudaMemcpyAsync(a.base + first, part.data(), part.size(), cudaMemcpyHostToDevice, st);
+            keep(std::move(part));
+        }
         part.clear();
         return err;
     }
+    // (a moved vector's elements stay where they are)
+    template <class T>
+    void keep(std::vector<T>&& v) { sent.push_back(std::make_shared<std::vector<T>>(std::move(v))); }
 };
 
 }  // namespace
@@ -185,8 +198,9 @@ bool compactPrograms(const CellPlan& P, Compact& C) {
 }  // namespace
 
 cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCap,
-                       cudaStream_t st, const CellShared* sh, Arena* spikes) {
-    Uploader u{a, st};
+                       cudaStream_t st, std::vector<std::shared_ptr<void>>& sent, const CellShared* sh,
+                       Arena* spikes) {
+    Uploader u{a, st, sent};
     const uint32_t N = P.N, H = P.H;
     std::memset(&c, 0, sizeof(c));
     c.N = N; c.H = H; c.C = P.C; c.G = P.G; c.P = P.P; c.K2 = P.K2; c.S = P.S; c.SG = P.SG;
@@ -204,7 +218,7 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         std::vector<double> M(3 * (size_t)N + H, 0.0);
         for (uint32_t h = 0; h < H; ++h) M[2 * N + h] = P.HJ0[h];
         for (uint32_t i = 0; i < N; ++i) M[2 * N + H + i] = P.off[i];
-        c.M = u.put(M);
+        c.M = u.put(std::move(M));
     }
     c.HJ0 = u.put(P.HJ0);
     c.HS2 = u.put(P.HS2);
@@ -243,15 +257,15 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         c.runRows = longest >= kWarpRun ? longest : 0;
         c.smWords = compact ? 2 * N + H + 2 * c.runRows : 0;
         c.fSplit = C.split;
-        c.fW = u.put(C.fW);
-        c.bW = u.put(C.bW);
-        c.bX = u.put(C.bX);
-        c.fLane = u.put(C.fLane);
-        c.bLane = u.put(C.bLane);
-        c.fSeg = u.put(C.fSeg);
-        c.bSeg = u.put(C.bSeg);
+        c.fW = u.put(std::move(C.fW));
+        c.bW = u.put(std::move(C.bW));
+        c.bX = u.put(std::move(C.bX));
+        c.fLane = u.put(std::move(C.fLane));
+        c.bLane = u.put(std::move(C.bLane));
         c.nfSeg = (uint32_t)C.fSeg.size();
         c.nbSeg = (uint32_t)C.bSeg.size();
+        c.fSeg = u.put(std::move(C.fSeg));
+        c.bSeg = u.put(std::move(C.bSeg));
     }
     c.Gbar = u.put(P.Gbar);
     c.Ek = u.put(P.Ek);
@@ -268,7 +282,7 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         for (uint32_t q = 0; q < P.C; ++q)
             ca[q] = make_uint4(powCode(P.Xpow[q]) | powCode(P.Ypow[q]) << 4 | powCode(P.Zpow[q]) << 8,
                                (uint32_t)P.stateOff[q], (uint32_t)P.colX[q], (uint32_t)P.colY[q]);
-        c.chanA = u.put(ca);
+        c.chanA = u.put(std::move(ca));
     }
     c.colZ = u.put(P.colZ);
     c.zSrc = u.put(P.zSrc);
@@ -276,7 +290,6 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         std::vector<uint32_t> cc(P.C);
         for (uint32_t ic = 0; ic < N; ++ic)
             for (uint32_t q = P.chanPtr[ic]; q < P.chanPtr[ic + 1]; ++q) cc[q] = ic;
-        c.chanCompt = u.put(cc);
         std::vector<uint32_t> poolCompt(P.P);
         for (uint32_t ic = 0; ic < N; ++ic)
             for (uint32_t p = P.poolPtr[ic]; p < P.poolPtr[ic + 1]; ++p) poolCompt[p] = ic;
@@ -288,6 +301,7 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         for (uint32_t k = 0; k < P.K2; ++k)
             for (int32_t p : {P.c2dConc1[k], P.c2dConc2[k]}) local = local && (p < 0 || poolCompt[p] == P.c2dCompt[k]);
         c.local = local;
+        c.chanCompt = u.put(std::move(cc));
     }
     c.c = u.put(P.c0);
     c.CaBasal = u.put(P.CaBasal);
@@ -324,11 +338,11 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
             c.g2dAB = sh->g2dBase;
             c.g2dOff = u.put(sh->g2dOff);
         } else {
-            c.g2dAB = u.put(AB);
-            c.g2dOff = u.put(off);
+            c.g2dAB = u.put(std::move(AB));
+            c.g2dOff = u.put(std::move(off));
         }
-        c.g2dGeom = u.put(geom);
-        c.g2dN = u.put(nn);
+        c.g2dGeom = u.put(std::move(geom));
+        c.g2dN = u.put(std::move(nn));
     }
     c.c2dCompt = u.put(P.c2dCompt);
     c.c2dGate = u.put(P.c2dGate);
@@ -338,7 +352,7 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         for (uint32_t k = 0; k < P.K2; ++k)
             ka[k] = powCode(P.c2dXpow[k]) | dep(P.c2dDep0[k]) << 4 | dep(P.c2dDep1[k]) << 8 |
                     ((uint32_t)P.c2dInstant[k] & 0xFu) << 12;
-        c.c2dA = u.put(ka);
+        c.c2dA = u.put(std::move(ka));
     }
     c.c2dConc1 = u.put(P.c2dConc1);
     c.c2dConc2 = u.put(P.c2dConc2);
@@ -392,7 +406,7 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
         std::vector<double> st((size_t)kDifState * P.nDif, 0.0);
         for (uint32_t k = 0; k < P.nDif; ++k)
             if (P.difKind[k] == HS_DIF_BUFFER) st[9 * (size_t)P.nDif + k] = P.difPar[(size_t)k * HS_DIF_NPAR + 11];
-        c.difState = u.put(st);
+        c.difState = u.put(std::move(st));
     }
     c.nRec = 0;
     c.recStride = 1;

@@ -31,7 +31,13 @@ cudaError_t push(std::function<void()> f) {
     g_queue.push_back(std::move(f));
     return cudaSuccess;
 }
+std::map<void*, std::pair<int, size_t>> g_made;      // device allocations: number, bytes
+int g_count = 0;
 void* grab(size_t n) { return std::aligned_alloc(256, (n + 255) / 256 * 256); }
+void drop(void* p) {
+    g_made.erase(p);
+    std::free(p);
+}
 
 int g_device = 0;
 std::map<std::pair<int, const void*>, int> g_limit;      // dynamic shared memory each kernel may take, per device
@@ -49,6 +55,23 @@ void fake_lazy(int reads, int writes) {
     g_lazyRead = reads;
     g_lazyWrite = writes;
 }
+
+// Digest of the device allocations made since the last call, in order, but for
+// those of `skip` bytes (the cells' descriptions, which hold addresses).
+uint64_t fake_digest(uint64_t skip) {
+    drain();
+    static int from = 0;
+    std::map<int, std::pair<const unsigned char*, size_t>> order;
+    for (const auto& m : g_made)
+        if (m.second.first >= from && m.second.second != skip)
+            order[m.second.first] = {static_cast<const unsigned char*>(m.first), m.second.second};
+    from = g_count;
+    uint64_t h = 1469598103934665603ull;
+    for (const auto& o : order)
+        for (size_t i = 0; i < o.second.second; ++i) h = (h ^ o.second.first[i]) * 1099511628211ull;
+    return h;
+}
+uint64_t fake_cell_bytes() { return sizeof(hsg::DevCell); }
 
 // Cell k's rate table on Vm as the last reinit had it: {columns, rows} and its data.
 const double* fake_table(uint32_t k, uint32_t* shape) {
@@ -92,10 +115,15 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
 }
 cudaError_t cudaDeviceGetDefaultMemPool(cudaMemPool_t* p, int) { *p = nullptr; return cudaSuccess; }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
-cudaError_t cudaMalloc(void** p, size_t n) { *p = grab(n); return cudaSuccess; }
-cudaError_t cudaFree(void* p) { drain(); std::free(p); return cudaSuccess; }
+cudaError_t cudaMalloc(void** p, size_t n) {
+    *p = grab(n);
+    std::memset(*p, 0xA5, n);
+    g_made[*p] = {g_count++, n};
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) { drain(); drop(p); return cudaSuccess; }
 cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
-cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return push([=] { std::free(p); }); }
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return push([=] { drop(p); }); }
 cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) { return push([=] { std::memset(p, v, n); }); }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind k, cudaStream_t) {
     push([=] { std::memcpy(d, s, n); });

@@ -47,6 +47,8 @@ def load():
         L.fake_table.argtypes = [C.c_uint32, C.POINTER(C.c_uint32)]
         L.fake_table.restype = C.POINTER(C.c_double)
         L.fake_allow.argtypes = L.fake_limit.argtypes = [C.c_uint64, C.c_int]
+        L.fake_digest.argtypes, L.fake_digest.restype = [C.c_uint64], C.c_uint64
+        L.fake_cell_bytes.restype = C.c_uint64
         yield L
         L.fake_lazy(0, 0)
     finally:

@@ -76,3 +76,30 @@ def test_shared_memory_limit_is_the_devices_and_stays(gpu):
             for _ in range(2):
                 assert gpu.fake_allow(kernel, dev) == 0
                 assert gpu.fake_limit(kernel, dev) == room - (kernel & 0xFFFF)
+
+
+@pytest.mark.parametrize("kind", ["dropin", "batch"])
+def test_uploads_read_their_source_late(gpu, kind):
+    """What creating a solver or an FP64 batch leaves on the device is the same
+    when the copies to it read the host's memory only at the next wait."""
+    # (tables, programs and parameters on both sides of the size sent by itself)
+    cells = [models.config1_cell(n_cable=200), _cell(60), _cell(1500, n_syn=30)]
+
+    def digest(lazy):
+        gpu.fake_digest(0)
+        gpu.fake_lazy(0, lazy)
+        if kind == "dropin":
+            made = []
+            for m in cells:
+                made.append(HSolve(m, dt=DT))
+                made[-1].target = m.seed
+        else:
+            made = [Batch(cells, DT, HS_PREC_FP64)]
+        h = gpu.fake_digest(len(cells) * gpu.fake_cell_bytes())
+        gpu.fake_lazy(0, 0)
+        for x in made:
+            x.close()
+        return h
+    now = digest(0)
+    assert digest(0) == now
+    assert digest(1) == now
