@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -45,6 +46,7 @@ int setLastError(int code, const std::string& msg) { return setErr(code, msg); }
 struct HsGroupDone {
     cudaEvent_t ev = nullptr;
     cudaStream_t st = nullptr;          // the stream the launch ran on
+    std::atomic<bool> over{false};      // the host has waited for it
     ~HsGroupDone() {
         if (ev) cudaEventDestroy(ev);   // released once it has completed
     }
@@ -108,15 +110,25 @@ namespace {
 // must come before the solver's next group launch.
 cudaStream_t stOf(HsSolver* s) {
     if (s->group) {
-        // (a launch that is over needs no wait: of the reads after a group's
-        // step only the first waits, and 256 take 1 ms less)
-        const cudaError_t e = cudaEventQuery(s->group->ev);
-        if (e == cudaErrorNotReady) cudaGetLastError();
-        if (e != cudaSuccess) cudaStreamWaitEvent(s->st, s->group->ev, 0);
+        // (a launch that is known to be over needs no wait: of the reads after
+        // a group's step only the first waits, and 256 take 1 ms less.  Known
+        // from a wait: a query of the event is not allowed to a thread that
+        // captures a graph.)
+        if (!s->group->over) cudaStreamWaitEvent(s->st, s->group->ev, 0);
         s->group.reset();
     }
     s->queued = true;
     return s->st;
+}
+
+// `bytes` from the device to pageable memory, there when it returns (such a
+// copy may be under way when its call returns).
+cudaError_t readBack(HsSolver* s, void* dst, const void* src, size_t bytes) {
+    const std::shared_ptr<HsGroupDone> group = s->group;
+    cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stOf(s));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
+    if (e == cudaSuccess && group) group->over = true;
+    return e;
 }
 
 // ---- field access between process calls ------------------------------------
@@ -893,9 +905,7 @@ int hs_read_vm(HsSolver* s, double* out, uint32_t n) {
     if (n != s->P.hinesOf.size()) return setErr(HS_EINVAL, "n must equal the model's compartment count");
     if (int rc = flushWrites(s)) return rc;
     std::vector<double> v(s->P.N);
-    cudaError_t e = cudaMemcpyAsync(v.data(), s->dc.V, v.size() * 8, cudaMemcpyDeviceToHost, stOf(s));
-    // (a copy to pageable memory may be under way when its call returns)
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
+    const cudaError_t e = readBack(s, v.data(), s->dc.V, v.size() * 8);
     if (e != cudaSuccess) return cudaErr(e, "read vm");
     for (uint32_t m = 0; m < n; ++m) out[m] = s->P.hinesOf[m] < 0 ? NAN : v[s->P.hinesOf[m]];
     return HS_OK;
@@ -906,8 +916,7 @@ int hs_read_ca(HsSolver* s, double* out, uint32_t n) {
     if (n != s->P.poolSolverOf.size()) return setErr(HS_EINVAL, "n must equal the model's pool count");
     if (int rc = flushWrites(s)) return rc;
     std::vector<double> v(s->P.P + 1);
-    cudaError_t e = cudaMemcpyAsync(v.data(), s->dc.ca, s->P.P * 8, cudaMemcpyDeviceToHost, stOf(s));
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
+    const cudaError_t e = readBack(s, v.data(), s->dc.ca, s->P.P * 8);
     if (e != cudaSuccess) return cudaErr(e, "read ca");
     for (uint32_t m = 0; m < n; ++m) out[m] = s->P.poolSolverOf[m] < 0 ? NAN : v[s->P.poolSolverOf[m]];
     return HS_OK;

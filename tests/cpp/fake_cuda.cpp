@@ -39,6 +39,7 @@ void drop(void* p) {
     std::free(p);
 }
 
+int g_queries = 0, g_waits = 0;     // calls of cudaEventQuery and cudaStreamWaitEvent
 int g_device = 0;
 std::map<std::pair<int, const void*>, int> g_limit;      // dynamic shared memory each kernel may take, per device
 const hsg::DevCell* g_cells = nullptr;      // of the last reinit
@@ -81,6 +82,9 @@ const double* fake_table(uint32_t k, uint32_t* shape) {
     shape[1] = g_cells[k].vRows;
     return g_cells[k].vTab;
 }
+
+int fake_queries() { return g_queries; }
+int fake_waits() { return g_waits; }
 
 // Readies a kernel for its launches on `device`, and what they may take there.
 int fake_allow(uint64_t id, int device) {
@@ -139,7 +143,10 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = (cudaStr
 cudaError_t cudaStreamDestroy(cudaStream_t s) { drain(); std::free(s); return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { drain(); return cudaSuccess; }
 cudaError_t cudaStreamQuery(cudaStream_t) { return g_queue.empty() ? cudaSuccess : cudaErrorNotReady; }
-cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) {
+    ++g_waits;
+    return cudaSuccess;
+}
 cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
 cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) { *g = nullptr; return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* x, cudaGraph_t, unsigned long long) { *x = nullptr; return cudaSuccess; }
@@ -150,7 +157,10 @@ cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)grab(1); return 
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { std::free(e); return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaEventQuery(cudaEvent_t) { return g_queue.empty() ? cudaSuccess : cudaErrorNotReady; }
+cudaError_t cudaEventQuery(cudaEvent_t) {
+    ++g_queries;
+    return g_queue.empty() ? cudaSuccess : cudaErrorNotReady;
+}
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 0; return cudaSuccess; }
 
 }  // extern "C"

@@ -9,7 +9,7 @@ import fake_gpu
 from moose_gb300 import models
 from moose_gb300.abi import HS_PREC_FP64
 from moose_gb300.batch import Batch
-from moose_gb300.hsolve import HSolve
+from moose_gb300.hsolve import HSolve, Tick
 
 DT = 25e-6
 
@@ -103,3 +103,24 @@ def test_uploads_read_their_source_late(gpu, kind):
     now = digest(0)
     assert digest(0) == now
     assert digest(1) == now
+
+
+def test_reads_after_a_group_wait_once_and_query_nothing(gpu):
+    """Of a group's solvers the first is on the launch's stream, the second's
+    read waits for the launch, and the others' know that it is over; none asks
+    by a query, which a thread that captures a graph may not make."""
+    cells = [_cell(20 + i) for i in range(6)]
+    solvers = []
+    for m in cells:
+        solvers.append(HSolve(m, dt=DT))
+        solvers[-1].target = m.seed
+        solvers[-1].reinit(DT)
+    tick = Tick(solvers)
+    for _ in range(2):
+        tick.process(3)
+        q, w = gpu.fake_queries(), gpu.fake_waits()
+        for h, m in zip(solvers, cells):
+            assert np.array_equal(h.vm(), m.initVm)
+        assert (gpu.fake_queries() - q, gpu.fake_waits() - w) == (0, 1)
+    for h in solvers:
+        h.close()
