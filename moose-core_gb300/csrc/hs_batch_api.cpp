@@ -246,13 +246,6 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
         return launchBatchStepFp64(b->dDcs, b->dWholePtr, b->dWholeCells, b->dTeamPtr, b->dTeamCells, b->nBlocks,
                                    b->nTeams, b->threadsPerCta, b->batchWords, k, b->st);
     uint32_t ew = b->elimWarps && b->threadsPerCta > 32 * b->elimWarps ? b->elimWarps : 0;
-    // Unless asked for a number, more eliminators for forests of wider levels:
-    // 4 up to 1,279 nodes, 8 from 2,048 (us per step with 4 / 6 / 8: 203 nodes
-    // 19.1 / 19.4 / 19.9, ~1,700 45.3 / 43.7 / 44.3, ~6,500 93.7 / 89.6 / 85.8).
-    if (ew && !b->elimSet && b->mixModes == 1u << kRowsGlobal && b->threadsPerCta >= 640)
-        ew = b->threadsPerCta * 10 / 1024;      // (4,096 cells merged: 6 487, 8 419, 10 396)
-    if (ew && !b->elimSet && b->mixModes == 1u << kRowsShared)
-        ew = std::max<uint32_t>(4, std::min(b->mixMaxNodes / 256, b->threadsPerCta / 128));
     b->mb.waitRounds = b->waitRounds;
     if (b->clusterCtas > 1) {
         // the cluster's forests are large: twice the eliminator warps, as
@@ -262,6 +255,13 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
                                             b->threadsPerCta, b->mixSmem, b->mixCap, b->mixStageCap, ce,
                                             b->mixModes, k, b->st);
     }
+    // Unless asked for a number, more eliminators for forests of wider levels:
+    // 4 up to 1,279 nodes, 8 from 2,048 (us per step with 4 / 6 / 8: 203 nodes
+    // 19.1 / 19.4 / 19.9, ~1,700 45.3 / 43.7 / 44.3, ~6,500 93.7 / 89.6 / 85.8).
+    if (ew && !b->elimSet && b->mixModes == 1u << kRowsGlobal && b->threadsPerCta >= 640)
+        ew = b->threadsPerCta * 10 / 1024;      // (4,096 cells merged: 6 487, 8 419, 10 396)
+    if (ew && !b->elimSet && b->mixModes == 1u << kRowsShared)
+        ew = std::max<uint32_t>(4, std::min(b->mixMaxNodes / 256, b->threadsPerCta / 128));
     // Eliminators of each forest of a pair: 3/16 of the CTA (of 32 warps 6 each;
     // a population of 1,024 cells, 8,850 nodes a pair: 4 124, 5 117, 6 112, 8
     // 125 us per step; 2,048 cells 5 227, 6 222), of pairs of more than 10,240

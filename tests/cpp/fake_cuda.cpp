@@ -40,6 +40,7 @@ void drop(void* p) {
 }
 
 int g_queries = 0, g_waits = 0;     // calls of cudaEventQuery and cudaStreamWaitEvent
+uint32_t g_elimWarps = 0;           // of the last mixed step
 int g_device = 0;
 std::map<std::pair<int, const void*>, int> g_limit;      // dynamic shared memory each kernel may take, per device
 const hsg::DevCell* g_cells = nullptr;      // of the last reinit
@@ -83,6 +84,7 @@ const double* fake_table(uint32_t k, uint32_t* shape) {
     return g_cells[k].vTab;
 }
 
+uint32_t fake_elim_warps() { return g_elimWarps; }
 int fake_queries() { return g_queries; }
 int fake_waits() { return g_waits; }
 
@@ -213,8 +215,9 @@ cudaError_t launchForestStepMixed(const MixBatch&, const uint32_t*, const uint32
     return cudaSuccess;
 }
 cudaError_t launchForestStepMixedCluster(const MixBatch&, const uint32_t*, const uint32_t*, uint32_t, uint32_t,
-                                         uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t,
-                                         cudaStream_t) {
+                                         uint32_t, uint32_t, uint32_t, uint32_t, uint32_t elimWarps, uint32_t,
+                                         uint32_t, cudaStream_t) {
+    g_elimWarps = elimWarps;
     return cudaSuccess;
 }
 cudaError_t launchBatchReinitMixed(const MixBatch&, uint32_t, const double*, const float*, const uint32_t*,

@@ -7,7 +7,7 @@ import pytest
 
 import fake_gpu
 from moose_gb300 import models
-from moose_gb300.abi import HS_PREC_FP64
+from moose_gb300.abi import HS_PREC_FP64, HS_PREC_MIXED
 from moose_gb300.batch import Batch
 from moose_gb300.hsolve import HSolve, Tick
 
@@ -124,3 +124,15 @@ def test_reads_after_a_group_wait_once_and_query_nothing(gpu):
         assert (gpu.fake_queries() - q, gpu.fake_waits() - w) == (0, 1)
     for h in solvers:
         h.close()
+
+
+@pytest.mark.parametrize("n", [300, 3000, 9001])
+@pytest.mark.parametrize("asked, warps", [(0, 8), (3, 6), (6, 12)])
+def test_eliminators_of_a_cluster(gpu, n, asked, warps):
+    """Twice the batch's eliminator warps, whatever the cell's size: the rule of
+    one CTA's forests, which have a CTA's threads and no more, is not theirs."""
+    b = Batch([_cell(n)], DT, HS_PREC_MIXED, cluster_ctas=4, max_ctas=4, elim_warps=asked)
+    b.reinit(DT)
+    b.process(1)
+    assert gpu.fake_elim_warps() == warps
+    b.close()
