@@ -209,6 +209,9 @@ struct ChanIn {
 // while the channel before it is computed and before its states are stored
 // (a load does not pass a store it may alias), and of FP64 instructions, 76
 // cycles each on this GPU, only the membrane's own five are left.
+// kAhead: that reading ahead, for ~12 registers.  Without it in the kernels
+// that hold several ways to step a forest, where it would spill.
+template <bool kAhead>
 __device__ __forceinline__ void assembleNode(const MixBatch& b, uint32_t n, uint32_t info, bool update,
                                              double vmPrev, double& diag, double& rhs) {
     const uint64_t ld = b.ld;
@@ -263,21 +266,25 @@ __device__ __forceinline__ void assembleNode(const MixBatch& b, uint32_t n, uint
         const float gb = __ldg(b.gbar + (uint64_t)j * ld + n);
         float2* const sj = st + (uint64_t)(3 * j) * ld;
         ChanIn in;
-        if (t.xp) {
+        auto readX = [&]() {
             in.x = sj[0];
             in.rx = rowOf(vr, t.colX);
-        }
-        if (t.yp) {
+        };
+        auto readY = [&]() {
             in.y = sj[ld];
             in.ry = rowOf(vr, t.colY);
-        }
+        };
+        if (kAhead && t.xp) readX();
+        if (kAhead && t.yp) readY();
         float frac = 1.f;
         if (t.xp) {
+            if (!kAhead) readX();
             const float2 x = gateStep(lerp(in.rx, vr.frac), in.x, dt, hdt, t.instant & 1);
             sj[0] = x;
             frac *= powi(x.x, t.xp, t.xp < 0 ? __ldg(&b.chanPow[tj].x) : 0.f);
         }
         if (t.yp) {
+            if (!kAhead) readY();
             const float2 y = gateStep(lerp(in.ry, vr.frac), in.y, dt, hdt, t.instant & 2);
             sj[ld] = y;
             frac *= powi(y.x, t.yp, t.yp < 0 ? __ldg(&b.chanPow[tj].y) : 0.f);
@@ -545,7 +552,7 @@ __device__ __forceinline__ void finishForest(const MixBatch& b, uint32_t f, cons
 // step's assembly, and after the last step.  A cell whose stop step is
 // reached stays as it is: its nodes get a neutral row (pivot 1, rhs 0) so
 // that the elimination of the forest goes on around them.
-template <class Rows>
+template <bool kAhead, class Rows>
 __device__ __forceinline__ void stepForest(const MixBatch& b, const MixForest& F, uint32_t f,
                                            const Rows& E, const uint32_t* lp, uint32_t nsteps) {
     const uint32_t tid = threadIdx.x, nth = blockDim.x;
@@ -574,7 +581,7 @@ __device__ __forceinline__ void stepForest(const MixBatch& b, const MixForest& F
             if (info & kNodeCenter) {
                 if (live) d = __ldg(b.HS2 + n);
             } else if (live) {
-                assembleNode(b, n, info, pending, pending ? E.R(i) : 0.0, d, r);
+                assembleNode<kAhead>(b, n, info, pending, pending ? E.R(i) : 0.0, d, r);
             } else if (pending) {
                 updateNode(b, n, info, E.R(i));
             }
@@ -667,7 +674,7 @@ __device__ __forceinline__ bool waitLevel(const MixBatch& b, const uint32_t* don
 // the assembly of the shallow ones; meanwhile the assemblers emit the
 // previous step's outputs and advance the next step's SynChans.  Then the
 // whole CTA substitutes back.  Forests of fewer than kWsLevels levels.
-template <bool kStops, class Rows>
+template <bool kStops, bool kAhead, class Rows>
 __device__ __forceinline__ void stepForestWS(const MixBatch& b, uint32_t f, const Rows& E, uint32_t elimWarps,
                                              uint32_t nsteps) {
     volatile const MixForest& F = sCtl().F;
@@ -730,7 +737,7 @@ __device__ __forceinline__ void stepForestWS(const MixBatch& b, uint32_t f, cons
                 if (info & kNodeCenter) {
                     if (live) d = __ldg(b.HS2 + n);
                 } else if (live) {
-                    assembleNode(b, n, info, pending, pending ? E.R(i) : 0.0, d, r);
+                    assembleNode<kAhead>(b, n, info, pending, pending ? E.R(i) : 0.0, d, r);
                 } else if (pending) {
                     updateNode(b, n, info, E.R(i));
                 }
@@ -1017,7 +1024,7 @@ __device__ __forceinline__ void stepPair(const MixBatch& b, uint32_t groups, uin
                 if (info & kNodeCenter) {
                     if (live) d = __ldg(b.HS2 + n);
                 } else if (live) {
-                    assembleNode(b, n, info, pending, pending ? E.R(i) : 0.0, d, r);
+                    assembleNode<true>(b, n, info, pending, pending ? E.R(i) : 0.0, d, r);
                 } else if (pending) {
                     updateNode(b, n, info, E.R(i));
                 }
@@ -1120,6 +1127,7 @@ template <bool kStops, uint32_t kSteps, uint32_t kModes>
 __global__ void __launch_bounds__(1024, 1) hsForestStepMixed(MixBatch b, const uint32_t* __restrict__ ctaPtr,
                                                              const uint32_t* __restrict__ ctaForests, uint32_t cap,
                                                              uint32_t deep, uint32_t elimWarps, uint32_t nsteps) {
+    constexpr bool kAhead = kSteps != (kSplit | kUnsplit) && (kModes & (kModes - 1)) == 0;
     copyTypes(b);
     for (uint32_t k = ctaPtr[blockIdx.x]; k < ctaPtr[blockIdx.x + 1]; ++k) {
         const MixForest F = b.forests[ctaForests[k]];
@@ -1160,13 +1168,13 @@ __global__ void __launch_bounds__(1024, 1) hsForestStepMixed(MixBatch b, const u
         const bool plain = kSteps == kUnsplit ||
                            (kSteps != kSplit && !(ew && F.nLevels < kWsLevels && blockDim.x > 32 * ew));
         if ((kModes & 1u << kRowsShared) && F.shared == kRowsShared) {
-            if (plain) stepForest(b, F, f, S, lp, nsteps);
-            else stepForestWS<kStops>(b, f, S, ew, nsteps);
+            if (plain) stepForest<kAhead>(b, F, f, S, lp, nsteps);
+            else stepForestWS<kStops, kAhead>(b, f, S, ew, nsteps);
         } else if (kModes & 1u << kRowsHalf) {
-            stepForest(b, F, f, HalfRows{b, F.node0, F.slot + deep, cap}, lp, nsteps);
+            stepForest<kAhead>(b, F, f, HalfRows{b, F.node0, F.slot + deep, cap}, lp, nsteps);
         } else if (kModes & 1u << kRowsGlobal) {
-            if (plain) stepForest(b, F, f, G, lp, nsteps);
-            else stepForestWS<kStops>(b, f, G, ew, nsteps);
+            if (plain) stepForest<kAhead>(b, F, f, G, lp, nsteps);
+            else stepForestWS<kStops, kAhead>(b, f, G, ew, nsteps);
         }
     }
 }
@@ -1303,7 +1311,7 @@ __device__ __forceinline__ void clusterMeet(const MixBatch& b, uint32_t* bar, ui
 
 // `nsteps` steps of forest F by the cluster.  dR0 and rR0: D and R in rank
 // 0's shared memory; E: the rows there, as rank 0 eliminates them.
-template <bool kStaged, class Rows>
+template <bool kStaged, bool kAhead, class Rows>
 __device__ __forceinline__ void stepForestCluster(const MixBatch& b, const MixForest& F, uint32_t f,
                                   const Rows& E, double* dR0, double* rR0, uint32_t* doneR0, uint32_t* barR0,
                                   uint32_t& gen, uint32_t rank, uint32_t kC, uint32_t elimWarps, uint32_t nsteps,
@@ -1361,7 +1369,7 @@ __device__ __forceinline__ void stepForestCluster(const MixBatch& b, const MixFo
                 if (info & kNodeCenter) {
                     if (live) d = __ldg(b.HS2 + n);
                 } else if (live) {
-                    assembleNode(b, n, info, pending, pending ? rR0[i] : 0.0, d, r);
+                    assembleNode<kAhead>(b, n, info, pending, pending ? rR0[i] : 0.0, d, r);
                 } else if (pending) {
                     updateNode(b, n, info, rR0[i]);
                 }
@@ -1416,6 +1424,7 @@ __global__ void __launch_bounds__(1024, 1) hsForestStepMixedCluster(MixBatch b, 
                                                                     const uint32_t* __restrict__ ctaForests,
                                                                     uint32_t kC, uint32_t cap, uint32_t stageCap,
                                                                     uint32_t elimWarps, uint32_t nsteps) {
+    constexpr bool kAhead = (kModes & (kModes - 1)) == 0;
     copyTypes(b);
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -1439,9 +1448,9 @@ __global__ void __launch_bounds__(1024, 1) hsForestStepMixedCluster(MixBatch b, 
         __syncthreads();
         double* const d = cluster.map_shared_rank(sArea(), 0);
         if ((kModes & 1u << kRowsShared) && stage)
-            stepForestCluster<true>(b, F, f, S, d, d + stageCap, doneR0, barR0, gen, rank, kC, elimWarps, nsteps, gaveUp);
+            stepForestCluster<true, kAhead>(b, F, f, S, d, d + stageCap, doneR0, barR0, gen, rank, kC, elimWarps, nsteps, gaveUp);
         else if (kModes & 1u << kRowsHalf)
-            stepForestCluster<false>(b, F, f, H, d, d + cap, doneR0, barR0, gen, rank, kC, elimWarps, nsteps, gaveUp);
+            stepForestCluster<false, kAhead>(b, F, f, H, d, d + cap, doneR0, barR0, gen, rank, kC, elimWarps, nsteps, gaveUp);
     }
     cluster.sync();                                   // rank 0's shared memory outlives every remote access
 }
@@ -1486,7 +1495,8 @@ cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, con
     }
     const uint32_t warps = b.anyStop ? std::min(2 * elimWarps, 16u) : elimWarps;
     constexpr uint32_t S = 1u << kRowsShared, G = 1u << kRowsGlobal;
-    auto kern = hsForestStepMixed<true, kSplit | kUnsplit, S | G>;
+    auto kern = b.anyStop ? hsForestStepMixed<true, kSplit | kUnsplit, S | G>
+                          : hsForestStepMixed<false, kSplit | kUnsplit, S | G>;
     if (elimWarps && maxLevels < kWsLevels && threadsPerCta > 32 * warps) {
         if (modes == S) kern = b.anyStop ? hsForestStepMixed<true, kSplit, S> : hsForestStepMixed<false, kSplit, S>;
         else if (modes == G) kern = b.anyStop ? hsForestStepMixed<true, kSplit, G> : hsForestStepMixed<false, kSplit, G>;
