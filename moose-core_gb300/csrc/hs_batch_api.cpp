@@ -766,33 +766,41 @@ int buildMixed(HsBatch* b) {
         uint32_t nodes = 0, rows = kRowsShared, mate = 0, slot = 0;
     };
     // The cells of a CTA (in order of size) as pairs of forests, of at most
-    // `lim` nodes a pair: as few pairs as hold them, the cells spread evenly,
-    // the largest forest with the smallest.  Empty if a cell does not fit.
+    // `lim` nodes a pair: as few pairs as hold them, the cells spread evenly
+    // over the pairs and then over a pair's two forests, so that one large cell
+    // takes a pair of its own (a lone forest) and not the room of a mate in
+    // every other.  Empty if a cell does not fit.
     auto pairForests = [&](const std::vector<uint32_t>& cells, uint32_t lim) {
+        std::vector<ForestPlan> out;
         uint64_t total = 0;
         for (uint32_t c : cells) total += trees[c].T;
+        if (cells.empty() || trees[cells[0]].T > lim) return out;
         auto fewer = [](const ForestPlan& x, const ForestPlan& y) { return x.nodes < y.nodes; };
-        for (size_t n = (total + lim - 1) / lim; 2 * n <= cells.size() + 1; ++n) {
-            std::vector<ForestPlan> bins(2 * n), out;
-            for (uint32_t c : cells) {
+        auto spread = [&](const std::vector<uint32_t>& cs, size_t n) {
+            std::vector<ForestPlan> bins(n);
+            for (uint32_t c : cs) {
                 ForestPlan& f = *std::min_element(bins.begin(), bins.end(), fewer);
                 f.cells.push_back(c);
                 f.nodes += trees[c].T;
             }
-            std::stable_sort(bins.rbegin(), bins.rend(), fewer);
-            bool fits = true;
-            for (size_t k = 0; k < n; ++k) {
-                ForestPlan &x = bins[k], &y = bins[2 * n - 1 - k];
+            return bins;
+        };
+        for (size_t n = (total + lim - 1) / lim; out.empty(); ++n)      // (ends: a cell each fits)
+            for (const ForestPlan& pair : spread(cells, n)) {
+                if (pair.cells.empty()) continue;
+                std::vector<ForestPlan> two = spread(pair.cells, 2);
+                ForestPlan &x = two[two[0].nodes < two[1].nodes], &y = two[two[0].nodes >= two[1].nodes];
                 x.rows = y.rows = kRowsHalf;
                 x.mate = y.nodes > 0;
                 y.slot = (x.nodes + 1) & ~1u;
-                fits = fits && y.slot + y.nodes <= lim;
+                if (y.slot + y.nodes > lim) {
+                    out.clear();
+                    break;
+                }
                 out.push_back(std::move(x));
                 if (out.back().mate) out.push_back(std::move(y));
             }
-            if (fits) return out;
-        }
-        return std::vector<ForestPlan>();
+        return out;
     };
     // Pairs where a CTA's cells do not fit one shared forest (1,024 cells, about
     // 8,850 nodes a CTA: 112 us per step, 140 in two shared forests one after

@@ -136,3 +136,12 @@ def test_eliminators_of_a_cluster(gpu, n, asked, warps):
     b.process(1)
     assert gpu.fake_elim_warps() == warps
     b.close()
+
+
+def test_pairs_are_as_few_as_the_nodes_need(gpu):
+    """One cell nearly as large as a pair of forests may be, and many small
+    ones: a lone forest and one pair, not a pair per handful of small cells."""
+    cells = [_cell(10700)] + [_cell(5 + i % 7, seed=i) for i in range(400)]
+    b = Batch(cells, DT, HS_PREC_MIXED, max_ctas=1)
+    assert (b.info()["n_forests"], b.info()["n_shared_forests"]) == (3, 3)
+    b.close()
