@@ -12,6 +12,7 @@ from moose_gb300.batch import Batch
 from moose_gb300.hsolve import HSolve, Tick
 
 DT = 25e-6
+KCA = models.kca_2d_tables(vdivs=30, cadivs=30)
 
 
 @pytest.fixture
@@ -23,7 +24,7 @@ def gpu():
 def _cell(n=40, seed=3, **kw):
     rng = np.random.default_rng([seed, n])
     parent, d, length = models.branched_morphology(rng, n, 0.5, 4)
-    return models.active_cell(parent, d, length, rng=rng, kca_tables=models.kca_2d_tables(vdivs=30, cadivs=30), **kw)
+    return models.active_cell(parent, d, length, rng=rng, kca_tables=KCA, **kw)
 
 
 def test_reads_wait_for_their_copy(gpu):
