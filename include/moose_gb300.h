@@ -401,11 +401,13 @@ typedef struct HsBatch HsBatch;
  * holds its elimination arrays in the CTA's shared memory (30 B per node),
  * so ctas_per_sm and forest_nodes set the forest size.  Cells of a CTA that do
  * not fit one such forest are stepped as pairs of forests that keep 16 B per
- * node there (CTAs of 640 threads or more, with eliminator warps), more than
- * two such pairs as one forest in global memory, or else as several forests,
- * the largest cells in global memory.  Changing either (or
- * max_ctas) on a mixed batch renumbers its nodes: its state, recording and
- * inject targets start over and hs_batch_reinit must follow. */
+ * node there, more than two such pairs as one forest in global memory; with
+ * trees of 256 levels or more, a cell too large for a pair, or the split off
+ * when the layout is made, as several forests, the largest cells in global
+ * memory.  Changing either (or max_ctas or cluster_ctas) on a mixed batch
+ * renumbers its nodes: its state, recording and inject targets start over and
+ * hs_batch_reinit must follow.  The other knobs change without a new layout,
+ * and no layout depends on their values before. */
 typedef struct HsBatchTuning {
     uint32_t threads_per_cta;   /* multiple of 32; FP64 <= 256 (default 128),
                                    mixed <= 1024 (default 1024) */
@@ -420,10 +422,16 @@ typedef struct HsBatchTuning {
                                    CTAs (0: ctas_per_sm x SM count); fewer,
                                    fuller forests leave SMs to other batches */
     uint32_t elim_warps;        /* mixed: warps of a CTA that eliminate while the
-                                   others assemble (default 4 to 8 by forest size;
-                                   of a pair, warps per forest, at most a fifth
-                                   of the CTA, the default; 0 keeps the
-                                   current value, 0xFFFFFFFF turns the split off) */
+                                   others assemble; 0 at creation: by layout (of
+                                   32 warps: 4 to 8 for a shared forest by its
+                                   size, 6 or 5 for each forest of a pair, 10 for
+                                   forests in global memory, twice the shared
+                                   ones' beside such with stop steps), later: the
+                                   current value.  A number is taken as it is for
+                                   shared forests, within 4 and the default for a
+                                   pair's, and from the default on for global
+                                   ones; a cluster has twice as many.
+                                   0xFFFFFFFF turns the split off */
     uint32_t wait_rounds;       /* mixed: most sleep rounds (~128 ns each) an
                                    eliminator waits for one level's assembly
                                    before it gives up; after that the launch
@@ -436,10 +444,10 @@ typedef struct HsBatchTuning {
                                    cluster (0 or 1: one CTA per group, the
                                    throughput layout; 2..8: a large cell
                                    assembled by several SMs, for latency).
-                                   With 2 or more every forest is eliminated
-                                   in global memory and may have at most 255
-                                   levels (else HS_ENOTSUP); changing it
-                                   re-lays the batch out. */
+                                   With 2 or more the first CTA eliminates, in
+                                   its shared memory, a forest of at most 255
+                                   levels and ~14,200 nodes (else HS_ENOTSUP);
+                                   changing it re-lays the batch out. */
 } HsBatchTuning;
 
 int hs_batch_create(const HsCellDesc* cells, const uint32_t* seeds,

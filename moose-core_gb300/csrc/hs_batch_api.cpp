@@ -37,8 +37,9 @@ namespace hsg {
 int setLastError(int code, const std::string& msg);
 cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, const uint32_t* ctaForests,
                                   uint32_t nCtas, uint32_t threadsPerCta, uint32_t smemBytes, uint32_t cap,
-                                  uint32_t deep, uint32_t pairWarps, uint32_t elimWarps, uint32_t minLevels,
-                                  uint32_t maxLevels, uint32_t modes, uint32_t nsteps, cudaStream_t st);
+                                  uint32_t deep, uint32_t pairWarps, uint32_t elimWarps, uint32_t globalWarps,
+                                  uint32_t minLevels, uint32_t maxLevels, uint32_t modes, uint32_t nsteps,
+                                  cudaStream_t st);
 cudaError_t launchForestStepMixedCluster(const MixBatch& b, const uint32_t* ctaPtr, const uint32_t* ctaForests,
                                          uint32_t nClusters, uint32_t kC, uint32_t threadsPerCta,
                                          uint32_t smemBytes, uint32_t cap, uint32_t stageCap, uint32_t elimWarps,
@@ -163,6 +164,7 @@ struct HsBatch {
     uint32_t mixMinLevels = 0, mixLevels = 0, mixMaxNodes = 0;      // of the forests
     uint32_t mixModes = 0;              // bits 1 << MixForest::shared (a cluster's: staged or not)
     bool mixPairs = false;              // forests stepped in pairs
+    bool mixMerged = false;             // CTAs of more than two pairs' nodes: one global forest each
     bool elimSet = false;               // elimWarps was asked for
     unsigned long long* dStopStep = nullptr;    // mixed: per-cell stop steps
     unsigned long long* dForestStop = nullptr;  // mixed: per-forest largest stop step
@@ -255,24 +257,33 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
                                             b->threadsPerCta, b->mixSmem, b->mixCap, b->mixStageCap, ce,
                                             b->mixModes, k, b->st);
     }
-    // Unless asked for a number, more eliminators for forests of wider levels:
-    // 4 up to 1,279 nodes, 8 from 2,048 (us per step with 4 / 6 / 8: 203 nodes
-    // 19.1 / 19.4 / 19.9, ~1,700 45.3 / 43.7 / 44.3, ~6,500 93.7 / 89.6 / 85.8).
-    if (ew && !b->elimSet && b->mixModes == 1u << kRowsGlobal && b->threadsPerCta >= 640)
-        ew = b->threadsPerCta * 10 / 1024;      // (4,096 cells merged: 6 487, 8 419, 10 396)
+    // The layout depends neither on threads_per_cta nor on how many elim_warps
+    // there are, which change without a new one: each layout takes any of them.
+    // Unless asked for a number, more eliminators for shared forests of wider
+    // levels: 4 up to 1,279 nodes, 8 from 2,048 (us per step with 4 / 6 / 8: 203
+    // nodes 19.1 / 19.4 / 19.9, ~1,700 45.3 / 43.7 / 44.3, ~6,500 93.7 / 89.6 / 85.8).
     if (ew && !b->elimSet && b->mixModes == 1u << kRowsShared)
         ew = std::max<uint32_t>(4, std::min(b->mixMaxNodes / 256, b->threadsPerCta / 128));
+    // A forest in global memory has wide levels of slow loads.  Where they bound
+    // the step, ten eliminator warps of 32, or more if asked for (4,096 cells
+    // merged: 4 612 us per step, 6 487, 8 420, 10 392; 608 cells and one of 30,000
+    // compartments, with stop steps: 10 322, 16 409).  Of a CTA's that has shared
+    // ones too, as a serving cohort's batch with its stop steps, twice the shared
+    // forests' (a 10,000-compartment cell 184 -> 159).
+    uint32_t gw = ew;
+    if (ew && (b->mixMerged || b->mixModes == 1u << kRowsGlobal)) gw = std::max(ew, b->threadsPerCta * 10 / 1024);
+    else if (b->mb.anyStop) gw = std::min(2 * ew, 16u);
     // Eliminators of each forest of a pair: 3/16 of the CTA (of 32 warps 6 each;
     // a population of 1,024 cells, 8,850 nodes a pair: 4 124, 5 117, 6 112, 8
     // 125 us per step; 2,048 cells 5 227, 6 222), of pairs of more than 10,240
-    // nodes, with their wider levels, one less (4,096 cells, 11,700 nodes: 5 406,
-    // 6 425); fewer if asked for; none (split off, or too few threads):
-    // forest after forest.
+    // nodes, with their wider levels, one less; fewer if asked for, but four (2:
+    // 172); none (split off, or too few threads): forest after forest.
     const uint32_t pw = b->threadsPerCta / (b->mixPairNodes > 10240 ? 192 : 160);
-    const uint32_t pairWarps = !b->mixPairs || !b->elimWarps ? 0 : b->elimSet ? std::min(b->elimWarps, pw) : pw;
+    const uint32_t pairWarps = !b->mixPairs || !b->elimWarps ? 0
+                               : b->elimSet ? std::min(std::max(b->elimWarps, 4u), pw) : pw;
     return launchForestStepMixed(b->mb, b->dCtaPtr, b->dCtaForests, b->nCtas, b->threadsPerCta, b->mixSmem,
-                                 b->mixPairs ? b->mixHalf : b->mixCap, b->mixDeep, pairWarps, ew, b->mixMinLevels,
-                                 b->mixLevels, b->mixModes, k, b->st);
+                                 b->mixPairs ? b->mixHalf : b->mixCap, b->mixDeep, pairWarps, ew, gw,
+                                 b->mixMinLevels, b->mixLevels, b->mixModes, k, b->st);
 }
 
 // Packing of the FP64 batch: one block per SM, in teams (hsBatchStepFp64).
@@ -811,28 +822,29 @@ int buildMixed(HsBatch* b) {
     // its tail and back substitution are a small part by then, and nothing
     // waits between the pairs (4,096 cells: 396 us per step with ten eliminator
     // warps, 415 in pairs; 2,048 cells, two pairs: 229 and 221).
-    bool merge = false;
+    // Without eliminator warps, or with a forest of 256 levels or more: shared
+    // and global forests one after the other.
     std::vector<std::vector<ForestPlan>> pairsOf;
-    b->mixPairs = false;
-    if (b->mixDeep && b->elimWarps && b->threadsPerCta >= 640) {
-        for (uint32_t k = 0; k < nCtas; ++k) {
-            uint64_t total = 0;
-            for (uint32_t c : ctaCells[k]) total += trees[c].T;
-            b->mixPairs = b->mixPairs || total > room;
-            merge = merge || total > 2 * half;
-        }
-        for (uint32_t c = 0; b->mixPairs && c < nC; ++c) b->mixPairs = treeLevels(trees[c]) < kWsLevels;
-        merge = merge && b->mixPairs && (!b->elimSet || b->elimWarps >= 10);   // (with 8: 419)
-        if (merge) b->mixPairs = false;
-        for (uint32_t k = 0; b->mixPairs && k < nCtas; ++k) {
-            pairsOf.push_back(pairForests(ctaCells[k], half));
-            b->mixPairs = !pairsOf.back().empty() || ctaCells[k].empty();
-        }
+    std::vector<uint64_t> total(nCtas, 0);
+    b->mixPairs = b->mixMerged = false;
+    for (uint32_t k = 0; k < nCtas; ++k) {
+        for (uint32_t c : ctaCells[k]) total[k] += trees[c].T;
+        b->mixPairs = b->mixPairs || total[k] > room;
+        b->mixMerged = b->mixMerged || total[k] > 2 * half;
+    }
+    b->mixPairs = b->mixPairs && b->mixDeep && b->elimWarps;
+    for (uint32_t c = 0; b->mixPairs && c < nC; ++c) b->mixPairs = treeLevels(trees[c]) < kWsLevels;
+    b->mixMerged = b->mixMerged && b->mixPairs;
+    if (b->mixMerged) b->mixPairs = false;
+    for (uint32_t k = 0; b->mixPairs && k < nCtas; ++k) {
+        pairsOf.push_back(pairForests(ctaCells[k], half));
+        b->mixPairs = !pairsOf.back().empty() || ctaCells[k].empty();
     }
     std::vector<ForestPlan> forests;
     std::vector<uint32_t> ctaPtr(nCtas + 1, 0), ctaForests;
     for (uint32_t k = 0; k < nCtas; ++k) {
         std::vector<ForestPlan> fs;
+        const bool merge = b->mixMerged;
         if (b->mixPairs) {
             fs.swap(pairsOf[k]);
             ctaCells[k].clear();

@@ -1114,6 +1114,8 @@ __device__ __forceinline__ void stageForest(const MixBatch& b, const MixForest& 
 // arrays of `cap` nodes: D, R, OFF (8 B each), TOPO (4 B), PAR (2 B); for
 // half-shared ones D and R of `cap` nodes.  `deep`: doubles before them that
 // belong to the level offsets.
+// `elimWarps`, `globalWarps`: eliminators of a forest in shared and in global
+// memory.
 // kStops: the batch has stop steps (b.anyStop); kSteps: how its forests are
 // stepped, kSplit (stepForestWS), kUnsplit (stepForest: 256 levels or more, or
 // no eliminator warps), or some each way; kModes: where their arrays may be
@@ -1126,7 +1128,8 @@ constexpr uint32_t kSplit = 1, kUnsplit = 2;      // bits of kSteps
 template <bool kStops, uint32_t kSteps, uint32_t kModes>
 __global__ void __launch_bounds__(1024, 1) hsForestStepMixed(MixBatch b, const uint32_t* __restrict__ ctaPtr,
                                                              const uint32_t* __restrict__ ctaForests, uint32_t cap,
-                                                             uint32_t deep, uint32_t elimWarps, uint32_t nsteps) {
+                                                             uint32_t deep, uint32_t elimWarps,
+                                                             uint32_t globalWarps, uint32_t nsteps) {
     constexpr bool kAhead = kSteps != (kSplit | kUnsplit) && (kModes & (kModes - 1)) == 0;
     copyTypes(b);
     for (uint32_t k = ctaPtr[blockIdx.x]; k < ctaPtr[blockIdx.x + 1]; ++k) {
@@ -1158,23 +1161,19 @@ __global__ void __launch_bounds__(1024, 1) hsForestStepMixed(MixBatch b, const u
             c.shared = F.shared;
         }
         __syncthreads();
-        // a forest not all in shared memory (a cell too large for it,
-        // as serving requests can be) has wide levels of slow loads:
-        // twice the eliminator warps (measured on a 10,000-compartment cell:
-        // 184 -> 159 us per step).  Only in the instantiation for batches
-        // with stop steps, so that the throughput kernel's registers stay
-        // as they are.
-        const uint32_t f = ctaForests[k], ew = kStops && F.shared != kRowsShared ? min(2 * elimWarps, 16u) : elimWarps;
-        const bool plain = kSteps == kUnsplit ||
-                           (kSteps != kSplit && !(ew && F.nLevels < kWsLevels && blockDim.x > 32 * ew));
+        const uint32_t f = ctaForests[k];
+        auto plain = [&](uint32_t warps) {
+            return kSteps == kUnsplit ||
+                   (kSteps != kSplit && !(warps && F.nLevels < kWsLevels && blockDim.x > 32 * warps));
+        };
         if ((kModes & 1u << kRowsShared) && F.shared == kRowsShared) {
-            if (plain) stepForest<kAhead>(b, F, f, S, lp, nsteps);
-            else stepForestWS<kStops, kAhead>(b, f, S, ew, nsteps);
+            if (plain(elimWarps)) stepForest<kAhead>(b, F, f, S, lp, nsteps);
+            else stepForestWS<kStops, kAhead>(b, f, S, elimWarps, nsteps);
         } else if (kModes & 1u << kRowsHalf) {
             stepForest<kAhead>(b, F, f, HalfRows{b, F.node0, F.slot + deep, cap}, lp, nsteps);
         } else if (kModes & 1u << kRowsGlobal) {
-            if (plain) stepForest<kAhead>(b, F, f, G, lp, nsteps);
-            else stepForestWS<kStops, kAhead>(b, f, G, ew, nsteps);
+            if (plain(globalWarps)) stepForest<kAhead>(b, F, f, G, lp, nsteps);
+            else stepForestWS<kStops, kAhead>(b, f, G, globalWarps, nsteps);
         }
     }
 }
@@ -1483,7 +1482,8 @@ cudaError_t launchForestStepMixedCluster(const MixBatch& b, const uint32_t* ctaP
 
 cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, const uint32_t* ctaForests,
                                   uint32_t nCtas, uint32_t threadsPerCta, uint32_t smemBytes, uint32_t cap,
-                                  uint32_t deep, uint32_t pairWarps, uint32_t elimWarps, uint32_t minLevels, uint32_t maxLevels, uint32_t modes, uint32_t nsteps,
+                                  uint32_t deep, uint32_t pairWarps, uint32_t elimWarps, uint32_t globalWarps,
+                                  uint32_t minLevels, uint32_t maxLevels, uint32_t modes, uint32_t nsteps,
                                   cudaStream_t st) {
     // maxLevels: the deepest forest's levels; modes: bits 1 << MixForest::shared
     if (pairWarps) {
@@ -1493,7 +1493,7 @@ cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, con
         kern<<<nCtas, threadsPerCta, smemBytes, st>>>(b, ctaPtr, ctaForests, cap, pairWarps, nsteps);
         return cudaGetLastError();
     }
-    const uint32_t warps = b.anyStop ? std::min(2 * elimWarps, 16u) : elimWarps;
+    const uint32_t warps = std::max(elimWarps, globalWarps);
     constexpr uint32_t S = 1u << kRowsShared, G = 1u << kRowsGlobal;
     auto kern = b.anyStop ? hsForestStepMixed<true, kSplit | kUnsplit, S | G>
                           : hsForestStepMixed<false, kSplit | kUnsplit, S | G>;
@@ -1501,13 +1501,13 @@ cudaError_t launchForestStepMixed(const MixBatch& b, const uint32_t* ctaPtr, con
         if (modes == S) kern = b.anyStop ? hsForestStepMixed<true, kSplit, S> : hsForestStepMixed<false, kSplit, S>;
         else if (modes == G) kern = b.anyStop ? hsForestStepMixed<true, kSplit, G> : hsForestStepMixed<false, kSplit, G>;
         else kern = b.anyStop ? hsForestStepMixed<true, kSplit, S | G> : hsForestStepMixed<false, kSplit, S | G>;
-    } else if (!elimWarps || minLevels >= kWsLevels || threadsPerCta <= 32 * elimWarps) {
+    } else if (!elimWarps || minLevels >= kWsLevels || threadsPerCta <= 32 * std::min(elimWarps, globalWarps)) {
         kern = modes == S ? hsForestStepMixed<true, kUnsplit, S> : hsForestStepMixed<true, kUnsplit, S | G>;
     }
     if (modes == 1u << kRowsHalf) kern = hsForestStepMixed<true, kUnsplit, 1u << kRowsHalf>;
     cudaError_t e = allowShared((const void*)kern);
     if (e != cudaSuccess) return e;
-    kern<<<nCtas, threadsPerCta, smemBytes, st>>>(b, ctaPtr, ctaForests, cap, deep, elimWarps, nsteps);
+    kern<<<nCtas, threadsPerCta, smemBytes, st>>>(b, ctaPtr, ctaForests, cap, deep, elimWarps, globalWarps, nsteps);
     return cudaGetLastError();
 }
 

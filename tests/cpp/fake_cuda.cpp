@@ -40,7 +40,7 @@ void drop(void* p) {
 }
 
 int g_queries = 0, g_waits = 0;     // calls of cudaEventQuery and cudaStreamWaitEvent
-uint32_t g_elimWarps = 0;           // of the last mixed step
+uint32_t g_elimWarps = 0;           // of the last mixed step: of a pair's, else a global, else a shared forest
 int g_device = 0;
 std::map<std::pair<int, const void*>, int> g_limit;      // dynamic shared memory each kernel may take, per device
 const hsg::DevCell* g_cells = nullptr;      // of the last reinit
@@ -210,8 +210,9 @@ cudaError_t launchGatherSpikes(const DevCell*, const uint32_t*, const float*, ui
 
 // ---- mixed ---------------------------------------------------------------------
 cudaError_t launchForestStepMixed(const MixBatch&, const uint32_t*, const uint32_t*, uint32_t, uint32_t, uint32_t,
-                                  uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t,
-                                  cudaStream_t) {
+                                  uint32_t, uint32_t, uint32_t pairWarps, uint32_t elimWarps, uint32_t globalWarps,
+                                  uint32_t, uint32_t, uint32_t modes, uint32_t, cudaStream_t) {
+    g_elimWarps = pairWarps ? pairWarps : modes == 1u << kRowsShared ? elimWarps : globalWarps;
     return cudaSuccess;
 }
 cudaError_t launchForestStepMixedCluster(const MixBatch&, const uint32_t*, const uint32_t*, uint32_t, uint32_t,

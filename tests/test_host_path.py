@@ -146,3 +146,45 @@ def test_pairs_are_as_few_as_the_nodes_need(gpu):
     b = Batch(cells, DT, HS_PREC_MIXED, max_ctas=1)
     assert (b.info()["n_forests"], b.info()["n_shared_forests"]) == (3, 3)
     b.close()
+
+
+# a CTA's cells: one shared forest, a pair of forests, one merged in global memory
+CTAS = {"shared": ([2000, 900], (1, 1)), "pair": ([5000, 4000], (2, 2)), "merged": ([12000, 9000, 8000], (1, 0))}
+
+
+def _forests(b):
+    return b.info()["n_forests"], b.info()["n_shared_forests"]
+
+
+@pytest.mark.parametrize("kind", CTAS)
+def test_layout_does_not_depend_on_the_tunings_before(gpu, kind):
+    """threads_per_cta and elim_warps change without a new layout, so the same
+    one is made for all of them, whichever came first."""
+    sizes, forests = CTAS[kind]
+    cells = [_cell(n) for n in sizes]
+    tunings = [dict(), dict(elim_warps=4), dict(elim_warps=8), dict(threads_per_cta=512), dict(threads_per_cta=128)]
+    for t in tunings:
+        b = Batch(cells, DT, HS_PREC_MIXED, max_ctas=1, **t)
+        assert _forests(b) == forests, t
+        for t2 in tunings:
+            b.tune(max_ctas=1, **t2)
+            assert _forests(b) == forests, (t, t2)
+            b.tune(max_ctas=2, **t2)
+            b.tune(max_ctas=1, **t)             # laid out again
+            assert _forests(b) == forests, (t, t2)
+        b.close()
+
+
+@pytest.mark.parametrize("kind, asked, warps", [("shared", 0, 8), ("shared", 3, 3), ("pair", 0, 6), ("pair", 2, 4),
+                                                ("pair", 5, 5), ("pair", 9, 6), ("merged", 0, 10), ("merged", 4, 10),
+                                                ("merged", 12, 12)])
+@pytest.mark.parametrize("stops", [False, True])
+def test_eliminators_by_layout(gpu, kind, asked, warps, stops):
+    cells = [_cell(n) for n in CTAS[kind][0]]
+    b = Batch(cells, DT, HS_PREC_MIXED, max_ctas=1, elim_warps=asked)
+    if stops:
+        b.set_stop_steps([100] * len(cells))
+    b.reinit(DT)
+    b.process(1)
+    assert gpu.fake_elim_warps() == warps
+    b.close()
