@@ -822,6 +822,9 @@ int buildMixed(HsBatch* b) {
     // its tail and back substitution are a small part by then, and nothing
     // waits between the pairs (4,096 cells: 396 us per step with ten eliminator
     // warps, 415 in pairs; 2,048 cells, two pairs: 229 and 221).
+    // Only CTAs that do not fit a shared forest are merged, so that beside one
+    // very large cell the others stay in shared memory (608 cells, one more of
+    // 30,000 compartments at its stop step: 91 us per step, 118 with all merged).
     // Without eliminator warps, or with a forest of 256 levels or more: shared
     // and global forests one after the other.
     std::vector<std::vector<ForestPlan>> pairsOf;
@@ -844,7 +847,7 @@ int buildMixed(HsBatch* b) {
     std::vector<uint32_t> ctaPtr(nCtas + 1, 0), ctaForests;
     for (uint32_t k = 0; k < nCtas; ++k) {
         std::vector<ForestPlan> fs;
-        const bool merge = b->mixMerged;
+        const bool merge = b->mixMerged && total[k] > room;
         if (b->mixPairs) {
             fs.swap(pairsOf[k]);
             ctaCells[k].clear();

@@ -188,3 +188,9 @@ def test_eliminators_by_layout(gpu, kind, asked, warps, stops):
     b.process(1)
     assert gpu.fake_elim_warps() == warps
     b.close()
+
+
+def test_one_very_large_cell_leaves_the_others_in_shared_memory(gpu):
+    b = Batch([_cell(22000)] + [_cell(900, seed=i) for i in range(4)], DT, HS_PREC_MIXED, max_ctas=3)
+    assert _forests(b) == (3, 2)
+    b.close()
