@@ -273,12 +273,13 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
     uint32_t gw = ew;
     if (ew && (b->mixMerged || b->mixModes == 1u << kRowsGlobal)) gw = std::max(ew, b->threadsPerCta * 10 / 1024);
     else if (b->mb.anyStop) gw = std::min(2 * ew, 16u);
-    // Eliminators of each forest of a pair: 3/16 of the CTA (of 32 warps 6 each;
-    // a population of 1,024 cells, 8,850 nodes a pair: 4 124, 5 117, 6 112, 8
-    // 125 us per step; 2,048 cells 5 227, 6 222), of pairs of more than 10,240
-    // nodes, with their wider levels, one less; fewer if asked for, but four (2:
-    // 172); none (split off, or too few threads): forest after forest.
-    const uint32_t pw = b->threadsPerCta / (b->mixPairNodes > 10240 ? 192 : 160);
+    // Eliminators of each forest of a pair: 3/16 of the CTA, of pairs of more than
+    // 12,288 nodes, with their wider levels, one of 32 warps less (us per step with
+    // 5 and 6; one pair of 8,850 nodes 117 and 114, of 11,100 127 and 123, of 13,700
+    // 152 and 160; two of 8,750 227 and 222, of 10,300 242 and 244); fewer if asked
+    // for, but four (8,850 nodes: 4 125, 2 172); none (split off, or too few
+    // threads): forest after forest.
+    const uint32_t pw = b->threadsPerCta / (b->mixPairNodes > 12288 ? 192 : 160);
     const uint32_t pairWarps = !b->mixPairs || !b->elimWarps ? 0
                                : b->elimSet ? std::min(std::max(b->elimWarps, 4u), pw) : pw;
     return launchForestStepMixed(b->mb, b->dCtaPtr, b->dCtaForests, b->nCtas, b->threadsPerCta, b->mixSmem,
