@@ -325,8 +325,8 @@ int hs_create(const HsCellDesc* cell, uint32_t seed, double dt, int precision, H
     }
     const uint32_t spikeCap = 1u << 16;
     Arena dry, drySpikes;
-    std::vector<std::shared_ptr<void>> sent;
-    layoutCell(s->P, dry, s->dc, spikeCap, stOf(s), sent, nullptr, &drySpikes);
+    CellUpload up;
+    layoutCell(s->P, dry, s->dc, spikeCap, stOf(s), up, nullptr, &drySpikes);
     dry.take<DevCell>(1);
     s->arena.size = dry.used + 256;
     s->spikes.size = drySpikes.used;
@@ -334,7 +334,7 @@ int hs_create(const HsCellDesc* cell, uint32_t seed, double dt, int precision, H
     if (e == cudaSuccess) e = cudaMalloc(&s->spikes.base, s->spikes.size);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->arena.base, 0, s->arena.size, stOf(s));
     if (e == cudaSuccess) e = cudaMemsetAsync(s->spikes.base, 0, s->spikes.size, stOf(s));
-    if (e == cudaSuccess) e = layoutCell(s->P, s->arena, s->dc, spikeCap, stOf(s), sent, nullptr, &s->spikes);
+    if (e == cudaSuccess) e = layoutCell(s->P, s->arena, s->dc, spikeCap, stOf(s), up, nullptr, &s->spikes);
     s->dcDev = s->arena.take<DevCell>(1);
     s->descPtr = s->dc.evPtr;
     s->descCur = s->dc.evCur;

@@ -406,7 +406,7 @@ uint32_t deliveryStep(double t, double dt) {
 
 int buildFp64(HsBatch* b, const HsCellDesc* cells) {
     const uint32_t nC = b->nCells;
-    std::vector<std::shared_ptr<void>> sent;        // host copies under way to the device
+    CellUpload up;
     // shared V/Ca tables by content and columns (pairTable's differences
     // depend on both), 2-D tables by source identity
     std::map<std::tuple<uint64_t, size_t, uint32_t>, const double*> tabDev;
@@ -442,7 +442,7 @@ int buildFp64(HsBatch* b, const HsCellDesc* cells) {
             if (it == tabDev.end()) {
                 auto pairs = std::make_shared<std::vector<double>>(pairTable(T));
                 it = tabDev.emplace(key, b->buf.up(*pairs, b->st)).first;
-                sent.push_back(pairs);
+                up.sent.push_back(pairs);
             }
             (pass ? catab : vtab)[c] = it->second;
         }
@@ -478,7 +478,8 @@ int buildFp64(HsBatch* b, const HsCellDesc* cells) {
         sh[c].caTab = catab[c];
         sh[c].g2dBase = g2dBase;
         sh[c].g2dOff = g2dOffs[c];
-        layoutCell(b->plans[c], dry, b->dcs[c], b->spikeCap, b->st, sent, &sh[c]);
+        layoutCell(b->plans[c], dry, b->dcs[c], b->spikeCap, b->st, up, &sh[c]);
+        up.programs.reset();        // (of all cells at once they are too many to keep)
     }
     b->arena.size = dry.used + 256;
     e = cudaMallocAsync(&b->arena.base, b->arena.size, b->st);
@@ -486,11 +487,11 @@ int buildFp64(HsBatch* b, const HsCellDesc* cells) {
     size_t kept = 0;
     for (uint32_t c = 0; c < nC && e == cudaSuccess; ++c) {
         const size_t from = b->arena.used;
-        e = layoutCell(b->plans[c], b->arena, b->dcs[c], b->spikeCap, b->st, sent, &sh[c]);
+        e = layoutCell(b->plans[c], b->arena, b->dcs[c], b->spikeCap, b->st, up, &sh[c]);
         kept += b->arena.used - from;
         if (e == cudaSuccess && (kept > (64u << 20) || c + 1 == nC)) {
             e = cudaStreamSynchronize(b->st);
-            sent.clear();
+            up.sent.clear();
             kept = 0;
         }
     }

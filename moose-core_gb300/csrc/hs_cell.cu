@@ -25,8 +25,12 @@ struct Uploader {
     template <class T>
     T* put(const std::vector<T>& v) {
         T* p = a.take<T>(v.empty() ? 1 : v.size());
-        if (p && !v.empty() && err == cudaSuccess) add(reinterpret_cast<char*>(p) - a.base, v.data(), v.size() * sizeof(T));
+        if (p) send(p, v);
         return p;
+    }
+    template <class T>
+    void send(T* p, const std::vector<T>& v) {
+        if (!v.empty() && err == cudaSuccess) add(reinterpret_cast<char*>(p) - a.base, v.data(), v.size() * sizeof(T));
     }
     template <class T>
     T* put(std::vector<T>&& v) {
@@ -95,12 +99,16 @@ struct Compact {
     std::vector<uint4> fW, bW, fLane, bLane;
     std::vector<uint32_t> bX;
     std::vector<uint2> fSeg, bSeg;
-    bool split = true;
+    bool split = true, made = false;
 };
 
 bool compactPrograms(const CellPlan& P, Compact& C) {
     const uint32_t N = P.N, offBase = 2 * N + P.H, kNone = 0xFFFFu, kOff = 0xFFFEu;
     if (offBase >= kOff) return false;
+    C.fW.reserve(2 * P.fWaveOps.size());
+    C.bW.reserve(2 * P.bRows.size());
+    C.fLane.reserve(32 * P.fWavePtr.size());
+    C.bLane.reserve(64 * P.bLevelPtr.size());
     auto offOf = [&](uint32_t row) {
         uint64_t u = 0;
         if (row < N) std::memcpy(&u, &P.off[row], 8);
@@ -198,9 +206,8 @@ bool compactPrograms(const CellPlan& P, Compact& C) {
 }  // namespace
 
 cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCap,
-                       cudaStream_t st, std::vector<std::shared_ptr<void>>& sent, const CellShared* sh,
-                       Arena* spikes) {
-    Uploader u{a, st, sent};
+                       cudaStream_t st, CellUpload& up, const CellShared* sh, Arena* spikes) {
+    Uploader u{a, st, up.sent};
     const uint32_t N = P.N, H = P.H;
     std::memset(&c, 0, sizeof(c));
     c.N = N; c.H = H; c.C = P.C; c.G = P.G; c.P = P.P; c.K2 = P.K2; c.S = P.S; c.SG = P.SG;
@@ -232,40 +239,48 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.poolPtr = u.put(P.poolPtr);
     c.extPtr = u.put(P.extPtr);
     c.extList = u.put(P.extList);
-    c.fLevelPtr = u.put(P.fLevelPtr);
-    c.fOpPtr = u.put(P.fOpPtr);
-    c.fOps = reinterpret_cast<const int4*>(u.put(P.fOps));
+    if (P.fWavePtr.empty()) {       // (with waves, nothing reads the forward level programs)
+        c.fLevelPtr = u.put(P.fLevelPtr);
+        c.fOpPtr = u.put(P.fOpPtr);
+        c.fOps = reinterpret_cast<const int4*>(u.put(P.fOps));
+        c.fRun = u.put(P.fRun);
+        c.fRunRow = u.put(P.fRunRow);
+    }
     c.bLevelPtr = u.put(P.bLevelPtr);
     c.bRows = u.put(P.bRows);
     c.bTermPtr = u.put(P.bTermPtr);
     c.bTerms = reinterpret_cast<const int2*>(u.put(P.bTerms));
-    c.fRun = u.put(P.fRun);
-    c.fRunRow = u.put(P.fRunRow);
     c.bRun = u.put(P.bRun);
     c.bRunRow = u.put(P.bRunRow);
     c.fWaves = P.fWavePtr.empty() ? 0 : (uint32_t)P.fWavePtr.size() - 1;
     c.fWavePtr = u.put(P.fWavePtr);
     c.fWaveOps = reinterpret_cast<const int4*>(u.put(P.fWaveOps));
     {
-        Compact C;
-        const bool compact = compactPrograms(P, C);
-        if (!compact) C = Compact();
+        auto programs = std::static_pointer_cast<Compact>(up.programs);
+        if (!programs) {
+            programs = std::make_shared<Compact>();
+            if (!compactPrograms(P, *programs)) *programs = Compact();
+            else programs->made = true;
+        }
+        up.programs = a.base ? nullptr : programs;
+        Compact& C = *programs;
         uint32_t longest = 0;      // runs walked as runs: forward only without waves
         for (uint32_t r : P.bRun) longest = std::max(longest, r);
         if (P.fWavePtr.empty())
             for (uint32_t r : P.fRun) longest = std::max(longest, r);
         c.runRows = longest >= kWarpRun ? longest : 0;
-        c.smWords = compact ? 2 * N + H + 2 * c.runRows : 0;
+        c.smWords = C.made ? 2 * N + H + 2 * c.runRows : 0;
         c.fSplit = C.split;
-        c.fW = u.put(std::move(C.fW));
-        c.bW = u.put(std::move(C.bW));
-        c.bX = u.put(std::move(C.bX));
-        c.fLane = u.put(std::move(C.fLane));
-        c.bLane = u.put(std::move(C.bLane));
         c.nfSeg = (uint32_t)C.fSeg.size();
         c.nbSeg = (uint32_t)C.bSeg.size();
-        c.fSeg = u.put(std::move(C.fSeg));
-        c.bSeg = u.put(std::move(C.bSeg));
+        c.fW = u.put(C.fW);
+        c.bW = u.put(C.bW);
+        c.bX = u.put(C.bX);
+        c.fLane = u.put(C.fLane);
+        c.bLane = u.put(C.bLane);
+        c.fSeg = u.put(C.fSeg);
+        c.bSeg = u.put(C.bSeg);
+        if (a.base) up.sent.push_back(programs);
     }
     c.Gbar = u.put(P.Gbar);
     c.Ek = u.put(P.Ek);
@@ -322,14 +337,13 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.caRows = P.caTable.nPts;
     c.caRdx = 1.0 / c.caDx;
     {
-        std::vector<double> AB, geom;
+        std::vector<double> geom;
         std::vector<uint64_t> off;
         std::vector<uint32_t> nn;
+        size_t nAB = 0;
         for (const Gate2D& g : P.gates2d) {
-            if (!sh) {
-                off.push_back(AB.size());
-                AB.insert(AB.end(), g.AB.begin(), g.AB.end());
-            }
+            off.push_back(nAB);
+            nAB += g.AB.size();
             geom.insert(geom.end(), {g.xmin, g.xmax, g.ymin, g.ymax, g.invDx, g.invDy});
             nn.push_back(g.nx);
             nn.push_back(g.ny);
@@ -338,7 +352,9 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
             c.g2dAB = sh->g2dBase;
             c.g2dOff = u.put(sh->g2dOff);
         } else {
-            c.g2dAB = u.put(std::move(AB));
+            double* AB = a.take<double>(nAB ? nAB : 1);
+            c.g2dAB = AB;
+            for (size_t g = 0; AB && g < off.size(); ++g) u.send(AB + off[g], P.gates2d[g].AB);
             c.g2dOff = u.put(std::move(off));
         }
         c.g2dGeom = u.put(std::move(geom));

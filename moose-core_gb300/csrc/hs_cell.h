@@ -31,9 +31,7 @@ struct Arena {
 // constants of all cells contiguous, for one-copy reinit) and rate tables
 // shared by the cells that have identical ones.  `spikes`: where the spike
 // buffers go, if not into `a` (a drop-in solver's: an allocation of more than
-// 1 MiB costs 57 us to make and free, two smaller ones 4).  `sent` takes the
-// host copies made on the way, which the caller keeps until it has waited for
-// `st`: a copy from pageable memory may be under way when its call returns.
+// 1 MiB costs 57 us to make and free, two smaller ones 4).
 std::vector<double> pairTable(const Table& t);   // rate table as the FP64 kernels read it (DevCell::vTab)
 struct CellShared {
     double* initVm = nullptr;
@@ -43,9 +41,16 @@ struct CellShared {
     const double* g2dBase = nullptr;
     std::vector<uint64_t> g2dOff;    // per gate2d of the cell, offset from g2dBase
 };
+// `sent`: host copies made on the way, which the caller keeps until it has
+// waited for `st` (a copy from pageable memory may be under way when its call
+// returns); `programs`: the cell's sweeps, from the dry run to the upload, or
+// null to work them out again.
+struct CellUpload {
+    std::vector<std::shared_ptr<void>> sent;
+    std::shared_ptr<void> programs;
+};
 cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& dc, uint32_t spikeCap,
-                       cudaStream_t st, std::vector<std::shared_ptr<void>>& sent,
-                       const CellShared* shared = nullptr, Arena* spikes = nullptr);
+                       cudaStream_t st, CellUpload& up, const CellShared* shared = nullptr, Arena* spikes = nullptr);
 
 // SynChan reinit constants of one cell at the clock dt, 5 per SynChan
 // (xc1, xc2, yc1, yc2, norm), computed with the host libm as the reference does.

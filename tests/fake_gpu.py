@@ -24,7 +24,7 @@ def _build():
         return so
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
     inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(nvcc))), "include")
-    flags = ["-O1", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fvisibility=default", "-I", CSRC, "-I", inc]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-ffp-contract=off", "-fvisibility=default", "-I", CSRC, "-I", inc]
     objs = [os.path.join(OUT, os.path.basename(u) + ".fake.o") for u in units]
     procs = [subprocess.Popen(["g++"] + flags + ["-x", "c++", "-c", u, "-o", o], stderr=subprocess.PIPE, text=True)
              for u, o in zip(units, objs)]
