@@ -239,7 +239,8 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.poolPtr = u.put(P.poolPtr);
     c.extPtr = u.put(P.extPtr);
     c.extList = u.put(P.extList);
-    if (P.fWavePtr.empty()) {       // (with waves, nothing reads the forward level programs)
+    c.fWaves = P.fWavePtr.empty() ? 0 : (uint32_t)P.fWavePtr.size() - 1;
+    if (!c.fWaves) {                // (with waves, nothing reads the forward level programs)
         c.fLevelPtr = u.put(P.fLevelPtr);
         c.fOpPtr = u.put(P.fOpPtr);
         c.fOps = reinterpret_cast<const int4*>(u.put(P.fOps));
@@ -252,7 +253,6 @@ cudaError_t layoutCell(const CellPlan& P, Arena& a, DevCell& c, uint32_t spikeCa
     c.bTerms = reinterpret_cast<const int2*>(u.put(P.bTerms));
     c.bRun = u.put(P.bRun);
     c.bRunRow = u.put(P.bRunRow);
-    c.fWaves = P.fWavePtr.empty() ? 0 : (uint32_t)P.fWavePtr.size() - 1;
     c.fWavePtr = u.put(P.fWavePtr);
     c.fWaveOps = reinterpret_cast<const int4*>(u.put(P.fWaveOps));
     {

@@ -88,6 +88,14 @@ uint32_t fake_elim_warps() { return g_elimWarps; }
 int fake_queries() { return g_queries; }
 int fake_waits() { return g_waits; }
 
+// Whether cell k of the last reinit has a program for its forward sweep.
+int fake_has_forward(uint32_t k) {
+    drain();
+    if (k >= g_nCells) return -1;
+    const hsg::DevCell& c = g_cells[k];
+    return c.fWaves ? c.fWavePtr && c.fWaveOps : c.fLevelPtr && c.fOpPtr && c.fOps && c.fRun && c.fRunRow;
+}
+
 // Readies a kernel for its launches on `device`, and what they may take there.
 int fake_allow(uint64_t id, int device) {
     g_device = device;

@@ -194,3 +194,14 @@ def test_one_very_large_cell_leaves_the_others_in_shared_memory(gpu):
     b = Batch([_cell(22000)] + [_cell(900, seed=i) for i in range(4)], DT, HS_PREC_MIXED, max_ctas=3)
     assert _forests(b) == (3, 2)
     b.close()
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 40, 300])
+def test_every_cell_has_its_forward_program(gpu, n):
+    """A cell of one compartment has waves, but none of them."""
+    for m in ([models.config1_cell(n_cable=n - 1)] if n > 1 else []) + [_cell(n)]:
+        h = HSolve(m, dt=DT)
+        h.target = m.seed
+        h.reinit(DT)
+        assert gpu.fake_has_forward(0) == 1
+        h.close()
