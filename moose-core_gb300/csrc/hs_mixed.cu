@@ -629,8 +629,10 @@ __device__ __forceinline__ void groupSync(uint32_t id, uint32_t count) {
 
 // A counter in shared memory that orders what its threads wrote before
 // (release) and read after (acquire), within the CTA: a full fence would also
-// wait for the reads a thread has under way.  kCluster: threads of the
-// cluster's other CTAs add to it too.
+// wait for the reads a thread has under way (in the eliminators of a cluster it
+// took 6 to 18 us of a step: 9,001 compartments on 4 CTAs 122 us with, 103 without;
+// 3,500 62 and 56).  kCluster: threads of the cluster's other CTAs add to it
+// too, after a fence of cluster scope.
 template <bool kCluster>
 __device__ __forceinline__ uint32_t loadAcquire(const uint32_t* p) {
     uint32_t v;
@@ -889,7 +891,6 @@ __device__ __forceinline__ void forwardHalf(const MixBatch& b, const HalfRows& E
     for (int L = (int)nL - 1; L >= 0; --L) {
         const bool narrow = 2 * (e - b0) <= nE;
         waitLevel<kCluster>(b, &done[L], e - b0, gaveUp);
-        if (kCluster) fenceCluster();
         for (;; i += nE) {
             const bool last = i + nE >= e;       // of this level
             const uint32_t i0 = i;
@@ -1343,7 +1344,6 @@ __device__ __forceinline__ void stepForestCluster(const MixBatch& b, const MixFo
                 for (int L = (int)F.nLevels - 1; L >= 0; --L) {
                     const uint32_t b0 = lp[L], e = lp[L + 1];
                     waitLevel<true>(b, &done[L], e - b0, waitGaveUp);
-                    fenceCluster();
                     if (2 * (e - b0) <= nE) {
                         pullNarrow(E, b0, e, tid);
                     } else {
