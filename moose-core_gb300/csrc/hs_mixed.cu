@@ -756,8 +756,9 @@ __device__ __forceinline__ void stepForestWS(const MixBatch& b, uint32_t f, cons
         __syncthreads();
         if (tid == 0) sCtl().step = sCtl().step + 1;      // (read next after the barriers of the back substitution)
         // back substitution by the whole CTA
+        const uint32_t nL = F.nLevels;
         if (F.shared == kRowsShared) {
-            for (uint32_t L = 0; L < F.nLevels; ++L) {
+            for (uint32_t L = 0; L < nL; ++L) {
                 const uint32_t e = lp[L + 1];
                 for (uint32_t i = lp[L] + tid; i < e; i += nth) {
                     const uint32_t p = E.PAR(i);
@@ -779,10 +780,10 @@ __device__ __forceinline__ void stepForestWS(const MixBatch& b, uint32_t f, cons
                 dn = E.D(nb);
                 rn = E.R(nb);
             }
-            for (uint32_t L = 0; L < F.nLevels; ++L) {
+            for (uint32_t L = 0; L < nL; ++L) {
                 const uint32_t i0 = nb, e = ne, p0 = pn;
                 const double d0 = dn, r0 = rn;
-                if (L + 1 < F.nLevels) {
+                if (L + 1 < nL) {
                     nb = lp[L + 1] + tid;
                     ne = lp[L + 2];
                     if (nb < ne) {
