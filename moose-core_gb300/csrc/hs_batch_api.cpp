@@ -161,7 +161,8 @@ struct HsBatch {
     uint32_t mixHalf = 0;               // nodes of the half-shared arrays
     uint32_t mixPairNodes = 0;          // nodes of a pair of forests, on average
     uint32_t mixDeep = 0;               // doubles of shared memory for deep forests' level offsets
-    uint32_t mixMinLevels = 0, mixLevels = 0, mixMaxNodes = 0;      // of the forests
+    uint32_t mixMinLevels = 0, mixLevels = 0;                       // of the forests
+    uint32_t mixMaxNodes = 0, mixMaxLevels = 1;                     // of the one with the most nodes
     uint32_t mixModes = 0;              // bits 1 << MixForest::shared (a cluster's: staged or not)
     bool mixPairs = false;              // forests stepped in pairs
     bool mixMerged = false;             // CTAs of more than two pairs' nodes: one global forest each
@@ -260,10 +261,14 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
     // The layout depends neither on threads_per_cta nor on how many elim_warps
     // there are, which change without a new one: each layout takes any of them.
     // Unless asked for a number, more eliminators for shared forests of wider
-    // levels: 4 up to 1,279 nodes, 8 from 2,048 (us per step with 4 / 6 / 8: 203
-    // nodes 19.1 / 19.4 / 19.9, ~1,700 45.3 / 43.7 / 44.3, ~6,500 93.7 / 89.6 / 85.8).
+    // levels: 4 up to 44 nodes a level on average, 7 from 75 (us per step with 4 / 5 /
+    // 6 / 7 / 8: a cell of 3,585 nodes in 144 levels 110 / 111 / 112 / 113 / 116, of
+    // 2,174 in 38 40 / 38 / 38 / 39 / 39, of 5,888 in 52 66 / 65 / 63 / 65 / 66;
+    // populations of 5,340 nodes a CTA in 53 levels 78 / 75 / 74 / 73 / 74, of 3,887
+    // in 45 61 / 60 / 59 / 58 / 57).
     if (ew && !b->elimSet && b->mixModes == 1u << kRowsShared)
-        ew = std::max<uint32_t>(4, std::min(b->mixMaxNodes / 256, b->threadsPerCta / 128));
+        ew = std::max<uint32_t>(4, std::min(std::min(b->mixMaxNodes / b->mixMaxLevels / 15 + 2, 7u),
+                                            b->threadsPerCta / 128));
     // A forest in global memory has wide levels of slow loads.  Where they bound
     // the step, ten eliminator warps of 32, or more if asked for (4,096 cells
     // merged: 4 612 us per step, 6 487, 8 420, 10 392; 608 cells and one of 30,000
@@ -935,7 +940,10 @@ int buildMixed(HsBatch* b) {
         F.nLevels = (uint32_t)(levelPtr.size() - F.level0 - 1);
         b->mixMinLevels = fi ? std::min(b->mixMinLevels, F.nLevels) : F.nLevels;
         b->mixLevels = std::max(b->mixLevels, F.nLevels);
-        b->mixMaxNodes = std::max(b->mixMaxNodes, F.nNodes);
+        if (F.nNodes > b->mixMaxNodes) {
+            b->mixMaxNodes = F.nNodes;
+            b->mixMaxLevels = F.nLevels;
+        }
         b->mixModes |= 1u << (!clustered ? F.shared : F.nNodes <= b->mixStageCap ? kRowsShared : kRowsHalf);
         if (nodeCT.size() - F.node0 != F.nNodes) return berr(HS_EINVAL, "mixed batch: forest layout failed");
         if (clustered && F.nLevels > kWsLevels - 1)

@@ -175,7 +175,7 @@ def test_layout_does_not_depend_on_the_tunings_before(gpu, kind):
         b.close()
 
 
-@pytest.mark.parametrize("kind, asked, warps", [("shared", 0, 8), ("shared", 3, 3), ("pair", 0, 6), ("pair", 2, 4),
+@pytest.mark.parametrize("kind, asked, warps", [("shared", 0, 7), ("shared", 3, 3), ("pair", 0, 6), ("pair", 2, 4),
                                                 ("pair", 5, 5), ("pair", 9, 6), ("merged", 0, 10), ("merged", 4, 10),
                                                 ("merged", 12, 12)])
 @pytest.mark.parametrize("stops", [False, True])
@@ -205,3 +205,16 @@ def test_every_cell_has_its_forward_program(gpu, n):
         h.reinit(DT)
         assert gpu.fake_has_forward(0) == 1
         h.close()
+
+
+@pytest.mark.parametrize("p, nodes, warps", [(0.03, 3500, 4), (0.5, 3500, 7), (0.5, 200, 4)])
+def test_eliminators_by_the_width_of_the_levels(gpu, p, nodes, warps):
+    """A shared forest's eliminators by its nodes per level: a long sparse tree of
+    many nodes has narrow levels."""
+    rng = np.random.default_rng(nodes)
+    parent, d, length = models.branched_morphology(rng, nodes, p, 3)
+    b = Batch([models.active_cell(parent, d, length, rng=rng, kca_tables=KCA)], DT, HS_PREC_MIXED)
+    b.reinit(DT)
+    b.process(1)
+    assert gpu.fake_elim_warps() == warps
+    b.close()
