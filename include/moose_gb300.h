@@ -396,9 +396,10 @@ typedef struct HsBatch HsBatch;
 
 /* Launch shape of the batched kernel (0 keeps the current value).
  * FP64: one block per SM, of up to ctas_per_sm teams of threads_per_cta
- * threads (512 threads in all); a team steps its cells one after the other,
- * and a cell too large for a team's share is stepped by the whole block.  Mixed: one CTA steps a forest of cells at a time; a forest
- * holds its elimination arrays in the CTA's shared memory (30 B per node),
+ * threads (512 threads in all), or of more and smaller ones for small cells; a
+ * team steps its cells one after the other, and a cell too large for a team's
+ * share is stepped by the whole block.
+ * Mixed: one CTA steps a forest of cells at a time; a forest holds its elimination arrays in the CTA's shared memory (30 B per node),
  * so ctas_per_sm and forest_nodes set the forest size.  Cells of a CTA that do
  * not fit one such forest are stepped as pairs of forests that keep 16 B per
  * node there, more than two such pairs as one forest in global memory; with
@@ -554,7 +555,8 @@ int hs_batch_read_cell_spikes(HsBatch* b, uint32_t cell, uint32_t first, uint32_
                               double* time, uint32_t capacity, uint32_t* n);
 /* The CUDA stream (a cudaStream_t) the batch runs on, for event timing. */
 int hs_batch_stream(HsBatch* b, void** stream);
-/* Statistics of the packing: compartments, cells, CTAs, launches/step. */
+/* Statistics of the packing: compartments, CTAs (FP64: SMs x teams of
+ * threads_per_cta threads), the tuning's threads_per_cta and steps_per_launch. */
 int hs_batch_info(HsBatch* b, uint64_t* n_compt, uint32_t* n_ctas,
                   uint32_t* threads_per_cta, uint32_t* steps_per_launch);
 /* Mixed batch: how many elimination forests the packing made and how many

@@ -151,9 +151,9 @@ struct HsBatch {
     uint32_t waitRounds = 1u << 24;   // mixed: sleep rounds of one bounded wait (~128 ns each)
     bool useGraph = true;
     uint32_t nCtas = 0;
-    // FP64: one block per SM of nTeams teams (threads_per_cta threads each,
-    // ctas_per_sm of them); cells stepped by a whole block, and by a team
-    uint32_t nBlocks = 0, nTeams = 0, batchWords = 0;
+    // FP64: one block per SM of nTeams teams (ctas_per_sm of threads_per_cta
+    // threads, or more and smaller); cells stepped by a whole block, and by a team
+    uint32_t nBlocks = 0, nTeams = 0, teamThreads = 0, batchWords = 0;
     uint32_t *dWholePtr = nullptr, *dWholeCells = nullptr, *dTeamPtr = nullptr, *dTeamCells = nullptr;
     // mixed: forests per CTA, shared-memory forest capacity
     uint32_t *dCtaPtr = nullptr, *dCtaForests = nullptr;
@@ -247,7 +247,7 @@ namespace {
 cudaError_t launchStep(HsBatch* b, uint32_t k) {
     if (b->precision == HS_PREC_FP64)
         return launchBatchStepFp64(b->dDcs, b->dWholePtr, b->dWholeCells, b->dTeamPtr, b->dTeamCells, b->nBlocks,
-                                   b->nTeams, b->threadsPerCta, b->batchWords, k, b->st);
+                                   b->nTeams, b->teamThreads, b->batchWords, k, b->st);
     uint32_t ew = b->elimWarps && b->threadsPerCta > 32 * b->elimWarps ? b->elimWarps : 0;
     b->mb.waitRounds = b->waitRounds;
     if (b->clusterCtas > 1) {
@@ -301,49 +301,32 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
 // whole block one after the other and the others by the teams side by side;
 // k is the one with the least estimated time, and at least covers the cells
 // whose matrix does not fit a team's share of the shared memory.
-int repack(HsBatch* b) {
-    if (b->gexec) {
-        cudaGraphExecDestroy(b->gexec);
-        b->gexec = nullptr;
-    }
-    if (b->precision != HS_PREC_FP64) return HS_OK;
-    b->packBuf.freeAll();
-    b->packBuf.err = cudaSuccess;
-    const uint32_t nC = b->nCells, warps = b->threadsPerCta / 32;
-    b->nTeams = std::max<uint32_t>(1, std::min<uint32_t>(b->ctasPerSm, kBatchThreads / b->threadsPerCta));
-    b->nBlocks = std::max(1, b->nSm);
-    b->nCtas = b->nBlocks * b->nTeams;
-    b->batchWords = fp64BatchWords(b->nTeams);
-    const uint32_t share = b->batchWords / b->nTeams;
-    std::vector<double> pipe(nC), chain(nC);
-    for (uint32_t c = 0; c < nC; ++c) {
-        const CellPlan& P = b->plans[c];
-        const double rows = std::ceil(P.N / 32.0), waves = P.fWavePtr.empty() ? 0.0 : P.fWavePtr.size() - 1.0;
-        const double ops = 20.0 + (13.0 * P.G + 5.0 * P.C + 45.0 * P.K2 + 9.0 * P.P) / P.N;
-        pipe[c] = 76.0 / 4 * (rows * (ops + 12.0) + 10.0 * P.S / 32 + 6.0 * P.fWaveOps.size() / 32 + 6.0 * waves +
-                              5.0 * P.bLevelPtr.size());
-        chain[c] = 650.0 * ((waves > 0 ? waves : (double)P.fLevelPtr.size()) + P.bLevelPtr.size()) + 4000.0;
-    }
-    auto alone = [&](uint32_t c, uint32_t w) { return pipe[c] * 4.0 / std::min<uint32_t>(4, w) + chain[c]; };
-    std::vector<uint32_t> order(nC);
-    for (uint32_t c = 0; c < nC; ++c) order[c] = c;
-    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return pipe[x] > pipe[y]; });
+// threads_per_cta x ctas_per_sm are the block's threads; where its cells are too
+// small for such teams, they make more and smaller ones (3,000 cells of 30
+// compartments 145 us per step in teams of 128 threads, 88 of 32; of 250 497 and
+// 520), if the slowest block is estimated faster by a tenth.
+struct Fp64Packing {
+    uint32_t teamThreads = 0, teams = 0, words = 0;
+    double time = 0;
+    std::vector<uint32_t> wholePtr, wholeCells, teamPtr, teamCells;
+};
+
+Fp64Packing packFp64(const HsBatch* b, const std::vector<std::vector<uint32_t>>& bins, const std::vector<double>& pipe,
+                     const std::vector<double>& chain, uint32_t teamThreads, uint32_t teams) {
     using Item = std::pair<double, uint32_t>;
     using Queue = std::priority_queue<Item, std::vector<Item>, std::greater<Item>>;
-    std::vector<std::vector<uint32_t>> bins(b->nBlocks);
-    {
-        Queue q;
-        for (uint32_t k = 0; k < b->nBlocks; ++k) q.push({0.0, k});
-        for (uint32_t c : order) {
-            Item it = q.top();
-            q.pop();
-            bins[it.second].push_back(c);
-            q.push({it.first + pipe[c] + 0.3 * chain[c], it.second});
-        }
-    }
-    std::vector<uint32_t> wholePtr(1, 0), wholeCells, teamPtr(1, 0), teamCells;
-    for (uint32_t k = 0; k < b->nBlocks; ++k) {
-        const std::vector<uint32_t>& cells = bins[k];
+    Fp64Packing K;
+    K.teamThreads = teamThreads;
+    K.teams = teams;
+    K.words = fp64BatchWords(teams);
+    K.wholePtr.assign(1, 0);
+    K.teamPtr.assign(1, 0);
+    const uint32_t warps = teamThreads / 32, share = K.words / teams;
+    // (a warp's rows of a cell are on one sub-partition)
+    auto alone = [&](uint32_t c, uint32_t w) {
+        return pipe[c] * 4.0 / std::min(std::min(4u, w), (b->plans[c].N + 31) / 32) + chain[c];
+    };
+    for (const std::vector<uint32_t>& cells : bins) {
         const uint32_t n = (uint32_t)cells.size();
         uint32_t least = 0;
         for (uint32_t i = 0; i < n; ++i)
@@ -354,10 +337,10 @@ int repack(HsBatch* b) {
         uint32_t bestK = n;
         for (uint32_t k0 = least; k0 <= n; ++k0) {
             double t = 0, sum = 0, longest = 0;
-            for (uint32_t i = 0; i < k0; ++i) t += alone(cells[i], warps * b->nTeams);
-            lists.assign(b->nTeams, {});
+            for (uint32_t i = 0; i < k0; ++i) t += alone(cells[i], warps * teams);
+            lists.assign(teams, {});
             Queue q;
-            for (uint32_t m = 0; m < b->nTeams; ++m) q.push({0.0, m});
+            for (uint32_t m = 0; m < teams; ++m) q.push({0.0, m});
             for (uint32_t i = k0; i < n; ++i) {
                 Item it = q.top();
                 q.pop();
@@ -374,25 +357,72 @@ int repack(HsBatch* b) {
                 best = lists;
             }
         }
-        wholeCells.insert(wholeCells.end(), cells.begin(), cells.begin() + bestK);
-        wholePtr.push_back((uint32_t)wholeCells.size());
-        best.resize(b->nTeams);
+        K.time = std::max(K.time, bestT);
+        K.wholeCells.insert(K.wholeCells.end(), cells.begin(), cells.begin() + bestK);
+        K.wholePtr.push_back((uint32_t)K.wholeCells.size());
+        best.resize(teams);
         for (const auto& l : best) {
-            teamCells.insert(teamCells.end(), l.begin(), l.end());
-            teamPtr.push_back((uint32_t)teamCells.size());
+            K.teamCells.insert(K.teamCells.end(), l.begin(), l.end());
+            K.teamPtr.push_back((uint32_t)K.teamCells.size());
         }
+    }
+    return K;
+}
+
+int repack(HsBatch* b) {
+    if (b->gexec) {
+        cudaGraphExecDestroy(b->gexec);
+        b->gexec = nullptr;
+    }
+    if (b->precision != HS_PREC_FP64) return HS_OK;
+    b->packBuf.freeAll();
+    b->packBuf.err = cudaSuccess;
+    const uint32_t nC = b->nCells;
+    const uint32_t teams = std::max<uint32_t>(1, std::min<uint32_t>(b->ctasPerSm, kBatchThreads / b->threadsPerCta));
+    b->nBlocks = std::max(1, b->nSm);
+    b->nCtas = b->nBlocks * teams;
+    std::vector<double> pipe(nC), chain(nC);
+    for (uint32_t c = 0; c < nC; ++c) {
+        const CellPlan& P = b->plans[c];
+        const double rows = std::ceil(P.N / 32.0), waves = P.fWavePtr.empty() ? 0.0 : P.fWavePtr.size() - 1.0;
+        const double ops = 20.0 + (13.0 * P.G + 5.0 * P.C + 45.0 * P.K2 + 9.0 * P.P) / P.N;
+        pipe[c] = 76.0 / 4 * (rows * (ops + 12.0) + 10.0 * P.S / 32 + 6.0 * P.fWaveOps.size() / 32 + 6.0 * waves +
+                              5.0 * P.bLevelPtr.size());
+        chain[c] = 650.0 * ((waves > 0 ? waves : (double)P.fLevelPtr.size()) + P.bLevelPtr.size()) + 4000.0;
+    }
+    std::vector<uint32_t> order(nC);
+    for (uint32_t c = 0; c < nC; ++c) order[c] = c;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return pipe[x] > pipe[y]; });
+    std::vector<std::vector<uint32_t>> bins(b->nBlocks);
+    {
+        using Item = std::pair<double, uint32_t>;
+        std::priority_queue<Item, std::vector<Item>, std::greater<Item>> q;
+        for (uint32_t k = 0; k < b->nBlocks; ++k) q.push({0.0, k});
+        for (uint32_t c : order) {
+            Item it = q.top();
+            q.pop();
+            bins[it.second].push_back(c);
+            q.push({it.first + pipe[c] + 0.3 * chain[c], it.second});
+        }
+    }
+    Fp64Packing K = packFp64(b, bins, pipe, chain, b->threadsPerCta, teams);
+    for (uint32_t part = 2; b->threadsPerCta % (32 * part) == 0 && teams * part <= kBatchThreads / 32; part *= 2) {
+        Fp64Packing smaller = packFp64(b, bins, pipe, chain, b->threadsPerCta / part, teams * part);
+        if (smaller.time < 0.9 * K.time) K = std::move(smaller);
     }
     // no more shared memory than these cells need: the rest is L1 (1,024 cells
     // of 50 to 400 compartments 156 us per step, 166 with all of it taken)
     uint32_t whole = 0, team = 0;
-    for (uint32_t c : wholeCells)
-        if (b->dcs[c].smWords <= b->batchWords) whole = std::max(whole, b->dcs[c].smWords);
-    for (uint32_t c : teamCells) team = std::max(team, b->dcs[c].smWords);
-    b->batchWords = std::max(whole, team * b->nTeams);
-    b->dWholePtr = b->packBuf.up(wholePtr, b->st);
-    b->dWholeCells = b->packBuf.up(wholeCells, b->st);
-    b->dTeamPtr = b->packBuf.up(teamPtr, b->st);
-    b->dTeamCells = b->packBuf.up(teamCells, b->st);
+    for (uint32_t c : K.wholeCells)
+        if (b->dcs[c].smWords <= K.words) whole = std::max(whole, b->dcs[c].smWords);
+    for (uint32_t c : K.teamCells) team = std::max(team, b->dcs[c].smWords);
+    b->nTeams = K.teams;
+    b->teamThreads = K.teamThreads;
+    b->batchWords = std::max(whole, team * K.teams);
+    b->dWholePtr = b->packBuf.up(K.wholePtr, b->st);
+    b->dWholeCells = b->packBuf.up(K.wholeCells, b->st);
+    b->dTeamPtr = b->packBuf.up(K.teamPtr, b->st);
+    b->dTeamCells = b->packBuf.up(K.teamCells, b->st);
     if (b->packBuf.err == cudaSuccess) b->packBuf.err = cudaStreamSynchronize(b->st);
     if (b->packBuf.err != cudaSuccess) return cerr(b->packBuf.err, "batch packing");
     return HS_OK;

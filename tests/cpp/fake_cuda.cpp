@@ -41,6 +41,7 @@ void drop(void* p) {
 
 int g_queries = 0, g_waits = 0;     // calls of cudaEventQuery and cudaStreamWaitEvent
 uint32_t g_elimWarps = 0;           // of the last mixed step: of a pair's, else a global, else a shared forest
+uint32_t g_teams = 0, g_teamThreads = 0;      // of the last FP64 batch step
 int g_device = 0;
 std::map<std::pair<int, const void*>, int> g_limit;      // dynamic shared memory each kernel may take, per device
 const hsg::DevCell* g_cells = nullptr;      // of the last reinit
@@ -84,6 +85,10 @@ const double* fake_table(uint32_t k, uint32_t* shape) {
     return g_cells[k].vTab;
 }
 
+void fake_teams(uint32_t* n, uint32_t* threads) {
+    *n = g_teams;
+    *threads = g_teamThreads;
+}
 uint32_t fake_elim_warps() { return g_elimWarps; }
 int fake_queries() { return g_queries; }
 int fake_waits() { return g_waits; }
@@ -186,7 +191,9 @@ cudaError_t launchGroupStepFp64(const DevCell*, uint32_t, uint32_t, uint32_t, ui
     return cudaSuccess;
 }
 cudaError_t launchBatchStepFp64(const DevCell*, const uint32_t*, const uint32_t*, const uint32_t*, const uint32_t*,
-                                uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, cudaStream_t) {
+                                uint32_t, uint32_t teams, uint32_t teamThreads, uint32_t, uint32_t, cudaStream_t) {
+    g_teams = teams;
+    g_teamThreads = teamThreads;
     return cudaSuccess;
 }
 cudaError_t launchReinitFp64(const DevCell* cells, uint32_t n, cudaStream_t) {

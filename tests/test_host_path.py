@@ -218,3 +218,19 @@ def test_eliminators_by_the_width_of_the_levels(gpu, p, nodes, warps):
     b.process(1)
     assert gpu.fake_elim_warps() == warps
     b.close()
+
+
+@pytest.mark.parametrize("n, count, tuning, teams", [(30, 3000, {}, (16, 32)), (100, 300, {}, (4, 128)),
+                                                     (900, 40, {}, (4, 128)), (30, 3000, dict(threads_per_cta=64, ctas_per_sm=2), (4, 32)),
+                                                     (30, 3000, dict(threads_per_cta=96, ctas_per_sm=2), (2, 96)),
+                                                     (12, 3000, dict(threads_per_cta=32, ctas_per_sm=8), (8, 32))])
+def test_teams_of_the_fp64_batch(gpu, n, count, tuning, teams):
+    """Small cells, many to a block, are stepped by more and smaller teams of as
+    many threads."""
+    b = Batch([_cell(n)] * count, DT, HS_PREC_FP64, **tuning)
+    b.reinit(DT)
+    b.process(1)
+    got = (C.c_uint32 * 2)()
+    gpu.fake_teams(C.byref(got), C.byref(got, 4))
+    assert tuple(got) == teams
+    b.close()
