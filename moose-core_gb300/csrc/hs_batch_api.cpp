@@ -857,11 +857,11 @@ int buildMixed(HsBatch* b) {
     // 7,000 nodes: 86 us, 93 in pairs; 250 nodes: 27 and 34).
     // From three pairs on, one forest of all of a CTA's cells in global memory:
     // its tail and back substitution are a small part by then, and nothing
-    // waits between the pairs (4,096 cells: 396 us per step with ten eliminator
+    // waits between the pairs (4,096 cells: 392 us per step with ten eliminator
     // warps, 415 in pairs; 2,048 cells, two pairs: 229 and 221).
     // Only CTAs that do not fit a shared forest are merged, so that beside one
     // very large cell the others stay in shared memory (608 cells, one more of
-    // 30,000 compartments at its stop step: 91 us per step, 118 with all merged).
+    // 30,000 compartments at its stop step: 78 us per step, 118 with all merged).
     // Without eliminator warps, or with a forest of 256 levels or more: shared
     // and global forests one after the other.
     std::vector<std::vector<ForestPlan>> pairsOf;

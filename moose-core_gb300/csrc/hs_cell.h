@@ -31,7 +31,7 @@ struct Arena {
 // constants of all cells contiguous, for one-copy reinit) and rate tables
 // shared by the cells that have identical ones.  `spikes`: where the spike
 // buffers go, if not into `a` (a drop-in solver's: an allocation of more than
-// 1 MiB costs 57 us to make and free, two smaller ones 4).
+// 1 MiB maps memory of its own, ~70 us; smaller ones share a mapping).
 std::vector<double> pairTable(const Table& t);   // rate table as the FP64 kernels read it (DevCell::vTab)
 struct CellShared {
     double* initVm = nullptr;

@@ -47,9 +47,9 @@ class Batch:
 
     def tune(self, threads_per_cta=0, ctas_per_sm=0, steps_per_launch=0, use_graph=True, forest_nodes=0,
              max_ctas=0, elim_warps=0, wait_rounds=0, cluster_ctas=0):
-        """New launch shape.  On a mixed batch a new ctas_per_sm or
-        forest_nodes rebuilds the layout: reinit (and re-register recording
-        and inject targets) before the next process()."""
+        """New launch shape.  On a mixed batch a new ctas_per_sm,
+        forest_nodes, max_ctas or cluster_ctas rebuilds the layout: reinit (and
+        re-register recording and inject targets) before the next process()."""
         t = HsBatchTuning(threads_per_cta, ctas_per_sm, steps_per_launch, 1 if use_graph else 0, forest_nodes,
                           max_ctas, elim_warps, wait_rounds, cluster_ctas)
         _native.check(_native.load().hs_batch_tune(self._h, C.byref(t)))
