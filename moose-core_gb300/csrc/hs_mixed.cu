@@ -379,6 +379,7 @@ struct SharedRows {              // all of them, `cap` nodes, from the area's do
     __device__ __forceinline__ double* base() const { return sArea() + first; }
     __device__ __forceinline__ double& D(uint32_t i) const { return base()[i]; }
     __device__ __forceinline__ double& R(uint32_t i) const { return base()[cap + i]; }
+    __device__ __forceinline__ double* side(bool r) const { return base() + (r ? cap : 0); }     // R or D
     __device__ __forceinline__ double& OFF(uint32_t i) const { return base()[2 * cap + i]; }
     __device__ __forceinline__ uint32_t& TOPO(uint32_t i) const { return reinterpret_cast<uint32_t*>(base() + 3 * cap)[i]; }
     __device__ __forceinline__ uint16_t& PAR(uint32_t i) const {
@@ -390,6 +391,7 @@ struct GlobalRows {
     uint32_t node0;
     __device__ __forceinline__ double& D(uint32_t i) const { return b.elimD[node0 + i]; }
     __device__ __forceinline__ double& R(uint32_t i) const { return b.elimR[node0 + i]; }
+    __device__ __forceinline__ double* side(bool r) const { return (r ? b.elimR : b.elimD) + node0; }
     __device__ __forceinline__ double OFF(uint32_t i) const { return __ldg(b.off + node0 + i); }
     __device__ __forceinline__ uint32_t TOPO(uint32_t i) const { return __ldg(b.topo + node0 + i); }
     __device__ __forceinline__ uint32_t PAR(uint32_t i) const { return __ldg(b.par + node0 + i); }
@@ -433,12 +435,13 @@ __device__ __forceinline__ void pullNarrow(const Rows& E, uint32_t b0, uint32_t 
     const bool on = i < e;
     const uint32_t t = on ? E.TOPO(i) : 0u;
     const uint32_t c0 = t & 0xFFFF, c1 = c0 + ((t >> 16) & 0xFF);
-    double x = on ? (rl ? E.R(i) : E.D(i)) : 1.0;
-    for (uint32_t c = c0; c < c1; ++c) x = fma(-E.OFF(c), rl ? E.R(c) : E.D(c), x);
+    double* const a = E.side(rl);
+    double x = on ? a[i] : 1.0;
+    for (uint32_t c = c0; c < c1; ++c) x = fma(-E.OFF(c), a[c], x);
     const double ivd = rcpPivot(x);
     const double iv = __shfl_sync(0xFFFFFFFFu, ivd, (tid & 31u) & ~1u);
     const double y = (rl ? x : (on ? E.OFF(i) : 0.0)) * iv;
-    if (on) (rl ? E.R(i) : E.D(i)) = y;
+    if (on) a[i] = y;
 }
 
 // Per-cell work of tick 0 (stimulus schedule) for the forest's cells.
