@@ -266,17 +266,19 @@ cudaError_t launchStep(HsBatch* b, uint32_t k) {
     // 2,174 in 38 40 / 38 / 38 / 39 / 39, of 5,888 in 52 66 / 65 / 63 / 65 / 66;
     // populations of 5,340 nodes a CTA in 53 levels 78 / 75 / 74 / 73 / 74, of 3,887
     // in 45 61 / 60 / 59 / 58 / 57).
+    const uint32_t width = b->mixMaxNodes / b->mixMaxLevels;
     if (ew && !b->elimSet && b->mixModes == 1u << kRowsShared)
-        ew = std::max<uint32_t>(4, std::min(std::min(b->mixMaxNodes / b->mixMaxLevels / 15 + 2, 7u),
-                                            b->threadsPerCta / 128));
+        ew = std::max<uint32_t>(4, std::min(std::min(width / 15 + 2, 7u), b->threadsPerCta / 128));
     // A forest in global memory has wide levels of slow loads.  Where they bound
     // the step, ten eliminator warps of 32, or more if asked for (4,096 cells
     // merged: 4 612 us per step, 6 487, 8 420, 10 392; 608 cells and one of 30,000
-    // compartments, with stop steps: 10 322, 16 409).  Of a CTA's that has shared
-    // ones too, as a serving cohort's batch with its stop steps, twice the shared
+    // compartments, with stop steps: 10 322, 16 409), but no more than elsewhere where
+    // levels are narrow (1,600 nodes in ~60 of them: 4 93, 10 100).  Beside shared
+    // ones, as in a serving cohort's batch with its stop steps, twice the shared
     // forests' (a 10,000-compartment cell 184 -> 159).
     uint32_t gw = ew;
-    if (ew && (b->mixMerged || b->mixModes == 1u << kRowsGlobal)) gw = std::max(ew, b->threadsPerCta * 10 / 1024);
+    if (ew && (b->mixMerged || b->mixModes == 1u << kRowsGlobal))
+        gw = width < 45 ? ew : std::max(ew, b->threadsPerCta * 10 / 1024);
     else if (b->mb.anyStop) gw = std::min(2 * ew, 16u);
     // Eliminators of each forest of a pair: 3/16 of the CTA, of pairs of more than
     // 12,288 nodes, with their wider levels, one of 32 warps less (us per step with

@@ -234,3 +234,16 @@ def test_teams_of_the_fp64_batch(gpu, n, count, tuning, teams):
     gpu.fake_teams(C.byref(got), C.byref(got, 4))
     assert tuple(got) == teams
     b.close()
+
+
+@pytest.mark.parametrize("n, warps", [(1700, 4), (9000, 10)])
+def test_eliminators_of_global_forests_by_the_width_of_the_levels(gpu, n, warps):
+    """Five CTAs an SM leave shared memory for ~1,400 nodes."""
+    rng = np.random.default_rng(n)
+    parent, d, length = models.branched_morphology(rng, n, 0.06 if warps == 4 else 0.5, 3)
+    b = Batch([models.active_cell(parent, d, length, rng=rng, kca_tables=KCA)], DT, HS_PREC_MIXED, ctas_per_sm=5)
+    b.reinit(DT)
+    b.process(1)
+    assert _forests(b) == (1, 0)
+    assert gpu.fake_elim_warps() == warps
+    b.close()
