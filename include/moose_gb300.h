@@ -424,10 +424,11 @@ typedef struct HsBatchTuning {
                                    fuller forests leave SMs to other batches */
     uint32_t elim_warps;        /* mixed: warps of a CTA that eliminate while the
                                    others assemble; 0 at creation: by layout (of
-                                   32 warps: 4 to 8 for a shared forest by its
-                                   size, 6 or 5 for each forest of a pair, 10 for
-                                   forests in global memory, twice the shared
-                                   ones' beside such with stop steps), later: the
+                                   32 warps: 4 to 7 for a shared forest by the
+                                   width of its levels, 6 or 5 for each forest of
+                                   a pair, 4 or 10 for forests in global memory,
+                                   beside shared ones with stop steps twice as
+                                   many as those), later: the
                                    current value.  A number is taken as it is for
                                    shared forests, within 4 and the default for a
                                    pair's, and from the default on for global
